@@ -25,6 +25,7 @@ NVFLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler"
 CU_UNITS = {
     "lt_api.cu": [],
     "lt_step_fp64.cu": ["-fmad=false"],
+    "lt_column_fp64.cu": ["-fmad=false"],
     "lt_step_mixed.cu": [],
     "lt_misc.cu": ["-fmad=false"],
     "lt_noalloc.cu": ["-fmad=false"],

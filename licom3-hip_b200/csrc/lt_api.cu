@@ -194,6 +194,8 @@ void plan_arena(Arena& a, Plan& pl) {
     D(&a.utf, F); D(&a.vtf, F); D(&a.utl, F); D(&a.vtl, F); D(&a.akt, 2 * F);
     D(&a.utf_out, F); D(&a.vtf_out, F); D(&a.ws, FB); D(&a.uwf, F); D(&a.vsf, F); D(&a.wka, F);
   }
+  pl.add(reinterpret_cast<void**>(&a.flags), sizeof(unsigned) * 2 * km * ((a.imt + kColX - 1) / kColX) * ((a.jmt + kColY - 1) / kColY) *
+                                               (kColX * kColY / 32));
   D(&a.h0f, A); D(&a.h0l, A); D(&a.h0f_out, A); D(&a.net, 2 * A);
   double** two_d[] = {&a.swv, &a.nswv, &a.sst, &a.sss, &a.fresh, &a.seaice, &a.tarea, &a.tarea_r, &a.htw,
                       &a.hts, &a.hun, &a.hue, &a.dxu, &a.dyu, &a.ahf, &a.dtn, &a.dts, &a.dte, &a.dtw,
@@ -213,7 +215,6 @@ void plan_arena(Arena& a, Plan& pl) {
     D(&a.ax, 2 * F); D(&a.ay, 2 * F); D(&a.az, 2 * F); D(&a.dzd, 2 * F);
     D(&a.tend, 2 * F); D(&a.dt_diff, 2 * F); D(&a.dt_conv, 2 * F); D(&a.penetrate, F);
     D(&a.fold_save, 2 * km * (size_t)a.imt);
-    I(&a.kfz, A);
   } else {
     D(&a.dt_conv, 2 * F);  // convadj writes it
     D(&a.tend, 2 * F);     // convadj accumulates into it
@@ -247,7 +248,8 @@ long slots_for(const Arena& a, int sms) {
 
 }  // namespace
 
-bool make_tensor_map_3d(CUtensorMap* map, const void* base, int esize, long nx, long ny, long nz, int bx, int by) {
+bool make_tensor_map_3d(CUtensorMap* map, const void* base, int esize, long nx, long ny, long nz, int bx, int by,
+                        int bz) {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   if (!encode) {
     cudaDriverEntryPointQueryResult q;
@@ -259,7 +261,7 @@ bool make_tensor_map_3d(CUtensorMap* map, const void* base, int esize, long nx, 
   if ((nx * esize) % 16 != 0 || (reinterpret_cast<uintptr_t>(base) % 16) != 0 || (bx * esize) % 16 != 0) return false;
   const cuuint64_t dims[3] = {(cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
   const cuuint64_t strides[2] = {(cuuint64_t)(nx * esize), (cuuint64_t)(nx * ny * esize)};
-  const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
+  const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
   const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult r = encode(map, esize == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                             const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -271,20 +273,34 @@ bool make_tensor_map_3d(CUtensorMap* map, const void* base, int esize, long nx, 
 bool build_tracer_maps(const Arena& a, TracerMaps* m) {
   const long imt = a.imt, jmt = a.jmt, km = a.km;
   const bool mx = a.precision == LT_PREC_MIXED;
-  const int ty = mx ? kMixedTileY : TY;   // tile rows of the column kernel
-  bool ok = true;
-  const int bw64 = mx ? kMixedBoxW64 : SW;   // state box width
-  for (int b = 0; b < 2; ++b) {
-    ok = ok && make_tensor_map_3d(&m->at[b], a.at[b], 8, imt, jmt, 2 * km, bw64, ty + 4);
-    ok = ok && make_tensor_map_3d(&m->atb[b], a.atb[b], 8, imt, jmt, 2 * (km + 1), bw64, ty + 4);
-  }
   const int es = mx ? 4 : 8;
-  ok = ok && make_tensor_map_3d(&m->ws, mx ? (const void*)a.ws32 : a.ws, es, imt, jmt, km + 1, SW, ty + 2);
-  // f64: face transports u_wface (rows y0-1..) and v_sface (rows y0-2..);
-  // mixed: the U-point means wkd, wkb (rows y0-2..), faces formed in the kernel
-  ok = ok && make_tensor_map_3d(&m->uw, mx ? (const void*)a.wkd32 : a.uwf, es, imt, jmt, km, SW, mx ? ty + 3 : ty + 2);
-  ok = ok && make_tensor_map_3d(&m->vs, mx ? (const void*)a.wkb32 : a.vsf, es, imt, jmt, km, SW, ty + 3);
-  ok = ok && make_tensor_map_3d(&m->akt, mx ? (const void*)a.akt32 : a.akt, es, imt, jmt, 2 * km, TX, ty);
+  bool ok = true;
+  if (mx) {
+    const int ty = kMixedTileY;   // tile rows of the column kernel
+    for (int b = 0; b < 2; ++b) {
+      ok = ok && make_tensor_map_3d(&m->at[b], a.at[b], 8, imt, jmt, 2 * km, kMixedBoxW64, ty + 4);
+      ok = ok && make_tensor_map_3d(&m->atb[b], a.atb[b], 8, imt, jmt, 2 * (km + 1), kMixedBoxW64, ty + 4);
+    }
+    ok = ok && make_tensor_map_3d(&m->ws, a.ws32, es, imt, jmt, km + 1, SW, ty + 2);
+    // the U-point means wkd, wkb (rows y0-2..), faces formed in the kernel
+    ok = ok && make_tensor_map_3d(&m->uw, a.wkd32, es, imt, jmt, km, SW, ty + 3);
+    ok = ok && make_tensor_map_3d(&m->vs, a.wkb32, es, imt, jmt, km, SW, ty + 3);
+    ok = ok && make_tensor_map_3d(&m->akt, a.akt32, es, imt, jmt, 2 * km, TX, ty);
+  } else {
+    for (int b = 0; b < 2; ++b) {
+      ok = ok && make_tensor_map_3d(&m->at[b], a.at[b], 8, imt, jmt, 2 * km, kColX + 8, kColY + 2);
+      ok = ok && make_tensor_map_3d(&m->atb[b], a.atb[b], 8, imt, jmt, 2 * (km + 1), kColX + 8, kColY + 2);
+      ok = ok && make_tensor_map_3d(&m->atb_own[b], a.atb[b], 8, imt, jmt, 2 * (km + 1), kColX, kColY);
+    }
+    ok = ok && make_tensor_map_3d(&m->ws, a.ws, es, imt, jmt, km + 1, kColX, kColY);
+    ok = ok && make_tensor_map_3d(&m->uw, a.uwf, es, imt, jmt, km, kColX + 8, kColY);
+    ok = ok && make_tensor_map_3d(&m->vs, a.vsf, es, imt, jmt, km, kColX, kColY + 1);
+    ok = ok && make_tensor_map_3d(&m->akt, a.akt, es, imt, jmt, 2 * km, kColX, kColY);
+  }
+  for (int b = 0; b < 2; ++b)
+    ok = ok && make_tensor_map_3d(&m->th_at[b], a.at[b], 8, imt, jmt, 2 * km, kThomasX, kThomasY, kThomasLevels);
+  ok = ok && make_tensor_map_3d(&m->th_akt, mx ? (const void*)a.akt32 : a.akt, es, imt, jmt, 2 * km, kThomasX,
+                                kThomasY, kThomasLevels);
   if (mx) {
     const float* vel[4] = {a.utf32, a.vtf32, a.utl32, a.vtl32};
     for (int v = 0; v < 4; ++v)
@@ -322,10 +338,7 @@ int run_step(lt_domain* d, cudaEvent_t forcing_ready) {
   if (a.precision == LT_PREC_MIXED) {
     if ((rc = launch_tracer_tma_mixed(a, d->maps, d->use_tma, s, d->tma_grid))) return rc;
   } else if (a.p.adv_tracer == LT_ADV_TSPAS) {
-    // the TMA-slot column kernel is the tspas scheme's (its level boxes by
-    // per-thread copies where the row pitch does not allow TMA); the centred
-    // and flux schemes run in the plain-load kernel
-    if ((rc = launch_tracer_tma64(a, d->maps, s, d->tma_grid, d->use_tma))) return rc;
+    if ((rc = launch_column_fp64(a, d->maps, d->use_tma, s))) return rc;
   } else {
     if ((rc = launch_tracer_fp64(a, s, d->slots))) return rc;
   }
@@ -572,6 +585,10 @@ int lt_create(const lt_grid* g, const lt_params* p, lt_domain** out) {
   cudaStreamCreateWithFlags(&d->copy_stream, cudaStreamNonBlocking);
   // TMA-fed tracer kernel where the row pitch is a multiple of 16 bytes
   d->use_tma = build_tracer_maps(d->a, &d->maps);
+  if (d->a.precision == LT_PREC_FP64 && prepare_column_fp64() != LT_OK) {
+    lt_destroy(d);
+    return LT_E_CUDA;
+  }
   // one persistent CTA per resident slot (kFp64CtasPerSm, kMixedCtasPerSm
   // per SM: the kernels' __launch_bounds__ and shared-memory footprints)
   const long per_sm = d->a.precision == LT_PREC_MIXED ? kMixedCtasPerSm : kFp64CtasPerSm;

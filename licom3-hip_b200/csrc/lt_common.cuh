@@ -28,6 +28,13 @@ constexpr int kMixedThreads = TX * kMixedTileY;
 constexpr int kMixedBoxW64 = TX + 4;
 constexpr int kMixedScratchPerLevel = 4;
 constexpr int kMixedMaxLevels = 128;
+// The FP64 limiter and explicit passes (lt_column_fp64.cu): blocks of kColX x
+// kColY columns.
+constexpr int kColX = 32, kColY = 4;
+// The implicit pass over the columns (lt_thomas.cuh): blocks of kThomasX x
+// kThomasY columns of one tracer, their level data in stages of
+// kThomasLevels levels.
+constexpr int kThomasX = 32, kThomasY = 4, kThomasLevels = 8;
 // The mixed continuity march: tiles of 32 x kMixedContTileY columns, each
 // level's U-point velocities as boxes kMixedContBoxW wide (x0 .. x0+35: the
 // 33 columns the march reads, rounded up to 16 bytes) and kMixedContTileY+1
@@ -69,14 +76,11 @@ struct alignas(16) Arena {   // copied into shared memory as 16-byte words
   double *duc, *dum, *dun, *dus, *due, *duw, *dmc, *dmn, *dms, *dme, *dmw, *amf, *uarea_r, *dxur, *dyur;
   // diagnostics (null when off)
   double *ax, *ay, *az, *dzd, *tend, *dt_diff, *dt_conv, *penetrate;
-  // [jmt][imt], with diagnostics: one past the deepest level at which the
-  // column's west or south face transport or its w is nonzero (written by
-  // the continuity; the column kernel's deep-level shortcut reads it)
-  int* kfz;
 
   // step scratch
   double *uwf, *vsf;          // face transports u_wface, v_sface [km][jmt][imt]
   double *wka;                // horizontal divergence [km][jmt][imt]
+  unsigned* flags;            // [2][km] limiter flags, one word per patch of 8 x 4 columns
   // mixed precision: f32 storage of the dynamics inputs, mixing and the
   // derived fields (the f64 pointers above are null for these; the
   // horizontal divergence lives only in registers of the continuity march)
@@ -130,6 +134,7 @@ int launch_ssh(const Arena& a, cudaStream_t s);
 int launch_surface_fluxes(const Arena& a, cudaStream_t s);
 int launch_continuity_fp64(const Arena& a, cudaStream_t s);
 int launch_tracer_fp64(const Arena& a, cudaStream_t s, int slots);
+int launch_assm_dt_restore(const Arena& a, cudaStream_t s);
 int launch_halo_state(const Arena& a, cudaStream_t s);
 int launch_halo_r8(double* f, int nz, int imt, int jmt, int ew_cyclic, int tripole, cudaStream_t s);
 int launch_tree_sum(const double* x, long n, double* part, double* out, cudaStream_t s);
@@ -147,6 +152,30 @@ int launch_f64_to_f32(const double* x, float* y, long n, cudaStream_t s);
 int launch_f32_to_f64(const float* x, double* y, long n, cudaStream_t s);
 int tracer_slots(const Arena& a);
 size_t tree_sum_part_elems(long n);
+
+// a / h for a divisor that serves many dividends: with y = RN(1/h) and a
+// quotient q within one unit of a/h, RN(q - y*(h*q - a)) is the correctly
+// rounded a/h (P. Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), as long as no
+// intermediate underflows or overflows; a first step of the same form brings
+// a*y within one unit.  The remainder is taken with this sign so that a zero
+// keeps its sign.  Dividends whose exponent is not within 400 of 0 (but zeros)
+// and divisors that are not positive or as far from 1 are divided.
+constexpr unsigned kDivLow = 2u * ((1023u - 400u) << 20), kDivSpan = 2u * (800u << 20);   // of twice the upper word
+__device__ __forceinline__ unsigned div_key(double a) { return 2u * (unsigned)__double2hiint(a) - kDivLow; }
+__device__ __forceinline__ bool div_admits(double h) { return h > 0.0 && div_key(h) < kDivSpan; }
+__device__ __forceinline__ double div_fast(double a, double h, double y) {
+  double q = a * y;
+  q = __fma_rn(-__fma_rn(h, q, -a), y, q);
+  return __fma_rn(-__fma_rn(h, q, -a), y, q);
+}
+// 1/h where quotient() may use it, else 0
+__host__ __device__ inline double quotient_reciprocal(double h) { return h > 1.0e-100 && h < 1.0e100 ? 1.0 / h : 0.0; }
+__device__ __forceinline__ double quotient(double a, double h, double y) {
+  double q = div_fast(a, h, y);
+  if (y == 0.0 || (div_key(a) >= kDivSpan && a != 0.0)) q = a / h;
+  return q;
+}
 
 // L2 policies of the column sweeps' scratch.  The elimination coefficients of
 // a work item's wet levels are written during its march and read once, in
@@ -180,6 +209,13 @@ __device__ __forceinline__ double2 ld_l2(const double2* p, uint64_t pol) {
   double2 v;
   asm volatile("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(p), "l"(pol));
   return v;
+}
+
+// tracer_7's nudging toward restore_at (simple_assm; tracer.cpp:1587-1611):
+// the rate of level k, 1/(5 days) down to level 45 and smaller by
+// ((k+1)/5)^2 below, in the reference's operation order
+__device__ __forceinline__ double assm_rate(int k) {
+  return k < 45 ? 1.0e0 / (5.e0 * 86400.e0) : 1.0e0 / (5.e0 * 86400.e0) / ((k + 1) * (k + 1) / 5.0 / 5.0);
 }
 
 }  // namespace lt

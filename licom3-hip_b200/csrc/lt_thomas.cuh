@@ -1,0 +1,219 @@
+// lt_thomas.cuh - the last pass over the columns, both precision forms: the
+// implicit half of the vertical mixing (invtrit, tracer.cpp:923-978), the new
+// state, and the dry levels.
+//
+// The pass finds the explicitly updated values in the new state at[cur^1].
+// One thread per column and tracer eliminates from the bottom level up and
+// substitutes from the top down; the elimination coefficients take the place
+// of the values they came from (f in at[cur^1], e in atb[cur^1]), written
+// with an L2 evict-last policy and read back evict-first, so that they stay
+// on chip: 16 B per level and column in flight.  The level data arrive in
+// stages of kThLevels levels through a ring of shared-memory slots, so a
+// warp's chain of divisions never waits for memory: by TMA boxes, or by
+// per-thread asynchronous copies where the row pitch does not allow boxes.
+// Every wait is bounded.
+#pragma once
+#include "lt_common.cuh"
+#include "lt_tracer_tma.cuh"
+
+namespace lt {
+
+constexpr int kThX = kThomasX, kThY = kThomasY, kThT = kThX * kThY;
+constexpr int kThLevels = kThomasLevels;
+constexpr int kThStages = 3;
+
+template <class AK>
+struct ThomasSmem {
+  struct alignas(128) Slot {
+    alignas(128) double d8[kThLevels * kThT];   // levels l0 .. l0+kThLevels-1 of the explicit values
+    alignas(128) AK akt[kThLevels * kThT];      // levels l0-1 .. of the mixing coefficient
+  } slot[kThStages];
+  uint64_t bar[kThStages];
+  int wmax[kThT / 32];
+};
+
+// Columns of one block: x0.., y0.., tracer n.  DIAG: with the diagnostics of
+// tracer_9 (tend, dt_diff) and the pre-fold values of the top row.
+template <class AK, bool DIAG>
+__device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& maps, bool tma, int x0, int y0, int n) {
+  extern __shared__ __align__(128) unsigned char smem_th[];
+  ThomasSmem<AK>& S = *reinterpret_cast<ThomasSmem<AK>*>(smem_th);
+  constexpr bool F64 = sizeof(AK) == 8;
+  const int tid = threadIdx.x, tx = tid % kThX, ty = tid / kThX;
+  const int i = x0 + tx, j = y0 + ty;
+  const int imt = a.imt, jmt = a.jmt, km = a.km;
+  const long A = a.A;
+  const bool inner = i >= 2 && i < imt - 2 && j >= 2 && j < jmt - 2;
+  const long q = inner ? (long)j * imt + i : 0;
+  const int kz = inner ? a.kmt[q] : 0;
+  const int top = __reduce_max_sync(0xffffffffu, kz);
+  if (tid % 32 == 0) S.wmax[tid / 32] = top;
+  if (tid == 0) {
+    for (int s = 0; s < kThStages; ++s) mbar_init(&S.bar[s], kThT);   // one arrival per thread and stage
+    mbar_fence_init();
+  }
+  __syncthreads();
+  int kmax = 0;
+#pragma unroll
+  for (int w = 0; w < kThT / 32; ++w) kmax = max(kmax, S.wmax[w]);
+
+  double* __restrict__ at_out = a.at[a.cur ^ 1] + n * a.F;
+  double* __restrict__ atb_out = a.atb[a.cur ^ 1] + n * a.FB;
+  const double* __restrict__ at_in = a.at[a.cur] + n * a.F;
+  const AK* __restrict__ akt = (F64 ? (const AK*)a.akt : (const AK*)a.akt32) + n * a.F;
+  // stage t holds levels l0(t) .. l0(t)+kThLevels-1, l0(t) = (stages-1-t)*kThLevels
+  const int stages = (kmax + kThLevels - 1) / kThLevels;
+  auto issue = [&](int t) {
+    const int l0 = (stages - 1 - t) * kThLevels, r = t % kThStages;
+    typename ThomasSmem<AK>::Slot& sl = S.slot[r];
+    if (tma) {
+      if (tid == 0) {
+        mbar_expect_tx(&S.bar[r], (uint32_t)(kThLevels * kThT * (sizeof(double) + sizeof(AK))));
+        // boxes of both tracers' levels: beyond a tracer's last level the box
+        // reads its neighbour's levels or zeros, which no column uses
+        tma_load_3d(sl.d8, &maps.th_at[a.cur ^ 1], x0, y0, n * km + l0, &S.bar[r]);
+        tma_load_3d(sl.akt, &maps.th_akt, x0, y0, n * km + l0 - 1, &S.bar[r]);
+      } else {
+        mbar_arrive(&S.bar[r]);
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < kThLevels; ++c) {
+        const int k = l0 + c;
+        const bool in = inner && k < kz;
+        cp_async8z(&sl.d8[c * kThT + tid], at_out + (in ? (long)k * A + q : 0), in);
+        const bool ia = in && k >= 1;
+        const AK* src = akt + (ia ? (long)(k - 1) * A + q : 0);
+        if (F64) cp_async8z(&sl.akt[c * kThT + tid], src, ia);
+        else cp_async4z(&sl.akt[c * kThT + tid], src, ia);
+      }
+      cp_async_mbar_arrive(&S.bar[r]);
+    }
+  };
+  for (int t = 0; t < kThStages && t < stages; ++t) issue(t);
+
+  // the dry levels keep their values (with diagnostics the explicit pass left
+  // them in the new state already): eight levels' loads ahead of their stores
+  if (!DIAG && inner) {
+    for (int k0 = kz; k0 < km; k0 += 8) {
+      double v[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v[c] = k0 + c < km ? __ldcs(at_in + (long)(k0 + c) * A + q) : 0.0;
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (k0 + c < km) {
+          __stcs(at_out + (long)(k0 + c) * A + q, v[c]);
+          __stcs(atb_out + (long)(k0 + c + 1) * A + q, v[c]);
+        }
+    }
+  }
+
+  const double dts = a.p.dts;
+  const double* __restrict__ odzp = a.odzp;
+  const double* __restrict__ odzt = a.odzt;
+  double e = 0.0, f = 0.0;                                       // of the level below
+  double ak = 0.0;                                               // akt of level k
+  const uint64_t keep = l2_evict_last();
+  for (int t = 0; t < stages; ++t) {
+    const int l0 = (stages - 1 - t) * kThLevels, r = t % kThStages;
+    const bool ok = mbar_wait(&S.bar[r], (uint32_t)((t / kThStages) & 1), a.wait_limit);
+    if (__syncthreads_or(!ok)) {
+      // a wait ran out: record it, let the copies still in flight land
+      // (bounded) and leave together
+      if (tid == 0) {
+        atomicExch(a.status + 1, 1);
+        for (int u = t; u < stages && u < t + kThStages; ++u)
+          mbar_wait(&S.bar[u % kThStages], (uint32_t)((u / kThStages) & 1));
+      }
+      __syncthreads();
+      return;
+    }
+    const typename ThomasSmem<AK>::Slot& sl = S.slot[r];
+#pragma unroll
+    for (int c = kThLevels - 1; c >= 0; --c) {
+      const int k = l0 + c;
+      if (k >= kz) continue;
+      const double d8 = sl.d8[c * kThT + tid], au = (double)sl.akt[c * kThT + tid];
+      double a8, c8, b8;
+      if (k >= 1) a8 = au * odzt[k] * odzp[k] * dts * 0.5;
+      else a8 = odzp[0] * dts * 0.5;
+      if (k == kz - 1) {
+        c8 = odzp[kz - 1] * dts * 0.5;
+        b8 = 1.0 + a8;
+      } else {
+        c8 = ak * odzt[k + 1] * odzp[k] * dts * 0.5;
+        b8 = k >= 1 ? 1.0 + a8 + c8 : 1.0 + c8;
+      }
+      const double g0 = 1.0 / (b8 - c8 * e);
+      e = a8 * g0;
+      f = (d8 + c8 * f) * g0;
+      ak = au;
+      st_l2(at_out + (long)k * A + q, f, keep);
+      st_l2(atb_out + (long)(k + 1) * A + q, e, keep);
+      if (DIAG) a.dt_diff[n * a.F + (long)k * A + q] = d8;
+    }
+    __syncthreads();   // the slot is read
+    if (t + kThStages < stages) issue(t + kThStages);
+  }
+  if (!inner) return;
+
+  // substitution, top down: the coefficients of SUB levels loaded together
+  const double stf = a.stf_n[n * A + q];
+  constexpr int SUB = 8;
+  const uint64_t once = l2_evict_first();
+  double x = 0.0;
+  const int kend = DIAG ? km : kz;
+  for (int k0 = 0; k0 < kend; k0 += SUB) {
+    double ev[SUB], fv[SUB];
+#pragma unroll
+    for (int c = 0; c < SUB; ++c) {
+      const int k = k0 + c;
+      ev[c] = k < kz ? ld_l2(atb_out + (long)(k + 1) * A + q, once) : 0.0;
+      fv[c] = k < kend ? ld_l2(at_out + (long)k * A + q, once) : 0.0;
+    }
+#pragma unroll
+    for (int c = 0; c < SUB; ++c) {
+      const int k = k0 + c;
+      if (k >= kend) break;
+      double v = fv[c];
+      if (k < kz) v = x = ev[c] * (k == 0 ? stf : x) + fv[c];
+      if (DIAG) {
+        const long cg = n * a.F + (long)k * A + q;
+        const double vit = k < kz ? 1.0 : 0.0;
+        const double d8 = k < kz ? a.dt_diff[cg] : v;
+        a.tend[cg] = (v - at_in[(long)k * A + q]) / dts * vit;
+        if (k == 0) a.dt_diff[cg] = (v - d8) / dts * vit - stf * 0.5 * odzp[0];
+        else a.dt_diff[cg] = (v - d8) / dts * vit;
+        if (j == 2 && a.tripole) a.fold_save[((long)(n * km + k)) * imt + i] = d8;
+      }
+      __stcs(at_out + (long)k * A + q, v);
+      __stcs(atb_out + (long)(k + 1) * A + q, v);
+    }
+  }
+}
+
+template <class AK, bool DIAG>
+__global__ void __launch_bounds__(kThT) k_thomas(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps,
+                                                 int tma) {
+  thomas_block<AK, DIAG>(a, maps, tma != 0, blockIdx.x * kThX, blockIdx.y * kThY, blockIdx.z);
+}
+
+// shared-memory size of the pass on the current device (not inside a capture)
+template <class AK>
+int prepare_thomas() {
+  const int sm = (int)sizeof(ThomasSmem<AK>);
+  LT_CUDA_OK(cudaFuncSetAttribute(k_thomas<AK, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+  if (sizeof(AK) == 8)
+    LT_CUDA_OK(cudaFuncSetAttribute(k_thomas<AK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+  return LT_OK;
+}
+
+template <class AK, bool DIAG>
+int launch_thomas(const Arena& a, const TracerMaps& maps, bool tma, cudaStream_t s) {
+  const size_t sm = sizeof(ThomasSmem<AK>);
+  k_thomas<AK, DIAG><<<dim3((a.imt + kThX - 1) / kThX, (a.jmt + kThY - 1) / kThY, 2), kThT, sm, s>>>(a, maps, tma ? 1 : 0);
+  LT_LAUNCHED();
+  return LT_OK;
+}
+
+}  // namespace lt

@@ -93,7 +93,8 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
 }
 
 // Host: encode a 3-D tiled tensor map over a [nz][ny][nx] array of `esize`-byte
-// elements with box (bx, by, 1).  Returns false if the driver refuses.
-bool make_tensor_map_3d(CUtensorMap* map, const void* base, int esize, long nx, long ny, long nz, int bx, int by);
+// elements with box (bx, by, bz).  Returns false if the driver refuses.
+bool make_tensor_map_3d(CUtensorMap* map, const void* base, int esize, long nx, long ny, long nz, int bx, int by,
+                        int bz = 1);
 
 }  // namespace lt

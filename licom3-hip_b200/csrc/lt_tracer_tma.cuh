@@ -28,6 +28,8 @@ constexpr int HN = HQX * HQY;
 struct TracerMaps {
   CUtensorMap at[2], atb[2], ws, uw, vs, akt;
   CUtensorMap vel[4];   // mixed: utf, vtf, utl, vtl (f32) in the continuity march's boxes
+  CUtensorMap atb_own[2];         // FP64: the previous state of a block's own columns
+  CUtensorMap th_at[2], th_akt;   // the state and the mixing in the implicit pass's boxes
 };
 
 template <class VT>
@@ -75,9 +77,11 @@ struct alignas(64) MemberDesc {
   int tma;       // 1: level boxes by TMA; 0: by per-thread copies (row pitch TMA cannot take)
 };
 
-// The FP64 column kernel of the tspas scheme; tma: its level boxes by TMA (else
-// per-thread copies, for row pitches TMA cannot take)
-int launch_tracer_tma64(const Arena& a, const TracerMaps& maps, cudaStream_t s, int grid, bool tma);
+// The FP64 tspas passes over the columns (lt_column_fp64.cu); tma: the
+// implicit pass's level data by TMA boxes (else per-thread copies)
+int launch_column_fp64(const Arena& a, const TracerMaps& maps, bool tma, cudaStream_t s);
+// sets its kernels' shared-memory size on the current device
+int prepare_column_fp64();
 // Batched forms (mixed precision): nmem members, total work items, one
 // persistent column launch of `grid` CTAs with per-CTA scratch of km_max
 // levels; continuity over every member's tiles with tiles of 32 x cby columns.

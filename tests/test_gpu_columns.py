@@ -1,0 +1,78 @@
+"""The FP64 column passes (limiter flags, explicit update, implicit sweep) at
+the sizes where their blocks, patches, level chunks and stages can go wrong,
+bit for bit against the oracle: grids one column short of, at and beyond the
+32 x 4 blocks and 8 x 4 patches, level counts around the chunk and stage
+lengths, row pitches with and without TMA boxes, closed and folded boundaries."""
+import numpy as np
+import pytest
+
+import pyoracle
+
+
+
+CASES = [
+    # nx, ny, km, cyclic, tripole, hypsometry
+    (8, 8, 3, 1, 1, 0),
+    (28, 9, 4, 1, 1, 1),
+    (30, 28, 8, 1, 1, 1),
+    (29, 12, 9, 0, 0, 1),
+    (33, 13, 17, 1, 0, 1),
+    (61, 31, 33, 0, 0, 1),
+    (64, 40, 65, 1, 1, 1),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("diagnostics", [False, True])
+@pytest.mark.parametrize("nx,ny,km,cyclic,tripole,hyp", CASES)
+def test_column_passes_bitexact(lt, nx, ny, km, cyclic, tripole, hyp, diagnostics):
+    syn = lt.Synth(nx, ny, km, seed=17 + nx, forced=1, ew_cyclic=cyclic, tripole=tripole, hypsometry=hyp,
+                   cap_north=0 if tripole else 2, cap_south=2)
+    f = syn.all_fields()
+    dom = lt.TracerDomain(nx, ny, km, syn.params, precision=lt.PREC_FP64, diagnostics=diagnostics,
+                          ew_cyclic=bool(cyclic), tripole=bool(tripole))
+    o = pyoracle.Oracle(nx, ny, km, syn.params, ew_cyclic=cyclic, tripole=tripole)
+    o.load(f)
+    o.sum_order(1)
+    for n in lt.INPUT_FIELDS:
+        dom.set(n, f[n])
+    dom.step(3)
+    dom.sync()
+    o.step(3)
+    for n in ("AT", "ATB", "WS", "NET") + (("AX", "AY", "AZ", "DZ", "PENETRATE", "TEND", "DT_DIFF") if diagnostics else ()):
+        g, r = dom.get(n), o.get(n)
+        assert g.tobytes() == r.tobytes(), (n, float(np.nanmax(np.abs(g - r))), int((g != r).sum()))
+
+
+def test_quotient_by_reciprocal_is_correctly_rounded():
+    """The face divisions' two-step form (a*y, then q - y*(h*q - a) twice, y the
+    rounded reciprocal) equals IEEE division for dividends and divisors of the
+    admitted range, zeros of both signs included: exact rational arithmetic
+    stands in for the fused operations."""
+    from fractions import Fraction
+
+    def fma(a, b, c):
+        v = Fraction(a) * Fraction(b) + Fraction(c)
+        if v == 0:   # the sign of an exact zero: that of the sum of signed zeros, else plus
+            p = a * b if a == 0 or b == 0 else 0.0
+            return p + c if p == 0 and c == 0 else 0.0
+        return v.numerator / v.denominator
+
+    def divide(a, h):
+        y = 1.0 / h
+        q = a * y
+        q = fma(-fma(h, q, -a), y, q)
+        return fma(-fma(h, q, -a), y, q)
+
+    rng = np.random.default_rng(3)
+    n = 20000
+    a = rng.uniform(1.0, 2.0, n) * 2.0 ** rng.integers(-120, 120, n) * rng.choice([-1.0, 1.0], n)
+    h = rng.uniform(1.0, 2.0, n) * 2.0 ** rng.integers(-60, 60, n)
+    # hard cases: mantissas at either end, quotients next to a rounding boundary
+    a[:2000] = np.nextafter(2.0 ** rng.integers(-20, 20, 2000).astype(float), 0.0)
+    h[1000:3000] = np.nextafter(2.0 ** rng.integers(-20, 20, 2000).astype(float), np.inf)
+    a[3000:6000] = h[3000:6000] * np.nextafter(a[3000:6000], np.inf)
+    a[6000], a[6001] = 0.0, -0.0
+    for x, d in zip(a.tolist(), h.tolist()):
+        got, want = divide(x, d), x / d
+        assert got == want and np.signbit(got) == np.signbit(want), (x, d, got, want)
