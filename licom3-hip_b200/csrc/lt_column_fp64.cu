@@ -3,7 +3,7 @@
 // (advection_tracer_2/3 with tracer_del4_1/2, tracer_5..9 and invtrit;
 // tracer.cpp:291-978, 1238-1699).  Compiled with -fmad=false.
 //
-//   k_laplace64   the first Laplacian of atb
+//   k_laplace64   the first Laplacian of atb (on a small grid in k_limit64's launch)
 //   k_limit64     per cell and tracer: the predictor, its masked extrema and
 //                 the limiter flag (one bit)
 //   k_explicit64  per wet cell and tracer: limited fluxes, second
@@ -127,6 +127,15 @@ __device__ __forceinline__ void fill_slot(Slot& sl, uint64_t* bar, const Arena& 
   cp_async_mbar_arrive(bar);
 }
 
+// The first D levels of the block's march on their way.
+template <bool EXPLICIT, int D, class Smem>
+__device__ __forceinline__ void start_levels(Smem& S, const Arena& a, const TracerMaps& maps, bool tma, int x0, int y0,
+                                             int k0, int kend) {
+  const int kdata = min(kend + 1, a.km);
+  for (int L = k0; L < k0 + D && L < kdata; ++L)
+    fill_slot<EXPLICIT>(S.slot[L - k0], &S.bar[L - k0], a, maps, tma, L, x0, y0);
+}
+
 // The block's march over its levels k0 .. kend-1 (top down): the slot of level
 // k+1 has arrived when body(k, slot(k), slot(k+1)) runs, the one of level k-1
 // is refilled D-1 levels ahead.  One barrier per level.  kdata: levels below
@@ -140,7 +149,6 @@ __device__ __forceinline__ void march(Smem& S, const Arena& a, const TracerMaps&
     const int s = slot_of(L);
     fill_slot<EXPLICIT>(S.slot[s], &S.bar[s], a, maps, tma, L, x0, y0);
   };
-  for (int L = k0; L < k0 + D && L < kdata; ++L) fill(L);
   for (int k = k0 - 1; k < kend; ++k) {
     // wait for level k+1 (k0 first)
     const int L = k + 1;
@@ -175,15 +183,20 @@ __device__ __forceinline__ int block_max(Smem& S, int v) {
   return v;
 }
 
-// The block's level-free data and its barriers (before a __syncthreads).
+// The block's level barriers (before a __syncthreads).
 template <int D, class Smem>
-__device__ __forceinline__ void init_block(Smem& S, const Arena& a, bool tma, int x0, int y0, int k0, int kc) {
-  const int tid = threadIdx.x, imt = a.imt, jmt = a.jmt, km = a.km;
-  if (tid == 0) {
+__device__ __forceinline__ void init_bars(Smem& S, bool tma) {
+  if (threadIdx.x == 0) {
     // arrivals per level: the issuing thread's (TMA), or one per copying thread
     for (int s = 0; s < D; ++s) mbar_init(&S.bar[s], tma ? 1 : CT);
     mbar_fence_init();
   }
+}
+
+// The block's level-free data, loaded while its first levels are on their way.
+template <class Smem>
+__device__ __forceinline__ void load_block(Smem& S, const Arena& a, int x0, int y0, int k0, int kc) {
+  const int tid = threadIdx.x, imt = a.imt, jmt = a.jmt, km = a.km;
   for (int m = tid; m < CY * (CX + 1) + (CY + 1) * CX; m += CT) {
     const bool x = m < CY * (CX + 1);
     const int f = x ? m : m - CY * (CX + 1);
@@ -207,6 +220,7 @@ __device__ __forceinline__ void init_block(Smem& S, const Arena& a, bool tma, in
     S.odzt[c] = k < km ? a.odzt[k] : 0.0;
     S.pen[c] = k >= 1 && k <= km ? a.pen[k - 1] : 0.0;
   }
+  __syncthreads();
 }
 
 // ----------------------------------------------------------------- divisions
@@ -283,6 +297,47 @@ __device__ __forceinline__ Kmt5 load_kmt5(const Arena& a, long q) {
   return {a.kmt[q], a.kmt[q - a.imt], a.kmt[q + a.imt], a.kmt[q + 1], a.kmt[q - 1]};
 }
 
+// ---------------------------------------------------------- first Laplacian
+// tracer_del4_1 at the wet cells of levels k0 .. k1-1 of one column: ahf *
+// (masked Laplacian of atb), left in the new previous state (level k at atb's
+// level k+1).  Memory bound: neighbours come through L1.
+__device__ __forceinline__ void laplace_column(const Arena& a, int i, int j, int k0, int k1) {
+  if (!(i >= 1 && i < a.imt - 1 && j >= 1 && j < a.jmt - 1)) return;
+  const int imt = a.imt;
+  const long A = a.A, FB = a.FB;
+  const long q = (long)j * imt + i;
+  const Kmt5 kq = load_kmt5(a, q);
+  k1 = min(k1, kq.c);
+  if (k0 >= k1) return;
+  const double dtn = a.dtn[q], dts = a.dts[q], dte = a.dte[q], dtw = a.dtw[q], ahf = a.ahf[q];
+  const double* __restrict__ atb = a.atb[a.cur];
+  double* __restrict__ d2 = a.atb[a.cur ^ 1];
+#pragma unroll 2
+  for (int k = k0; k < k1; ++k) {
+    const long c0 = (long)(k + 1) * A + q;
+    double h[2] = {0.0, 0.0}, cc = 0.0;
+    auto term = [&](bool there, long at, double cf) {
+      if (there) {
+        h[0] += cf * atb[at];
+        h[1] += cf * atb[FB + at];
+        cc -= cf;
+      }
+    };
+    term(k < kq.n, c0 - imt, dtn);
+    term(k < kq.s, c0 + imt, dts);
+    term(k < kq.e, c0 + 1, dte);
+    term(k < kq.w, c0 - 1, dtw);
+#pragma unroll
+    for (int n = 0; n < 2; ++n) d2[n * FB + c0] = ahf * (cc * atb[n * FB + c0] + h[n]);
+  }
+}
+
+constexpr int kLaplaceLevels = 8;
+__global__ void __launch_bounds__(128) k_laplace64(const __grid_constant__ Arena a) {
+  const int k0 = blockIdx.z * kLaplaceLevels;
+  laplace_column(a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, k0 + kLaplaceLevels);
+}
+
 // The thread's column in the block: warp w is the patch (w % (CX/PX), w / (CX/PX)).
 struct Column {
   int tx, ty;
@@ -298,13 +353,18 @@ __device__ __forceinline__ int patches_y() { return gridDim.y * (CY / PY); }
 
 template <bool DIAG>
 __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps,
-                                                   int kc, int tma) {
+                                                          int kc, int nch, int tma) {
   extern __shared__ __align__(128) unsigned char smem_col[];
   LimitSmem& S = *reinterpret_cast<LimitSmem*>(smem_col);
   const Column col;
   const int tx = col.tx, ty = col.ty;
   const int x0 = blockIdx.x * CX, y0 = blockIdx.y * CY, i = x0 + tx, j = y0 + ty;
   const int km = a.km;
+  if ((int)blockIdx.z >= nch) {   // the Laplacian's blocks
+    const int k = ((int)blockIdx.z - nch) * kc;
+    laplace_column(a, i, j, k, min(k + kc, km));
+    return;
+  }
   const bool ring = i >= 1 && i < a.imt - 1 && j >= 1 && j < a.jmt - 1;
   const long q = (long)j * a.imt + i;
   const int k0 = blockIdx.z * kc;
@@ -314,9 +374,11 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
     kq = load_kmt5(a, q);
     k1 = min(k0 + kc, DIAG ? km : kq.deepest());
   }
-  init_block<kLimitDepth>(S, a, tma != 0, x0, y0, k0, kc);
+  init_bars<kLimitDepth>(S, tma != 0);
   const int kend = block_max(S, k1);
   if (k0 >= kend) return;
+  start_levels<false, kLimitDepth>(S, a, maps, tma != 0, x0, y0, k0, kend);
+  load_block(S, a, x0, y0, k0, kc);
   const double dts = a.p.dts;
   const Faces g = column_faces(S, tx, ty);
   double up[2] = {0.0, 0.0}, cc[2] = {0.0, 0.0};   // levels k-1 and k
@@ -420,42 +482,6 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
   });
 }
 
-// ---------------------------------------------------------- first Laplacian
-// tracer_del4_1 at the wet cells of kc levels: ahf * (masked Laplacian of
-// atb), left in the new previous state (level k at atb's level k+1).  Memory
-// bound: neighbours come through L1.
-__global__ void __launch_bounds__(128) k_laplace64(const __grid_constant__ Arena a, int kc) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (!(i >= 1 && i < a.imt - 1 && j >= 1 && j < a.jmt - 1)) return;
-  const int imt = a.imt;
-  const long A = a.A, FB = a.FB;
-  const long q = (long)j * imt + i;
-  const Kmt5 kq = load_kmt5(a, q);
-  const int k0 = blockIdx.z * kc, k1 = min(k0 + kc, kq.c);
-  if (k0 >= k1) return;
-  const double dtn = a.dtn[q], dts = a.dts[q], dte = a.dte[q], dtw = a.dtw[q], ahf = a.ahf[q];
-  const double* __restrict__ atb = a.atb[a.cur];
-  double* __restrict__ d2 = a.atb[a.cur ^ 1];
-#pragma unroll 2
-  for (int k = k0; k < k1; ++k) {
-    const long c0 = (long)(k + 1) * A + q;
-    double h[2] = {0.0, 0.0}, cc = 0.0;
-    auto term = [&](bool there, long at, double cf) {
-      if (there) {
-        h[0] += cf * atb[at];
-        h[1] += cf * atb[FB + at];
-        cc -= cf;
-      }
-    };
-    term(k < kq.n, c0 - imt, dtn);
-    term(k < kq.s, c0 + imt, dts);
-    term(k < kq.e, c0 + 1, dte);
-    term(k < kq.w, c0 - 1, dtw);
-#pragma unroll
-    for (int n = 0; n < 2; ++n) d2[n * FB + c0] = ahf * (cc * atb[n * FB + c0] + h[n]);
-  }
-}
-
 // ----------------------------------------------------------- explicit update
 // Without diagnostics the wet inner cells; with them every ring cell of every
 // level (ax, ay, az) and every inner cell (dz, penetrate, the value).
@@ -480,23 +506,25 @@ __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_consta
     k1 = min(k0 + kc, DIAG ? km : kq.c);
   }
   const int kz = kq.c;
-  init_block<kExplicitDepth>(S, a, tma != 0, x0, y0, k0, kc);
+  init_bars<kExplicitDepth>(S, tma != 0);
   const int kend = block_max(S, k1);
   if (k0 >= kend) return;
+  start_levels<true, kExplicitDepth>(S, a, maps, tma != 0, x0, y0, k0, kend);
+  load_block(S, a, x0, y0, k0, kc);
   const lt_params& p = a.p;
   const double dts = p.dts;
   const Faces g = column_faces(S, tx, ty);
   double swv = 0.0;
   double up[2] = {0.0, 0.0}, cc[2] = {0.0, 0.0};                         // at of levels k-1, k
-  double bu[2] = {0.0, 0.0}, bc[2] = {0.0, 0.0}, ku[2] = {0.0, 0.0};     // atb of levels k-1, k; akt of level k-1
+  double bc[2] = {0.0, 0.0}, mix[2] = {0.0, 0.0};                        // atb of level k; mixing flux from above it
   if (k0 < k1) {
     swv = inner ? a.swv[q] : 0.0;
     if (k0 > 0)
       for (int n = 0; n < 2; ++n) {
         const long c = (long)(k0 - 1) * A + q;
+        const double* atb = a.atb[a.cur] + n * a.FB + c + A;   // level k0-1
         up[n] = a.at[a.cur][n * F + c];
-        bu[n] = a.atb[a.cur][n * a.FB + c + A];
-        ku[n] = a.akt[n * F + c];
+        mix[n] = a.akt[n * F + c] * (atb[0] - atb[A]) * a.odzt[k0] * (k0 < kz ? 1.0 : 0.0);
       }
   }
   // Flag words of the warp's patch at levels k-1, k, k+1; those of level k+1's
@@ -645,22 +673,20 @@ __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_consta
           }
         }
         // explicit half of the vertical mixing (tracer.cpp:1476-1543)
-        const double bl = last ? 0.0 : D.atb[n][rv], kk = L.akt[n][rv];
+        // (the flux through a face is one expression in both of its cells)
+        const double bl = last ? 0.0 : D.atb[n][rv];
+        const double w1 = mix[n], w2 = last ? 0.0 : L.akt[n][rv] * (bc[n] - bl) * odzt1 * vit_kp1;
         if (k == 0) {
-          const double w1 = kk * (bc[n] - bl) * odzt1 * vit_kp1;
-          tf = tf - odzp * w1 * 0.5;
-          if (DIAG) a.dzd[cg] = -odzp * w1 * 0.5;
+          tf = tf - odzp * w2 * 0.5;
+          if (DIAG) a.dzd[cg] = -odzp * w2 * 0.5;
         } else if (last) {
-          const double w2 = ku[n] * (bu[n] - bc[n]) * odzt * vit_k;
-          tf = tf + odzp * w2 * (1.0 - 0.5);
-          if (DIAG) a.dzd[cg] = odzp * w2 * 0.5;
+          tf = tf + odzp * w1 * (1.0 - 0.5);
+          if (DIAG) a.dzd[cg] = odzp * w1 * 0.5;
         } else {
-          const double w1 = ku[n] * (bu[n] - bc[n]) * odzt * vit_k;
-          const double w2 = kk * (bc[n] - bl) * odzt1 * vit_kp1;
           tf = tf + odzp * (w1 - w2) * 0.5;
           if (DIAG) a.dzd[cg] = odzp * (w1 - w2) * 0.5;
         }
-        ku[n] = kk;
+        mix[n] = w2;
         if (dry) {
           // below the bottom every term is masked: the value stays
           out[cg] = c;
@@ -681,7 +707,6 @@ __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_consta
           }
           out[cg] = c + dts * tf;
         }
-        bu[n] = bc[n];
         bc[n] = bl;
       }
       up[n] = c;
@@ -695,9 +720,10 @@ __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_consta
 
 // Levels per block: a thread keeps the levels above and below in registers,
 // so long chunks read each level once; short ones give a small grid enough
-// blocks (about eight per SM) to fill the GPU.
+// blocks (eight rounds of the resident ones) to fill the GPU evenly although
+// most of a shallow grid's levels are dry.
 static int chunk_levels(long column_blocks, int km) {
-  const long want = 148L * 8;
+  const long want = 148L * kColCtas * 8;
   long chunks = (want + column_blocks - 1) / column_blocks;
   const long most = (km + 3) / 4, least = (km + kChunkMax - 1) / kChunkMax;
   chunks = chunks > most ? most : chunks < least ? least : chunks;
@@ -721,12 +747,19 @@ int launch_column_fp64(const Arena& a, const TracerMaps& maps, bool tma, cudaStr
   if (int rc = launch_assm_dt_restore(a, s)) return rc;
   const unsigned gx = (a.imt + CX - 1) / CX, gy = (a.jmt + CY - 1) / CY;
   const int kc = chunk_levels((long)gx * gy, a.km);
-  const dim3 grid(gx, gy, (a.km + kc - 1) / kc);
-  k_laplace64<<<dim3(gx, (a.jmt + 3) / 4, (a.km + 7) / 8), dim3(CX, 4), 0, s>>>(a, 8);
-  LT_LAUNCHED();
+  const int nch = (a.km + kc - 1) / kc;
+  const dim3 grid(gx, gy, nch);
   const int t = tma ? 1 : 0;
+  // The first Laplacian: on a small grid in the limiter's launch, whose blocks
+  // leave the GPU partly idle (36 x 40 x 55: a launch of 14 us less per step);
+  // on a large one in a kernel of its own, at three times the occupancy.
+  const bool together = (long)gx * gy * nch < 148L * kColCtas * 4;
+  if (!together) {
+    k_laplace64<<<dim3(gx, (a.jmt + 3) / 4, (a.km + kLaplaceLevels - 1) / kLaplaceLevels), dim3(CX, 4), 0, s>>>(a);
+    LT_LAUNCHED();
+  }
   auto kl = a.diagnostics ? k_limit64<true> : k_limit64<false>;
-  kl<<<grid, CT, sizeof(LimitSmem), s>>>(a, maps, kc, t);
+  kl<<<dim3(gx, gy, together ? 2 * nch : nch), CT, sizeof(LimitSmem), s>>>(a, maps, kc, nch, t);
   LT_LAUNCHED();
   auto ke = a.diagnostics ? k_explicit64<true> : k_explicit64<false>;
   ke<<<grid, CT, sizeof(ExplicitSmem), s>>>(a, maps, kc, t);

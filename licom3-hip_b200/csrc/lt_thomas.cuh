@@ -20,7 +20,7 @@ namespace lt {
 
 constexpr int kThX = kThomasX, kThY = kThomasY, kThT = kThX * kThY;
 constexpr int kThLevels = kThomasLevels;
-constexpr int kThStages = 3;
+constexpr int kThStages = 2;
 
 template <class AK>
 struct ThomasSmem {
@@ -92,22 +92,6 @@ __device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& m
   };
   for (int t = 0; t < kThStages && t < stages; ++t) issue(t);
 
-  // the dry levels keep their values (with diagnostics the explicit pass left
-  // them in the new state already): eight levels' loads ahead of their stores
-  if (!DIAG && inner) {
-    for (int k0 = kz; k0 < km; k0 += 8) {
-      double v[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) v[c] = k0 + c < km ? __ldcs(at_in + (long)(k0 + c) * A + q) : 0.0;
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        if (k0 + c < km) {
-          __stcs(at_out + (long)(k0 + c) * A + q, v[c]);
-          __stcs(atb_out + (long)(k0 + c + 1) * A + q, v[c]);
-        }
-    }
-  }
-
   const double dts = a.p.dts;
   const double* __restrict__ odzp = a.odzp;
   const double* __restrict__ odzt = a.odzt;
@@ -157,26 +141,37 @@ __device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& m
   }
   if (!inner) return;
 
-  // substitution, top down: the coefficients of SUB levels loaded together
+  // substitution, top down: the coefficients of SUB levels are loaded while
+  // the SUB levels above are substituted
   const double stf = a.stf_n[n * A + q];
   constexpr int SUB = 8;
   const uint64_t once = l2_evict_first();
   double x = 0.0;
   const int kend = DIAG ? km : kz;
-  for (int k0 = 0; k0 < kend; k0 += SUB) {
-    double ev[SUB], fv[SUB];
+  double ev[SUB], fv[SUB];
+  auto load = [&](int k0) {
 #pragma unroll
     for (int c = 0; c < SUB; ++c) {
       const int k = k0 + c;
       ev[c] = k < kz ? ld_l2(atb_out + (long)(k + 1) * A + q, once) : 0.0;
       fv[c] = k < kend ? ld_l2(at_out + (long)k * A + q, once) : 0.0;
     }
+  };
+  load(0);
+  for (int k0 = 0; k0 < kend; k0 += SUB) {
+    double ec[SUB], fc[SUB];
+#pragma unroll
+    for (int c = 0; c < SUB; ++c) {
+      ec[c] = ev[c];
+      fc[c] = fv[c];
+    }
+    load(k0 + SUB);
 #pragma unroll
     for (int c = 0; c < SUB; ++c) {
       const int k = k0 + c;
       if (k >= kend) break;
-      double v = fv[c];
-      if (k < kz) v = x = ev[c] * (k == 0 ? stf : x) + fv[c];
+      double v = fc[c];
+      if (k < kz) v = x = ec[c] * (k == 0 ? stf : x) + fc[c];
       if (DIAG) {
         const long cg = n * a.F + (long)k * A + q;
         const double vit = k < kz ? 1.0 : 0.0;
@@ -192,10 +187,40 @@ __device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& m
   }
 }
 
+// The dry levels of a block's columns keep their values (with diagnostics the
+// sweep writes them): eight levels' loads ahead of their stores.
+__device__ __forceinline__ void copy_dry(const Arena& a, int x0, int y0, int n) {
+  const int i = x0 + threadIdx.x % kThX, j = y0 + threadIdx.x / kThX;
+  if (!(i >= 2 && i < a.imt - 2 && j >= 2 && j < a.jmt - 2)) return;
+  const long A = a.A, q = (long)j * a.imt + i;
+  const int km = a.km;
+  const double* __restrict__ src = a.at[a.cur] + n * a.F + q;
+  double* __restrict__ at_out = a.at[a.cur ^ 1] + n * a.F + q;
+  double* __restrict__ atb_out = a.atb[a.cur ^ 1] + n * a.FB + A + q;
+  for (int k0 = a.kmt[q]; k0 < km; k0 += 8) {
+    double v[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) v[c] = k0 + c < km ? __ldcs(src + (long)(k0 + c) * A) : 0.0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (k0 + c < km) {
+        __stcs(at_out + (long)(k0 + c) * A, v[c]);
+        __stcs(atb_out + (long)(k0 + c) * A, v[c]);
+      }
+  }
+}
+
 template <class AK, bool DIAG>
 __global__ void __launch_bounds__(kThT) k_thomas(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps,
                                                  int tma) {
-  thomas_block<AK, DIAG>(a, maps, tma != 0, blockIdx.x * kThX, blockIdx.y * kThY, blockIdx.z);
+  // blockIdx.x: the column of tiles and the block's part (the sweep of either
+  // tracer, the dry levels of either tracer): the copying blocks only move
+  // memory, the sweeping ones mostly wait for their chains of divisions, so
+  // the two kinds run side by side
+  constexpr int PARTS = DIAG ? 2 : 4;
+  const int part = blockIdx.x % PARTS, x0 = blockIdx.x / PARTS * kThX, y0 = blockIdx.y * kThY;
+  if (part < 2) thomas_block<AK, DIAG>(a, maps, tma != 0, x0, y0, part);
+  else copy_dry(a, x0, y0, part - 2);
 }
 
 // shared-memory size of the pass on the current device (not inside a capture)
@@ -211,7 +236,7 @@ int prepare_thomas() {
 template <class AK, bool DIAG>
 int launch_thomas(const Arena& a, const TracerMaps& maps, bool tma, cudaStream_t s) {
   const size_t sm = sizeof(ThomasSmem<AK>);
-  k_thomas<AK, DIAG><<<dim3((a.imt + kThX - 1) / kThX, (a.jmt + kThY - 1) / kThY, 2), kThT, sm, s>>>(a, maps, tma ? 1 : 0);
+  k_thomas<AK, DIAG><<<dim3((a.imt + kThX - 1) / kThX * (DIAG ? 2 : 4), (a.jmt + kThY - 1) / kThY), kThT, sm, s>>>(a, maps, tma ? 1 : 0);
   LT_LAUNCHED();
   return LT_OK;
 }
