@@ -42,6 +42,10 @@ constexpr int kThomasX = 32, kThomasY = 4, kThomasLevels = 8;
 constexpr int kMixedContTileY = 4;
 constexpr int kMixedContBoxW = 36;
 
+// a.status word that counts the column work items drawn in a step (cleared by
+// the step's surface kernel)
+constexpr int kTicket = 2;
+
 // Everything the step kernels touch, as raw device pointers (dense
 // [n][k][j][i] layout of the reference, i fastest).
 struct alignas(16) Arena {   // copied into shared memory as 16-byte words
@@ -92,7 +96,7 @@ struct alignas(16) Arena {   // copied into shared memory as 16-byte words
   double *scalars;            // [0] err_norm2 (fw_norm2), [1..2] tracer content, [3..] spare
   double *col_scratch;        // per-slot Thomas sweep storage
   double *fold_save;          // [2][km][2][imt] pre-fold values of the top physical row (diagnostics)
-  int *status;                // [4] device status words
+  int *status;                // [16] device status words: [0] NaN count, [1] timeout, [kTicket] work items drawn
   long col_scratch_slots;
   int nv_scratch;             // values per level per column in col_scratch
   unsigned wait_limit;        // polls of each level wait in the column kernels before giving up

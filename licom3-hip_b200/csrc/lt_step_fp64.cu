@@ -49,6 +49,7 @@ __device__ __forceinline__ double ssh_col(const Arena& a, long q) {
 
 __device__ __forceinline__ void flux_col(const Arena& a, int i, int j, long q, double ssh) {
   const lt_params& p = a.p;
+  if (q == 0) a.status[kTicket] = 0;   // the column kernel's work items start over
   if (i >= 1 && i < a.imt - 1 && j >= 1 && j < a.jmt - 1) {
     if (a.akt) {
       if (a.akt[q] < p.dwndmix) a.akt[q] = p.dwndmix;

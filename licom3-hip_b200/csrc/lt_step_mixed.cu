@@ -468,6 +468,7 @@ struct MxSmem {
   float hw[FN];                        // htw at x faces, hts at y faces
   uint16_t kmt[(MY + 4) * SW64];       // bottom level of the tile's columns and their 2-cell halo
   int wmax[MTH / 32];                  // per-warp maxima of the region's bottom level
+  int next;                            // the CTA's next work item
   uint64_t bar[NSM];
 };
 // followed by the km level constants (dynamic shared memory)
@@ -507,43 +508,46 @@ __device__ __forceinline__ void issue_mx(MxSlot& sl, uint64_t* bar, const Tracer
 // its share of the boxes' elements (zeros outside the domain, as TMA fills)
 // and the slot's mbarrier counts one arrival per thread once its copies have
 // landed.  The slot layout and the waits are the TMA path's.
-constexpr int kF64Elems = 4 * (MY + 4) * SW64;
-constexpr int kWsElems = (MY + 2) * SW, kWkElems = (MY + 3) * SW, kAktElems = TX * MY;
-constexpr int kF32Elems = kWsElems + 2 * kWkElems + 2 * kAktElems;
 __device__ __forceinline__ void copy_level_mx(MxSlot& sl, uint64_t* bar, const Arena& a, int km, int L, int x0,
                                               int y0) {
   const int imt = a.imt, jmt = a.jmt;
-  const long A = a.A, F = a.F, FB = a.FB;
-  for (int e = threadIdx.x; e < kF64Elems; e += MTH) {
-    constexpr int BOX = (MY + 4) * SW64;
-    const int b = e / BOX, r = e % BOX;
-    const int gj = y0 - 2 + r / SW64, gi = x0 - 2 + r % SW64;
-    const bool in = gj >= 0 && gj < jmt && gi >= 0 && gi < imt;
-    const int n = b & 1;
-    const double* src = (b < 2) ? a.at[a.cur] + n * F + (long)L * A : a.atb[a.cur] + n * FB + (long)(L + 1) * A;
-    double* dst = (b < 2) ? sl.at[n] : sl.atb[n];
-    cp_async8z(dst + r, src + (in ? (long)gj * imt + gi : 0), in);
-  }
-  for (int e = threadIdx.x; e < kF32Elems; e += MTH) {
-    const float* base;
-    float* dst;
-    int r, w, gj0, gi0;
-    if (e < kWsElems) {
-      r = e; w = SW; gj0 = y0 - 1; gi0 = x0 - 4; base = a.ws32 + (long)L * A; dst = sl.ws;
-    } else if (e < kWsElems + 2 * kWkElems) {
-      const int q = e - kWsElems, b = q / kWkElems;
-      r = q % kWkElems; w = SW; gj0 = y0 - 2; gi0 = x0 - 4;
-      base = (b == 0 ? a.wkd32 : a.wkb32) + (long)L * A;
-      dst = b == 0 ? sl.wkd : sl.wkb;
-    } else {
-      const int q = e - kWsElems - 2 * kWkElems, n = q / kAktElems;
-      r = q % kAktElems; w = TX; gj0 = y0; gi0 = x0;
-      base = a.akt32 + n * F + (long)L * A;
-      dst = sl.akt[n];
+  const long A = a.A, l = (long)L * A;
+  // each thread's points of the boxes' geometries, every box of a geometry
+  // from one index
+  const double* at = a.at[a.cur] + l;
+  const double* atb = a.atb[a.cur] + l + A;
+#pragma unroll
+  for (int it = 0; it < ((MY + 4) * SW64 + MTH - 1) / MTH; ++it) {
+    const int e = threadIdx.x + it * MTH;
+    if (e < (MY + 4) * SW64) {
+      const int gj = y0 - 2 + e / SW64, gi = x0 - 2 + e % SW64;
+      const bool in = gj >= 0 && gj < jmt && gi >= 0 && gi < imt;
+      const long o = in ? (long)gj * imt + gi : 0;
+      cp_async8z(sl.at[0] + e, at + o, in);
+      cp_async8z(sl.at[1] + e, at + a.F + o, in);
+      cp_async8z(sl.atb[0] + e, atb + o, in);
+      cp_async8z(sl.atb[1] + e, atb + a.FB + o, in);
     }
-    const int gj = gj0 + r / w, gi = gi0 + r % w;
-    const bool in = gj >= 0 && gj < jmt && gi >= 0 && gi < imt;
-    cp_async4z(dst + r, base + (in ? (long)gj * imt + gi : 0), in);
+  }
+#pragma unroll
+  for (int it = 0; it < ((MY + 3) * SW + MTH - 1) / MTH; ++it) {
+    const int e = threadIdx.x + it * MTH;
+    if (e < (MY + 3) * SW) {
+      const int gj = y0 - 2 + e / SW, gi = x0 - 4 + e % SW;
+      const bool in = gj >= 0 && gj < jmt && gi >= 0 && gi < imt;
+      const long o = l + (in ? (long)gj * imt + gi : 0);
+      cp_async4z(sl.wkd + e, a.wkd32 + o, in);
+      cp_async4z(sl.wkb + e, a.wkb32 + o, in);
+      if (e >= SW) cp_async4z(sl.ws + e - SW, a.ws32 + o, in);   // rows from y0-1
+    }
+  }
+  {
+    static_assert(TX * MY == MTH, "one column per thread");
+    const int e = threadIdx.x, gj = y0 + e / TX, gi = x0 + e % TX;
+    const bool in = gj < jmt && gi < imt;
+    const long o = l + (in ? (long)gj * imt + gi : 0);
+    cp_async4z(sl.akt[0] + e, a.akt32 + o, in);
+    cp_async4z(sl.akt[1] + e, a.akt32 + a.F + o, in);
   }
   cp_async_mbar_arrive(bar);
 }
@@ -850,8 +854,8 @@ constexpr int kIssueThread = 4 * TX;
 // drained its boxes, and must return.
 template <bool kLoadsAhead>
 __device__ __forceinline__ bool mixed_item(bool tma, MxSmem& S, const MxLevel* __restrict__ lvs, const Arena& a,
-                                           const TracerMaps& maps, double* scr, int ntx, long tile, uint32_t& par,
-                                           uint32_t& outstanding) {
+                                           const TracerMaps& maps, double* scr, int* ticket, int ntx, long tile,
+                                           uint32_t& par, uint32_t& outstanding) {
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   const int imt = a.imt, jmt = a.jmt, km = a.km;
   const long A = a.A, F = a.F, FB = a.FB;
@@ -902,15 +906,14 @@ __device__ __forceinline__ bool mixed_item(bool tma, MxSmem& S, const MxLevel* _
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < MTH / 32; ++w) kmax = max(kmax, S.wmax[w]);
-  const int ks = min(km - 1, kmax);   // the march's first (deepest) level
-  for (int L = ks; L >= (ks - NSM + 1 > 0 ? ks - NSM + 1 : 0); --L) issue(L, L % NSM);
-  stage_tile<kLoadsAhead>(S, a, x0, y0, dts);
-  if (inner) {
-    // eight levels' loads in flight ahead of their stores
+  // the next item: asked for here or ahead of the substitution, known after it
+  auto draw = [&]() { return tid == kIssueThread ? (int)gridDim.x + atomicAdd(ticket, 1) : 0; };
+  // eight levels' loads in flight ahead of their stores
+  auto copy_below = [&](int k0) {
     const double* __restrict__ at_in = a.at[a.cur];
     double* __restrict__ at_out = a.at[a.cur ^ 1];
     double* __restrict__ atb_out = a.atb[a.cur ^ 1];
-    for (int k0 = ks + 1; k0 < km; k0 += 8) {
+    for (; k0 < km; k0 += 8) {
       double v[8][2];
 #pragma unroll
       for (int c = 0; c < 8; ++c)
@@ -925,7 +928,19 @@ __device__ __forceinline__ bool mixed_item(bool tma, MxSmem& S, const MxLevel* _
             __stcs(atb_out + n * FB + (long)(k0 + c + 1) * A + qo, v[c][n]);
           }
     }
+  };
+  if (kmax == 0) {
+    // no wet column: the tile is copied whole (marching its top level, dry
+    // everywhere, would only copy it too)
+    const int nx = draw();
+    if (inner) copy_below(0);
+    if (tid == kIssueThread) S.next = nx;
+    return true;
   }
+  const int ks = min(km - 1, kmax);   // the march's first (deepest) level
+  for (int L = ks; L >= (ks - NSM + 1 > 0 ? ks - NSM + 1 : 0); --L) issue(L, L % NSM);
+  stage_tile<kLoadsAhead>(S, a, x0, y0, dts);
+  if (inner) copy_below(ks + 1);
 
   const int kz = own ? a.kmt[qo] : 0;
   // The region's extra cells and faces are spread so that no warp carries
@@ -1165,6 +1180,7 @@ __device__ __forceinline__ bool mixed_item(bool tma, MxSmem& S, const MxLevel* _
   // substitution, top down through the wet levels: the elimination
   // coefficients of SUB levels are loaded together ahead of their stores (one
   // scratch round trip per SUB levels)
+  const int nx = draw();
   if (inner) {
     double* at_out = a.at[a.cur ^ 1];
     double* atb_out = a.atb[a.cur ^ 1];
@@ -1193,6 +1209,7 @@ __device__ __forceinline__ bool mixed_item(bool tma, MxSmem& S, const MxLevel* _
       }
     }
   }
+  if (tid == kIssueThread) S.next = nx;
   return true;
 }
 
@@ -1212,6 +1229,10 @@ __device__ __forceinline__ MxLevel* mixed_levels() {
   return reinterpret_cast<MxLevel*>(smem_mx + kMxLevOff);
 }
 
+// Work items beyond the first one of each CTA are drawn from a counter that
+// the step's surface kernel cleared (a.status[kTicket]): tiles differ in depth
+// from land (a copy) to the full column, so a fixed deal left the CTAs with
+// the deepest tiles working alone at the end.
 __global__ void __launch_bounds__(MTH, kMixedCtasPerSm)
     k_tracer_mixed(Arena a, const __grid_constant__ TracerMaps maps, int ntx, long ntiles, int tma) {
   MxSmem& S = mixed_smem_init();
@@ -1219,8 +1240,10 @@ __global__ void __launch_bounds__(MTH, kMixedCtasPerSm)
   stage_levels(lv, a);
   uint32_t par = 0, outstanding = 0;
   double* scr = a.col_scratch + (long)blockIdx.x * a.km * kMixedScratchPerLevel * MTH;
-  for (long w = blockIdx.x; w < ntiles; w += gridDim.x)
-    if (!mixed_item<false>(tma != 0, S, lv, a, maps, scr, ntx, w, par, outstanding)) return;
+  for (long w = blockIdx.x; w < ntiles; w = S.next) {
+    if (!mixed_item<false>(tma != 0, S, lv, a, maps, scr, a.status + kTicket, ntx, w, par, outstanding)) return;
+    __syncthreads();   // S.next is written (and next rewritten after this item's barriers)
+  }
 }
 
 // Several domains (ensemble members, serving requests; any sizes) in one
@@ -1245,7 +1268,8 @@ __global__ void __launch_bounds__(MTH, kMixedCtasPerSm)
   uint32_t par = 0, outstanding = 0;
   double* scr = scratch + (long)blockIdx.x * km_max * kMixedScratchPerLevel * MTH;
   int m = 0, staged = -1;
-  for (long w = blockIdx.x; w < total; w += gridDim.x) {
+  int* const ticket = mem[0].a.status + kTicket;
+  for (long w = blockIdx.x; w < total; w = S.next) {
     while (m + 1 < nmem && mem[m + 1].item0 <= w) ++m;
     const MemberDesc& d = mem[m];
     if (m != staged) {
@@ -1257,7 +1281,8 @@ __global__ void __launch_bounds__(MTH, kMixedCtasPerSm)
       stage_levels(lv, sa);
       staged = m;
     }
-    if (!mixed_item<true>(d.tma != 0, S, lv, sa, d.maps, scr, d.ntx, w - d.item0, par, outstanding)) return;
+    if (!mixed_item<true>(d.tma != 0, S, lv, sa, d.maps, scr, ticket, d.ntx, w - d.item0, par, outstanding)) return;
+    __syncthreads();   // S.next is written
   }
 }
 
