@@ -321,20 +321,21 @@ int run_step(lt_domain* d, cudaEvent_t forcing_ready) {
   // events bound the phases in launch order (LT_PHASE_ORDER)
   auto mark = [&](int ph) { if (ev) cudaEventRecord(ev[ph], s); };
   mark(0);
-  // continuity first: it reads the SSH mean and the velocities, not the
-  // surface forcing
-  if ((rc = launch_ssh(a, s))) return rc;
+  // the continuity reads the SSH mean and the velocities, not the surface
+  // forcing: with a forcing still on its way it comes before the fluxes
+  if ((rc = forcing_ready ? launch_ssh(a, s) : launch_surface(a, s))) return rc;
   if (a.precision == LT_PREC_MIXED) rc = launch_continuity_mixed(a, d->maps, d->use_tma, s);
   else rc = launch_continuity_fp64(a, s);
   if (rc) return rc;
   mark(1);
-  if (forcing_ready) LT_CUDA_OK(cudaStreamWaitEvent(s, forcing_ready, 0));
-  if ((rc = launch_surface_fluxes(a, s))) return rc;
+  if (forcing_ready) {
+    LT_CUDA_OK(cudaStreamWaitEvent(s, forcing_ready, 0));
+    if ((rc = launch_surface_fluxes(a, s))) return rc;
+  }
   mark(2);
   if ((rc = launch_interior_sum_sss(a, s))) return rc;
   mark(3);
-  if ((rc = launch_halo_r8(a.net, 2, a.imt, a.jmt, a.ew_cyclic, a.tripole, s))) return rc;
-  mark(4);
+  mark(4);   // net's ghost cells are filled with the state's
   if (a.precision == LT_PREC_MIXED) {
     if ((rc = launch_tracer_tma_mixed(a, d->maps, d->use_tma, s, d->tma_grid))) return rc;
   } else if (a.p.adv_tracer == LT_ADV_TSPAS) {

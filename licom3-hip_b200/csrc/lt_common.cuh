@@ -45,6 +45,8 @@ constexpr int kMixedContBoxW = 36;
 // a.status word that counts the column work items drawn in a step (cleared by
 // the step's surface kernel)
 constexpr int kTicket = 2;
+// a.status word that counts the SSS norm's finished blocks
+constexpr int kSssDone = 3;
 
 // Everything the step kernels touch, as raw device pointers (dense
 // [n][k][j][i] layout of the reference, i fastest).
@@ -135,6 +137,7 @@ void set_error(const char* fmt, ...);
 // continuity needs, and the surface fluxes, net and the mixing floor (which
 // read stf_ssh and the forcing)
 int launch_ssh(const Arena& a, cudaStream_t s);
+int launch_surface(const Arena& a, cudaStream_t s);   // both parts
 int launch_surface_fluxes(const Arena& a, cudaStream_t s);
 int launch_continuity_fp64(const Arena& a, cudaStream_t s);
 int launch_tracer_fp64(const Arena& a, cudaStream_t s, int slots);

@@ -113,6 +113,11 @@ __global__ void k_surface_fluxes(Arena a) {
   flux_col(a, i, j, q, a.stf_ssh[q]);
 }
 
+// both, where the forcing is already there
+__global__ void k_surface(const __grid_constant__ Arena a) {
+  surface_col(a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
+}
+
 // every member's columns in one launch: blockIdx.z is the member
 __global__ void k_surface_batch(const MemberDesc* __restrict__ mem) {
   surface_col(mem[blockIdx.z].a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
@@ -161,8 +166,43 @@ struct SssTerm {
   }
 };
 
-__global__ void k_finish_sss(double* scalars, const double* sum, double area_t) {
-  scalars[0] = -sum[0] / area_t;
+// The whole sum and fw_norm2 in one launch: the last block to finish its part
+// (counted in a.status[kSssDone], which it clears again) takes the tree's
+// further passes over the block sums, which are few: the same fixed tree, so
+// the same bits, without a launch per pass, a copy of the result and a launch
+// to finish it (about 12 us of a small grid's step).
+struct PartTerm {   // block sums of other blocks of this launch: past L1
+  const double* x;
+  __device__ double operator()(long m) const { return __ldcg(x + m); }
+};
+__global__ void k_sss_norm(const __grid_constant__ Arena a) {
+  long n = (long)a.nx * a.ny, nb = gridDim.x;
+  tree_block(SssTerm{a.tarea, a.net + a.A, a.kmt, a.nx, a.imt}, n, a.red_part, blockIdx.x);
+  __shared__ int last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(a.status + kSssDone, 1) == (int)nb - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  double* cur = a.red_part;
+  while (nb > 1) {
+    __threadfence();
+    double* nxt = cur + nb;
+    n = nb;
+    nb = (n + 2 * RB - 1) / (2 * RB);
+    for (long blk = 0; blk < nb; ++blk) {
+      tree_block(PartTerm{cur}, n, nxt, blk);
+      __syncthreads();   // the block's sums and its shared array are free again
+    }
+    cur = nxt;
+  }
+  if (threadIdx.x == 0) {
+    const double sum = *cur;
+    a.scalars[4] = sum;
+    a.scalars[0] = -sum / a.p.area_t;
+    a.status[kSssDone] = 0;
+  }
 }
 
 // The same tree for every member of a batch, pass by pass: pass 0 sums the
@@ -257,9 +297,8 @@ __device__ __forceinline__ bool halo_part(long nc, int imt, int tripole, int par
   return m0 < m1;
 }
 
-// part blockIdx.x of level blockIdx.y
-__global__ void k_halo_r8(double* f, int imt, int jmt, int ew_cyclic, int tripole) {
-  double* lvl = f + (long)blockIdx.y * imt * jmt;
+// part blockIdx.x of one level
+__device__ __forceinline__ void halo_r8_part(double* lvl, int imt, int jmt, int ew_cyclic, int tripole) {
   HaloCells hc{imt, jmt, tripole};
   long m0, m1;
   if (!halo_part(hc.count(), imt, tripole, blockIdx.x, m0, m1)) return;
@@ -275,6 +314,11 @@ __global__ void k_halo_r8(double* f, int imt, int jmt, int ew_cyclic, int tripol
     double v;
     if (halo_cell_value(lvl, top, j, i, imt, jmt, ew_cyclic, tripole, v)) lvl[(long)j * imt + i] = v;
   }
+}
+
+// part blockIdx.x of level blockIdx.y
+__global__ void k_halo_r8(double* f, int imt, int jmt, int ew_cyclic, int tripole) {
+  halo_r8_part(f + (long)blockIdx.y * imt * jmt, imt, jmt, ew_cyclic, tripole);
 }
 
 // net (both tracers) of every member: blockIdx.x the level, blockIdx.y the member
@@ -835,10 +879,16 @@ __global__ void k_halo_state(Arena a, int n) {
 
 // Without diagnostics the two tracers' ghost fills are independent: one
 // launch, part blockIdx.x (as k_halo_r8) of level blockIdx.y of tracer
-// blockIdx.z, the same values as halo_state_level<false>.
-__global__ void k_halo_state_parts(Arena a) {
+// blockIdx.z, the same values as halo_state_level<false>; blockIdx.z 2 is the
+// surface flux net (both tracers), whose ghost cells nothing reads within the
+// step.
+__global__ void k_halo_state_parts(const __grid_constant__ Arena a) {
   const int n = blockIdx.z, k = blockIdx.y;
   const int imt = a.imt, jmt = a.jmt;
+  if (n == 2) {
+    if (k < 2) halo_r8_part(a.net + (long)k * a.A, imt, jmt, a.ew_cyclic, a.tripole);
+    return;
+  }
   HaloCells hc{imt, jmt, a.tripole};
   long m0, m1;
   if (!halo_part(hc.count(), imt, a.tripole, blockIdx.x, m0, m1)) return;
@@ -897,6 +947,13 @@ int launch_ssh(const Arena& a, cudaStream_t s) {
   return LT_OK;
 }
 
+int launch_surface(const Arena& a, cudaStream_t s) {
+  dim3 b(32, 8), g((a.imt + 31) / 32, (a.jmt + 7) / 8);
+  k_surface<<<g, b, 0, s>>>(a);
+  LT_LAUNCHED();
+  return LT_OK;
+}
+
 int launch_surface_fluxes(const Arena& a, cudaStream_t s) {
   dim3 b(32, 8), g((a.imt + 31) / 32, (a.jmt + 7) / 8);
   k_surface_fluxes<<<g, b, 0, s>>>(a);
@@ -914,10 +971,8 @@ size_t tree_sum_part_elems(long n) {
 }
 
 int launch_interior_sum_sss(const Arena& a, cudaStream_t s) {
-  SssTerm t{a.tarea, a.net + a.A, a.kmt, a.nx, a.imt};
-  int rc = tree_sum(t, (long)a.nx * a.ny, a.red_part, a.scalars + 4, s);
-  if (rc) return rc;
-  k_finish_sss<<<1, 1, 0, s>>>(a.scalars, a.scalars + 4, a.p.area_t);
+  const long n = (long)a.nx * a.ny, nb = (n + 2 * RB - 1) / (2 * RB);
+  k_sss_norm<<<(unsigned)nb, RB, 0, s>>>(a);
   LT_LAUNCHED();
   return LT_OK;
 }
@@ -975,14 +1030,14 @@ int launch_tracer_fp64(const Arena& a, cudaStream_t s, int slots) {
 
 int launch_halo_state(const Arena& a, cudaStream_t s) {
   if (!a.diagnostics) {
-    k_halo_state_parts<<<dim3(kHaloParts, a.km, 2), 256, a.imt * sizeof(double), s>>>(a);
+    k_halo_state_parts<<<dim3(kHaloParts, a.km, 3), 256, a.imt * sizeof(double), s>>>(a);
     LT_LAUNCHED();
     return LT_OK;
   }
+  if (int rc = launch_halo_r8(a.net, 2, a.imt, a.jmt, a.ew_cyclic, a.tripole, s)) return rc;
   // with diagnostics, salinity's dt_diff reads temperature's new ghost values
   for (int n = 0; n < 2; ++n) {
-    if (a.diagnostics) k_halo_state<true><<<a.km, 256, a.imt * sizeof(double), s>>>(a, n);
-    else k_halo_state<false><<<a.km, 256, a.imt * sizeof(double), s>>>(a, n);
+    k_halo_state<true><<<a.km, 256, a.imt * sizeof(double), s>>>(a, n);
     LT_LAUNCHED();
   }
   return LT_OK;
