@@ -140,6 +140,12 @@ int launch_ssh(const Arena& a, cudaStream_t s);
 int launch_surface(const Arena& a, cudaStream_t s);   // both parts
 int launch_surface_fluxes(const Arena& a, cudaStream_t s);
 int launch_continuity_fp64(const Arena& a, cudaStream_t s);
+// Which form of the continuity: below this many 32 x 8 tiles (half an SM each)
+// every level at once, where the march would be a chain of km levels on a few
+// SMs (36 x 40 x 55, FP64: 60 us per step against 28 us); from there on the
+// march, which reads and writes each field once (360 x 218 x 30: 60 against
+// 79 us in FP64, 39 against 60 us in mixed precision).
+inline bool continuity_by_levels(long tiles) { return tiles < 74; }
 int launch_tracer_fp64(const Arena& a, cudaStream_t s, int slots);
 int launch_assm_dt_restore(const Arena& a, cudaStream_t s);
 int launch_halo_state(const Arena& a, cudaStream_t s);

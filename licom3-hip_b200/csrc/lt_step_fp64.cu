@@ -511,6 +511,118 @@ __global__ void __launch_bounds__(32 * BY) k_cont_march64(Arena a) {
   }
 }
 
+// The same continuity for grids whose tiles do not fill the GPU, where the
+// march is a chain of km levels on a few SMs: first every level at once
+// (k_cont_levels64: face transports, scaled velocities, divergence; the
+// neighbours' velocities come through L1), then the two sums of each column
+// (k_cont_columns64).  Same expressions in the same order.
+// Step at 36 x 40 x 55 and 360 x 218 x 30: see launch_continuity_fp64.
+constexpr int kContChunk = 4;   // levels per thread of k_cont_levels64
+__global__ void __launch_bounds__(256) k_cont_levels64(const __grid_constant__ Arena a) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+  const int imt = a.imt, jmt = a.jmt;
+  if (i >= imt || j >= jmt) return;
+  const long A = a.A, q = q2(j, i, imt);
+  const lt_params& p = a.p;
+  const bool north = j >= 1, east = i < imt - 1;
+  // the free-surface factor at U point (uj, ui), 0 where uk, vk are zero
+  auto factor = [&](int uj, int ui) {
+    if (!(uj >= 0 && uj < jmt - 1 && ui >= 1 && ui < imt)) return 0.0;
+    const long c = q2(uj, ui, imt);
+    const double work = a.au0[c] * a.stf_ssh[c] + a.aus[c] * a.stf_ssh[c + imt] + a.auw[c] * a.stf_ssh[c - 1] +
+                        a.ausw[c] * a.stf_ssh[c + imt - 1];
+    return 1.0 + work * a.ohbu[c];
+  };
+  const bool div = north && east;
+  const int kz = a.kmt[q];
+  const double f0 = factor(j, i), fn = factor(j - 1, i), f1 = factor(j, i + 1), fn1 = factor(j - 1, i + 1);
+  const double htw_o = a.htw[q], hts_o = a.hts[q];
+  const double htw_e = east ? a.htw[q + 1] : 0.0, hts_n = north ? a.hts[q - imt] : 0.0;
+  const bool flux = p.adv_tracer == LT_ADV_FLUX;
+  const double dyu_o = flux ? a.dyu[q] : 0.0, dyu_n = flux && north ? a.dyu[q - imt] : 0.0;
+  const double dxu_o = flux ? a.dxu[q] : 0.0, dxu_e = flux && east ? a.dxu[q + 1] : 0.0;
+  const double trr = a.tarea_r[q];
+  const double* __restrict__ utf = a.utf;
+  const double* __restrict__ utl = a.utl;
+  const double* __restrict__ vtf = a.vtf;
+  const double* __restrict__ vtl = a.vtl;
+  const int k0 = blockIdx.z * kContChunk;
+#pragma unroll
+  for (int d = 0; d < kContChunk; ++d) {
+    const int k = k0 + d;
+    if (k >= a.km) break;
+    const long c = (long)k * A + q;
+    // mean velocities of the four U points: here, north, east, north-east
+    // (zero outside the domain)
+    double wd[4], wb[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const bool in = (!(m & 1) || north) && (!(m & 2) || east);
+      const long u = c - (m & 1 ? imt : 0) + (m & 2 ? 1 : 0);
+      wd[m] = in ? 0.5 * (utf[u] * p.oncc) + 0.5 * utl[u] : 0.0;
+      wb[m] = in ? 0.5 * (vtf[u] * p.oncc) + 0.5 * vtl[u] : 0.0;
+    }
+    a.utf_out[c] = utf[c] * p.oncc;
+    a.vtf_out[c] = vtf[c] * p.oncc;
+    if (flux) {
+      if (j >= 1 && j < jmt - 1) a.uwf[c] = (wd[1] * dyu_n + wd[0] * dyu_o) * 0.25;
+      if (i >= 1 && i < imt - 1) a.vsf[c] = (wb[0] * dxu_o + wb[2] * dxu_e) * 0.25;
+    } else {
+      if (j >= 1 && j < jmt - 1) a.uwf[c] = (wd[1] + wd[0]) * htw_o * 0.25;
+      if (i >= 1 && i < imt - 1) a.vsf[c] = (wb[0] + wb[2]) * hts_o * 0.25;
+    }
+    double wka = 0.0;
+    if (div && k <= kz - 1) {
+      auto times = [](double fac, double w) { return fac == 0.0 ? 0.0 : fac * w; };
+      const double uk0 = times(f0, wd[0]), ukn = times(fn, wd[1]), uk1 = times(f1, wd[2]), ukn1 = times(fn1, wd[3]);
+      const double vk0 = times(f0, wb[0]), vkn = times(fn, wb[1]), vk1 = times(f1, wb[2]), vkn1 = times(fn1, wb[3]);
+      const double e = (uk1 + ukn1) * htw_e;
+      const double w = (uk0 + ukn) * htw_o;
+      const double s = (vk1 + vk0) * hts_o;
+      const double n = (vkn1 + vkn) * hts_n;
+      wka = 0.5 * (e - w + s - n) * trr;
+    }
+    a.wka[c] = wka;
+  }
+}
+
+__global__ void __launch_bounds__(128) k_cont_columns64(const __grid_constant__ Arena a) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
+  const int imt = a.imt, km = a.km;
+  if (!(j >= 1 && j < a.jmt - 1 && i >= 1 && i < imt - 1)) return;
+  const long A = a.A, q = q2(j, i, imt);
+  const int kz = a.kmt[q];
+  const double* __restrict__ wka = a.wka + q;
+  const double* __restrict__ dzp = a.dzp;
+  constexpr int CH = 8;
+  double W = 0.0;
+  for (int k0 = 0; k0 < km; k0 += CH) {
+    double w[CH];
+#pragma unroll
+    for (int c = 0; c < CH; ++c) w[c] = k0 + c < km ? wka[(long)(k0 + c) * A] : 0.0;
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+      if (k0 + c < km) W = W - dzp[k0 + c] * w[c] * (k0 + c < kz ? 1.0 : 0.0);
+  }
+  const double ohbt = a.ohbt[q];
+  const double fac = 1.0 / (1.0 + a.stf_ssh[q] * ohbt);
+  double wsp = a.ws[q];
+  double* __restrict__ ws = a.ws + q;
+  for (int k0 = 1; k0 < km; k0 += CH) {
+    double w[CH];
+#pragma unroll
+    for (int c = 0; c < CH; ++c) w[c] = k0 + c < km ? wka[(long)(k0 + c - 1) * A] : 0.0;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int k = k0 + c;
+      if (k >= km) break;
+      const double raw = (k < kz ? 1.0 : 0.0) * (wsp + dzp[k - 1] * (W * ohbt + w[c]));
+      ws[(long)k * A] = raw * fac;
+      wsp = raw;
+    }
+  }
+}
+
 // ------------------------------------------- plain-load march (centred, flux)
 // The column march of the centred and flux advection schemes (no predictor
 // or limiter), with each level's region loaded by plain loads.
@@ -990,6 +1102,13 @@ int launch_halo_r8(double* f, int nz, int imt, int jmt, int ew_cyclic, int tripo
 int launch_continuity_fp64(const Arena& a, cudaStream_t s) {
   constexpr int BY = kCont64TileY;
   dim3 b(32, BY), g((a.imt + 31) / 32, (a.jmt + BY - 1) / BY);
+  if (continuity_by_levels((long)g.x * g.y)) {
+    k_cont_levels64<<<dim3(g.x, g.y, (a.km + kContChunk - 1) / kContChunk), b, 0, s>>>(a);
+    LT_LAUNCHED();
+    k_cont_columns64<<<dim3(g.x, (a.jmt + 3) / 4), dim3(32, 4), 0, s>>>(a);
+    LT_LAUNCHED();
+    return LT_OK;
+  }
   k_cont_march64<BY><<<g, b, 0, s>>>(a);
   LT_LAUNCHED();
   return LT_OK;

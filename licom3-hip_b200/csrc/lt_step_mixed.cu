@@ -369,6 +369,102 @@ __global__ void __launch_bounds__(CBX * kContTileY) k_cont_march32(Arena a) {
   cont_tile<kContTileY>(a, blockIdx.x, blockIdx.y);
 }
 
+// The same continuity for grids whose tiles do not fill the GPU (as
+// k_cont_levels64 and k_cont_columns64): every level at once, the divergence
+// in f64 in the new state's buffer, which the step has not written yet, then
+// the sums of each column, with the roundings of the march's parked sums.
+constexpr int kContChunk32 = 4;
+__global__ void __launch_bounds__(256) k_cont_levels32(const __grid_constant__ Arena a) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+  const int imt = a.imt, jmt = a.jmt;
+  if (i >= imt || j >= jmt) return;
+  const long A = a.A, q = (long)j * imt + i;
+  const float oncc = (float)a.p.oncc;
+  const bool north = j >= 1, east = i < imt - 1;
+  auto fm1_at = [&](int uj, int ui) {
+    float fm1 = -1.f;
+    if (uj >= 0 && uj < jmt - 1 && ui >= 1 && ui < imt) {
+      const long c = (long)uj * imt + ui;
+      const double work = a.au0[c] * a.stf_ssh[c] + a.aus[c] * a.stf_ssh[c + imt] + a.auw[c] * a.stf_ssh[c - 1] +
+                          a.ausw[c] * a.stf_ssh[c + imt - 1];
+      fm1 = (float)(work * a.ohbu[c]);
+    }
+    return fm1;
+  };
+  const bool col = j >= 1 && j < jmt - 1 && i >= 1 && i < imt - 1;
+  const int kz = a.kmt[q];
+  const ContCell g{a.htw[q], east ? a.htw[q + 1] : 0.0, a.hts[q], north ? a.hts[q - imt] : 0.0,
+                   north && east ? a.tarea_r[q] : 0.0};
+  const float f0 = fm1_at(j, i), fn = fm1_at(j - 1, i), f1 = fm1_at(j, i + 1), fn1 = fm1_at(j - 1, i + 1);
+  const float* __restrict__ utf = a.utf32;
+  const float* __restrict__ utl = a.utl32;
+  const float* __restrict__ vtf = a.vtf32;
+  const float* __restrict__ vtl = a.vtl32;
+  double* __restrict__ wka = a.at[a.cur ^ 1];
+  const int k0 = blockIdx.z * kContChunk32;
+#pragma unroll
+  for (int d = 0; d < kContChunk32; ++d) {
+    const int k = k0 + d;
+    if (k >= a.km) break;
+    const long c = (long)k * A + q;
+    float wd[4], wb[4];   // the U points here, north, east, north-east
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const bool in = (!(m & 1) || north) && (!(m & 2) || east);
+      const long u = c - (m & 1 ? imt : 0) + (m & 2 ? 1 : 0);
+      wd[m] = in ? u_mean32(utf[u], utl[u], oncc) : 0.f;
+      wb[m] = in ? u_mean32(vtf[u], vtl[u], oncc) : 0.f;
+    }
+    a.utf_out32[c] = utf[c] * oncc;
+    a.vtf_out32[c] = vtf[c] * oncc;
+    a.wkd32[c] = wd[0];
+    a.wkb32[c] = wb[0];
+    if (col && k < kz)
+      wka[c] = cont_wka(g, wd[1], wd[0], wd[3], wd[2], wb[1], wb[0], wb[3], wb[2], fn, f0, fn1, f1);
+  }
+}
+
+__global__ void __launch_bounds__(128) k_cont_columns32(const __grid_constant__ Arena a) {
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
+  const int imt = a.imt, km = a.km;
+  if (!(j >= 1 && j < a.jmt - 1 && i >= 1 && i < imt - 1)) return;
+  const long A = a.A, q = (long)j * imt + i;
+  const int kz = a.kmt[q];
+  const double* __restrict__ wka = a.at[a.cur ^ 1] + q;
+  const double* __restrict__ dzp = a.dzp;
+  constexpr int CH = 8;
+  double P = 0.0;
+  for (int k0 = 0; k0 < kz; k0 += CH) {
+    double w[CH];
+#pragma unroll
+    for (int c = 0; c < CH; ++c) w[c] = k0 + c < kz ? wka[(long)(k0 + c) * A] : 0.0;
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+      if (k0 + c < kz) P = __fma_rn(dzp[k0 + c], w[c], P);
+  }
+  const double ohbt = a.ohbt[q];
+  const double fac = 1.0 / (1.0 + a.stf_ssh[q] * ohbt);
+  const double W = -P;
+  float* __restrict__ ws = a.ws32 + q;
+  const double ws0 = ws[0];
+  double Z = 0.0;
+  P = 0.0;
+  for (int k0 = 1; k0 < km; k0 += CH) {
+    double w[CH];
+#pragma unroll
+    for (int c = 0; c < CH; ++c) w[c] = k0 + c - 1 < kz ? wka[(long)(k0 + c - 1) * A] : 0.0;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int k = k0 + c;
+      if (k >= km) break;
+      if (k - 1 < kz) P = __fma_rn(dzp[k - 1], w[c], P);
+      Z = __dadd_rn(Z, dzp[k - 1]);
+      ws[(long)k * A] =
+          (k < kz) ? (float)__dmul_rn(fac, __dadd_rn(__fma_rn(__dmul_rn(W, ohbt), Z, ws0), (double)(float)P)) : 0.f;
+    }
+  }
+}
+
 // every member's tiles in one launch: blockIdx.z is the member; tiles beyond
 // a smaller member's grid leave at once
 // (the member's arena is read from a shared-memory copy, which the march's
@@ -1335,6 +1431,14 @@ int launch_continuity_mixed_batch(const MemberDesc* mem, int nmem, int max_imt, 
 
 int launch_continuity_mixed(const Arena& a, const TracerMaps& maps, bool tma, cudaStream_t s) {
   dim3 b(CBX, kContTileY), g((a.imt + CBX - 1) / CBX, (a.jmt + kContTileY - 1) / kContTileY);
+  const unsigned rows = (a.jmt + 7) / 8;
+  if (continuity_by_levels((long)g.x * rows)) {
+    k_cont_levels32<<<dim3(g.x, rows, (a.km + kContChunk32 - 1) / kContChunk32), dim3(32, 8), 0, s>>>(a);
+    LT_LAUNCHED();
+    k_cont_columns32<<<dim3(g.x, (a.jmt + 3) / 4), dim3(32, 4), 0, s>>>(a);
+    LT_LAUNCHED();
+    return LT_OK;
+  }
   if (tma) {
     static int attr_dev = -1;
     int dev = 0;
