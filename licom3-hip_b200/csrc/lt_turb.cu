@@ -17,6 +17,9 @@
 //      neighbouring levels it looks at in registers, and the diffusivities
 //      written as soon as a level is done (level 0 last: the wind-mixing floor
 //      applies to it once the column is complete).
+#include <cmath>
+#include <new>
+#include <vector>
 #include "lt_common.cuh"
 #include "lt_domain.h"
 
@@ -37,17 +40,17 @@ constexpr double kBackTidal = 1.0e-6, kMaxTidal = 1.0e-2, kMixingEf = 0.20, kLoc
 constexpr double kEpson2 = 0.288e0, kEplatMin = 7.0e-2, kS2min = 1.0e-14;
 
 __device__ __forceinline__ double sgn(double x, double y) { return y >= 0.0 ? fabs(x) : -fabs(x); }
-__device__ __forceinline__ int sgn_i(int x, int y) { return y >= 0 ? abs(x) : -abs(x); }
 
-// Values the reference recomputes at every call from constants: atan(1),
-// the denominator of eplatidepend_fun, the logarithms of the geometric table
-// parts.  Computed once per thread with the same functions, so the bits are
-// those of the per-call evaluation.
+// Values the reference recomputes at every call from constants, formed once
+// per launch on the host.
 struct TurbConst {
   double pi4;               // atan(1.0)
   double eplat_den;         // wavelat(f_30, an0)
-  double log_gm, log_rri;   // 2-D tables: log(rib[mt + mt0]), log(rri)
-  double log_gm1, log_rnd;  // zero-shear table: log(and2on2a1[mt + mt0]), log(rnd2on2)
+  double inv_ncc;           // 1/ncc (0: divide)
+  double inv_dth;           // 1/deltheta_r
+  double inv_dri, inv_da;   // 1/dri, 1/dand2on2
+  float log2_gm, per_log2;     // 2-D tables: log2(rib[mt + mt0]), 1/log2(rri)
+  float log2_gm1, per_log21;   // zero-shear table
 };
 
 // wavelat / eplatidepend_fun (readyc.cpp:880-896)
@@ -56,172 +59,163 @@ __device__ __forceinline__ double eplat(const TurbConst& C, double f, double an)
   return anum / C.eplat_den;
 }
 
-// Table index of x on an "expabs" grid (linear spacing delta up to
-// grid[mt + mt0], geometric ratio rat beyond), as interp1d_expabs and
-// interp2d_expabs find it (readyc.cpp:922-941, 1014-1031).  Sets l0, l1.
-__device__ __forceinline__ void expabs_index(double x, const double* g, double delta, double log_gm, double log_rat,
-                                             int& l0, int& l1) {
-  const double gm = g[MT + MT0], gmax = g[2 * MT];
-  if (fabs(x) >= gm && fabs(x) >= gmax) {
-    l0 = (int)sgn((double)MT, x);
-    l1 = l0;
-    return;
-  }
-  if (fabs(x) < gm) {
-    l1 = (int)(x / delta) + (int)sgn(1.0, x);
-  } else {
-    const double ti = sgn((double)MT0 + ((log(fabs(x)) - log_gm) / log_rat), x);
-    l1 = (int)ti + (int)sgn(1.0, x);
-  }
-  // a rounding of the logarithms could put x's index one past the table
-  // end, where the reference reads beyond its array; stay inside
-  l1 = max(-MT, min(MT, l1));
-  if (fabs(g[MT + l1]) < fabs(x)) l1 += sgn_i(1, l1);
-  else if (fabs(g[MT + l1 - sgn_i(1, l1)]) > fabs(x)) l1 += -sgn_i(1, l1);
-  l0 = l1 - (int)sgn(1.0, x);
+// Indices (offset by MT) of the entries that bracket x on an "expabs" grid
+// (linear spacing delta up to grid[mt + mt0] = gm, geometric beyond), which
+// interp1d_expabs and interp2d_expabs find from a quotient or a logarithm and
+// a correction (readyc.cpp:922-941, 1014-1031).  Here the first guess is a
+// single-precision one and the grid itself decides: lo towards zero, an entry
+// that x meets counts as lo.
+struct Bracket {
+  int lo, hi;
+};
+__device__ __forceinline__ Bracket bracket(double x, const double* __restrict__ g, double gm, double inv_delta,
+                                           float log2_gm, float per_log2) {
+  const double ax = fabs(x);
+  const int s = x >= 0.0 ? 1 : -1;
+  int m;
+  if (ax < gm) m = 1 + (int)(ax * inv_delta);
+  else m = 1 + MT0 + (int)((__log2f((float)ax) - log2_gm) * per_log2);
+  m = max(1, min(MT, m));
+  while (m < MT && fabs(g[MT + s * m]) <= ax) ++m;
+  while (m > 1 && fabs(g[MT + s * (m - 1)]) > ax) --m;
+  return {MT + s * (m - 1), MT + s * m};
 }
 
-// interp1d_expabs (readyc.cpp:915-973): outputs left as they were when x
-// falls outside the bracketing entries
-__device__ void interp1d(double x, const TurbTabDev& T, const TurbConst& C, double& slq2, double& sm, double& sh,
-                         double& ss) {
+// interp1d_expabs (readyc.cpp:915-973): false, outputs left as they were, when
+// x falls outside the bracketing entries
+__device__ __noinline__ bool interp1d(double x, const TurbTabDev& T, const TurbConst& C, double out[4]) {
   const double* x1 = T.and2on2a1;
   if (x > x1[2 * MT]) x = x1[2 * MT];
   else if (x < x1[0]) x = x1[0];
-  int l0, l1;
   const double gm = x1[MT + MT0], gmax = x1[2 * MT];
-  if (fabs(x) >= gm && fabs(x) >= gmax) {
-    l0 = (int)sgn((double)MT, x);
-    l1 = l0;
-  } else {
-    expabs_index(x, x1, T.dand2on2, C.log_gm1, C.log_rnd, l0, l1);
-    if (fabs(x) <= 0.0e0) l1 = 1;
+  Bracket b;
+  if (fabs(x) >= gm && fabs(x) >= gmax) b.lo = b.hi = x >= 0.0 ? 2 * MT : 0;
+  else b = bracket(x, x1, gm, C.inv_da, C.log2_gm1, C.per_log21);
+  const double x0 = x1[b.lo], xh = x1[b.hi];
+  if ((x > 0.0e0 && (x < x0 || x > xh)) || (x < 0.0e0 && (x > x0 || x < xh))) return false;
+  const double dta = xh - x0;
+  const double dx = x - x0;
+  const double* tab[4] = {T.amtaun2a1, T.sma1, T.sha1, T.ssa1};
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const double v = tab[m][b.lo];
+    out[m] = v + (b.hi == b.lo ? 0.0e0 : (tab[m][b.hi] - v) / dta) * dx;
   }
-  if ((x > 0.0e0 && (x < x1[MT + l0] || x > x1[MT + l1])) || (x < 0.0e0 && (x > x1[MT + l0] || x < x1[MT + l1])))
-    return;
-  const double dta = x1[MT + l1] - x1[MT + l0];
-  const double dx = x - x1[MT + l0];
-  double d_slq2, d_sm, d_sh, d_ss;
-  if (l1 == l0) {
-    d_slq2 = d_sm = d_sh = d_ss = 0.0e0;
-  } else {
-    d_slq2 = (T.amtaun2a1[MT + l1] - T.amtaun2a1[MT + l0]) / dta;
-    d_sm = (T.sma1[MT + l1] - T.sma1[MT + l0]) / dta;
-    d_sh = (T.sha1[MT + l1] - T.sha1[MT + l0]) / dta;
-    d_ss = (T.ssa1[MT + l1] - T.ssa1[MT + l0]) / dta;
-  }
-  slq2 = T.amtaun2a1[MT + l0] + d_slq2 * dx;
-  sm = T.sma1[MT + l0] + d_sm * dx;
-  sh = T.sha1[MT + l0] + d_sh * dx;
-  ss = T.ssa1[MT + l0] + d_ss * dx;
+  return true;
 }
 
 // interp2d_expabs (readyc.cpp:975-1114): ri, rid clipped to the table in
 // place; outputs left as they were on the reference's early returns
-__device__ void interp2d(double& ri, double& rid, const TurbTabDev& T, const TurbConst& C, double& slq2, double& sm,
-                         double& sh, double& ss) {
+// (false).  The four tables are interleaved, so a corner of the four is one
+// 32-byte sector and two corners of a row are adjacent: the gathers, which
+// miss L2 (274 MB of tables), touch 3 sectors per cell instead of 8.
+struct Stab {
+  double slq2, sm, sh, ss;
+};
+__device__ __forceinline__ Stab quad_at(const TurbTabDev& T, long c) {
+  const double2* p = reinterpret_cast<const double2*>(T.quad) + 2 * c;
+  const double2 u = __ldg(p), v = __ldg(p + 1);
+  return {u.x, u.y, v.x, v.y};
+}
+
+__device__ __forceinline__ bool interp2d(double& ri, double& rid, const TurbTabDev& T, const TurbConst& C, Stab& out) {
   const double* rib = T.rib;
-  const double rmax = rib[2 * MT], rmin = rib[0];
-  if (ri > rmax) {
-    if (fabs(rid) <= ri) {
-      rid = rmax * (rid / ri);
-      ri = rmax;
-    } else if (rid > ri) {
+  const double rmax = T.gmax, rmin = T.rib0, gm = T.gm;
+  if (ri > rmax || ri < rmin || rid > rmax || rid < rmin) {
+    if (ri > rmax) {
+      if (fabs(rid) <= ri) {
+        rid = rmax * (rid / ri);
+        ri = rmax;
+      } else if (rid > ri) {
+        ri = rmax * (ri / rid);
+        rid = rmax;
+      } else if (rid < -ri) {
+        ri = rmin * (ri / rid);
+        rid = rmin;
+      }
+    } else if (ri < rmin) {
+      if (fabs(rid) <= -ri) {
+        rid = rmin * (rid / ri);
+        ri = rmin;
+      } else if (rid > -ri) {
+        ri = rmax * (ri / rid);
+        rid = rmax;
+      } else if (rid < ri) {
+        ri = rmin * (ri / rid);
+        rid = rmin;
+      }
+    } else if (rid > rmax) {
       ri = rmax * (ri / rid);
       rid = rmax;
-    } else if (rid < -ri) {
+    } else if (rid < rmin) {
       ri = rmin * (ri / rid);
       rid = rmin;
     }
-  } else if (ri < rmin) {
-    if (fabs(rid) <= -ri) {
-      rid = rmin * (rid / ri);
-      ri = rmin;
-    } else if (rid > -ri) {
-      ri = rmax * (ri / rid);
-      rid = rmax;
-    } else if (rid < ri) {
-      ri = rmin * (ri / rid);
-      rid = rmin;
-    }
-  } else if (rid > rmax) {
-    ri = rmax * (ri / rid);
-    rid = rmax;
-  } else if (rid < rmin) {
-    ri = rmin * (ri / rid);
-    rid = rmin;
   }
   const double x_ri = ri, x_rid = rid;
-  const double gm = rib[MT + MT0];
-  int d0, d1, r0, r1;
-  if (fabs(x_rid) >= gm && fabs(x_rid) >= rmax) {
-    d0 = (int)sgn((double)MT, x_rid);
-    d1 = d0;
-  } else {
-    expabs_index(x_rid, rib, T.dri, C.log_gm, C.log_rri, d0, d1);
-    if (x_rid == 0.0e0) d1 = 1;
+  Bracket d, r;
+  if (fabs(x_rid) >= gm && fabs(x_rid) >= rmax) d.lo = d.hi = x_rid >= 0.0 ? 2 * MT : 0;
+  else d = bracket(x_rid, rib, gm, C.inv_dri, C.log2_gm, C.per_log2);
+  const double d0 = rib[d.lo], d1 = rib[d.hi];
+  if ((x_rid > 0.0e0 && (x_rid < d0 || x_rid > d1)) || (x_rid < 0.0e0 && (x_rid > d0 || x_rid < d1))) return false;
+  if (x_ri > fmin(T.rilim[d.lo], T.rilim[d.hi])) {
+    out = {0.0e0, 0.0e0, 0.0e0, 0.0e0};
+    return true;
   }
-  if ((x_rid > 0.0e0 && (x_rid < rib[MT + d0] || x_rid > rib[MT + d1])) ||
-      (x_rid < 0.0e0 && (x_rid > rib[MT + d0] || x_rid < rib[MT + d1])))
-    return;
-  if (x_ri > fmin(rib[MT + T.irimax[MT + d0]], rib[MT + T.irimax[MT + d1]])) {
-    slq2 = 0.0e0;
-    sm = 0.0e0;
-    sh = 0.0e0;
-    ss = 0.0e0;
-    return;
+  if (fabs(x_ri) >= gm && fabs(x_ri) >= rmax) r.lo = r.hi = x_ri >= 0.0 ? 2 * MT : 0;
+  else r = bracket(x_ri, rib, gm, C.inv_dri, C.log2_gm, C.per_log2);
+  const double r0 = rib[r.lo], r1 = rib[r.hi];
+  if ((x_ri > 0.0e0 && (x_ri < r0 || x_ri > r1)) || (x_ri < 0.0e0 && (x_ri > r0 || x_ri < r1))) return false;
+  const Stab t00 = quad_at(T, (long)N1 * d.lo + r.lo);
+  out = t00;
+  if (d.hi != d.lo) {
+    const Stab t10 = quad_at(T, (long)N1 * d.hi + r.lo), t01 = quad_at(T, (long)N1 * d.lo + r.hi);
+    const double gd = 1.0 / (d1 - d0), gr = 1.0 / (r1 - r0);
+    const double drid = x_rid - d0, dri = x_ri - r0;
+    out.slq2 = t00.slq2 + (t01.slq2 - t00.slq2) * gr * dri + (t10.slq2 - t00.slq2) * gd * drid;
+    out.sm = t00.sm + (t01.sm - t00.sm) * gr * dri + (t10.sm - t00.sm) * gd * drid;
+    out.sh = t00.sh + (t01.sh - t00.sh) * gr * dri + (t10.sh - t00.sh) * gd * drid;
+    out.ss = t00.ss + (t01.ss - t00.ss) * gr * dri + (t10.ss - t00.ss) * gd * drid;
   }
-  if (fabs(x_ri) >= gm && fabs(x_ri) >= rmax) {
-    r0 = (int)sgn((double)MT, x_ri);
-    r1 = r0;
-  } else {
-    expabs_index(x_ri, rib, T.dri, C.log_gm, C.log_rri, r0, r1);
-    if (x_ri == 0.0e0) r1 = 1;
-  }
-  if ((x_ri > 0.0e0 && (x_ri < rib[MT + r0] || x_ri > rib[MT + r1])) ||
-      (x_ri < 0.0e0 && (x_ri > rib[MT + r0] || x_ri < rib[MT + r1])))
-    return;
-  const double dridta = rib[MT + d1] - rib[MT + d0];
-  const double drita = rib[MT + r1] - rib[MT + r0];
-  const double drid = x_rid - rib[MT + d0];
-  const double dri = x_ri - rib[MT + r0];
-  const long c00 = (long)N1 * (d0 + MT) + r0 + MT;
-  const long c10 = (long)N1 * (d1 + MT) + r0 + MT;
-  const long c01 = (long)N1 * (d0 + MT) + r1 + MT;
-  double a_rid[4], a_ri[4];
-  const double* tab[4] = {T.slq2b, T.smb, T.shb, T.ssb};
-#pragma unroll
-  for (int m = 0; m < 4; ++m) {
-    if (d1 == d0) {
-      a_rid[m] = 0.0e0;
-      a_ri[m] = 0.0e0;
-    } else {
-      a_rid[m] = (tab[m][c10] - tab[m][c00]) / dridta;
-      a_ri[m] = (tab[m][c01] - tab[m][c00]) / drita;
-    }
-  }
-  slq2 = T.slq2b[c00] + a_ri[0] * dri + a_rid[0] * drid;
-  sm = T.smb[c00] + a_ri[1] * dri + a_rid[1] * drid;
-  sh = T.shb[c00] + a_ri[2] * dri + a_rid[2] * drid;
-  ss = T.ssb[c00] + a_ri[3] * dri + a_rid[3] * drid;
+  return true;
+}
+// the background's second look-up (rare), kept out of the level loop's code
+__device__ __noinline__ bool interp2d_back(double& ri, double& rid, const TurbTabDev& T, const TurbConst& C, Stab& out) {
+  return interp2d(ri, rid, T, C, out);
 }
 
 // The column's interface values (the reference's wp1, wp3, wp8 at level k,
 // k < kmt-1): temperature and density interpolated to the interface below
 // level k, and its depth in cm
 struct Iface {
-  const double *T, *pd, *dzp, *zkp;
+  const double *T, *pd;
+  const double *dz, *hs, *ys, *zz;   // shared memory: dzp, dzp + dzp of the next level, its reciprocal, depth
   long A;
   __device__ double t(int k) const {
-    return T[k * A] - (T[k * A] - T[(k + 1) * A]) * dzp[k] / (dzp[k] + dzp[k + 1]);
+    const double a = T[k * A];
+    return a - quotient((a - T[(k + 1) * A]) * dz[k], hs[k], ys[k]);
   }
-  __device__ double rh(int k) const {
-    return (pd[k * A] + (pd[(k + 1) * A] - pd[k * A]) * dzp[k] / (dzp[k] + dzp[k + 1])) * 1.0e-3;
+  __device__ double rh_of(int k, double p0, double p1) const {
+    return (p0 + quotient((p1 - p0) * dz[k], hs[k], ys[k])) * 1.0e-3;
   }
-  __device__ double z(int k) const { return -zkp[k + 1] * 1.0e+2; }
+  __device__ double rh(int k) const { return rh_of(k, pd[k * A], pd[(k + 1) * A]); }
+  __device__ double z(int k) const { return zz[k]; }
 };
 
-__global__ void __launch_bounds__(128, 5) k_turb(Arena a, TurbTabDev T, double ncc_f, double fricmx, double wndmix) {
+constexpr int kTurbLevels = 256;   // most levels a domain may have
+
+__global__ void __launch_bounds__(128, 5)
+    k_turb(const __grid_constant__ Arena a, const __grid_constant__ TurbTabDev T, const __grid_constant__ TurbConst C,
+           double ncc_f, double fricmx, double wndmix) {
+  __shared__ double s_dz[kTurbLevels], s_hs[kTurbLevels], s_ys[kTurbLevels], s_zz[kTurbLevels];
+  for (int k = threadIdx.y * blockDim.x + threadIdx.x; k < a.km; k += blockDim.x * blockDim.y) {
+    const double dz = a.dzp[k], h = dz + (k + 1 < a.km ? a.dzp[k + 1] : 0.0);
+    s_dz[k] = dz;
+    s_hs[k] = h;
+    s_ys[k] = quotient_reciprocal(h);
+    s_zz[k] = -a.zkp[k + 1] * 1.0e+2;
+  }
+  __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= a.imt || j >= a.jmt) return;
@@ -239,26 +233,41 @@ __global__ void __launch_bounds__(128, 5) k_turb(Arena a, TurbTabDev T, double n
     return;
   }
   const int n = kz - 1;   // interfaces of the column (iwk)
-  Iface f{a.at[a.cur] + q, a.pdensity + q, a.dzp, a.zkp, A};
-  const double* rict = a.rict + q;
+  const Iface f{a.at[a.cur] + q, a.pdensity + q, s_dz, s_hs, s_ys, s_zz, A};
+  const double* __restrict__ rict = a.rict + q;
 
-  // ---- 1. tidal mixing, bottom-up minimum (readyc.cpp:1534-1557)
+  // ---- 1. tidal mixing, bottom-up minimum (readyc.cpp:1534-1557); four
+  // levels' loads ahead of their stores
   {
     double below = 0.0;
     const double wd = a.wave_dis[q];
+    const double* __restrict__ fzt = a.fz_tide + q;
     for (int k = km - 1; k >= n; --k) a.ak_tide[k * A + q] = 0.0;
-    for (int k = n - 1; k >= 0; --k) {
-      const double wp3 = f.rh(k);
-      const double rc = rict[k * A];
-      const double fz = a.fz_tide[k * A + q];
-      double v = kBackTidal + kMixingEf * kLocalFrac * wd * fz / (fmax(rc, 1.0e-8) * (wp3 * 1000.0));
-      if (v > kMaxTidal) v = kMaxTidal;
-      if (k <= n - 2) v = fmin(v, below);
-      below = v;
-      a.ak_tide[k * A + q] = v;
-      a.richardson[k * A + q] = rc;
-      a.fztidal[k * A + q] = fz;
-      a.wp3_tidal[k * A + q] = wp3;
+    double pd1 = n > 0 ? f.pd[n * A] : 0.0;
+    for (int k0 = n - 1; k0 >= 0; k0 -= 4) {
+      double pd0[4], rc[4], fz[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int k = k0 - c >= 0 ? k0 - c : 0;
+        pd0[c] = f.pd[k * A];
+        rc[c] = rict[k * A];
+        fz[c] = fzt[k * A];
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int k = k0 - c;
+        if (k < 0) break;
+        const double wp3 = f.rh_of(k, pd0[c], pd1);
+        pd1 = pd0[c];
+        double v = kBackTidal + kMixingEf * kLocalFrac * wd * fz[c] / (fmax(rc[c], 1.0e-8) * (wp3 * 1000.0));
+        if (v > kMaxTidal) v = kMaxTidal;
+        if (k <= n - 2) v = fmin(v, below);
+        below = v;
+        a.ak_tide[k * A + q] = v;
+        a.richardson[k * A + q] = rc[c];
+        a.fztidal[k * A + q] = fz[c];
+        a.wp3_tidal[k * A + q] = wp3;
+      }
     }
   }
 
@@ -284,24 +293,14 @@ __global__ void __launch_bounds__(128, 5) k_turb(Arena a, TurbTabDev T, double n
   a.amld[q] = amld * 1.0e-2;
 
   // ---- 3. the closure, level by level (turb_device, readyc.cpp:1116-1454)
-  TurbConst C;
-  C.pi4 = atan(1.0e0);
-  {
-    const double an0 = 5.24e-3, f30 = 4.0e0 * C.pi4 / 43082.0e0;
-    C.eplat_den = f30 * acosh(an0 / f30);
-  }
-  C.log_gm = log(T.rib[MT + MT0]);
-  C.log_rri = log(T.rri);
-  C.log_gm1 = log(T.and2on2a1[MT + MT0]);
-  C.log_rnd = log(T.rnd2on2);
   const double coriol = a.fcort[q];
   const double buoytot = a.buoytur[q] * 1.0e+4 + a.buoysol[q] * 1.0e+4;
   const double b1 = T.b1;
   const double al0 = 0.17 * amld;
   double ifbelow = 0.0;
   double an = 0.0;                     // unset in the reference until N^2 >= 0 is met
-  double slq2 = 0.0, sm = 0.0, sh = 0.0, ss = 0.0, amtaun2 = 0.0;
-  double slq2_back = 0.0, sm_back = 0.0, sh_back = 0.0, ss_back = 0.0;
+  Stab st{0.0, 0.0, 0.0, 0.0}, back{0.0, 0.0, 0.0, 0.0};
+  double amtaun2 = 0.0;
   double back_ri1 = 0.0, tmp = 0.0;
   double km0 = 0.0, kh0 = 0.0, ks0 = 0.0;   // level 0, written last
   double* akt_t = a.precision == LT_PREC_MIXED ? nullptr : a.akt + q;
@@ -310,8 +309,8 @@ __global__ void __launch_bounds__(128, 5) k_turb(Arena a, TurbTabDev T, double n
   auto put = [&](int k, double akm, double akh, double aks) {
     const double tide = a.ak_tide[k * A + q];
     a.akmt[k * A + q] = akm * 1.0e-4 + tide * 5.0;
-    const double t_ = (akh * 1.0e-4 + tide) / ncc_f;
-    const double s_ = (aks * 1.0e-4 + tide) / ncc_f;
+    const double t_ = quotient(akh * 1.0e-4 + tide, ncc_f, C.inv_ncc);
+    const double s_ = quotient(aks * 1.0e-4 + tide, ncc_f, C.inv_ncc);
     if (akt_t) {
       akt_t[k * A] = t_;
       akt_t[F + k * A] = s_;
@@ -325,53 +324,69 @@ __global__ void __launch_bounds__(128, 5) k_turb(Arena a, TurbTabDev T, double n
   double rh_m2 = 0.0, rh_m1 = 0.0, rh_0 = n > 0 ? f.rh(0) : 0.0, rh_p1 = n > 1 ? f.rh(1) : 0.0;
   int done = 0;   // levels whose diffusivities the closure set
   bool quit = false;
+  // the level's inputs are loaded a level ahead
+  const double* __restrict__ rit_ = a.rit + q;
+  const double* __restrict__ rid_ = a.ricdttms + q;
+  const double* __restrict__ s2t_ = a.s2t + q;
+  double in_an2 = 0.0, in_ri = 0.0, in_rid = 0.0, in_s2 = 0.0;
+  auto fetch = [&](int k) {
+    if (k < n) {
+      in_an2 = rict[k * A];
+      in_ri = rit_[k * A];
+      in_rid = rid_[k * A];
+      in_s2 = s2t_[k * A];
+    }
+  };
+  fetch(0);
   for (int k = 0; k < n; ++k) {
-    const double an2 = rict[k * A];
-    const double rik = a.rit[k * A + q];
-    const double ridk = a.ricdttms[k * A + q];
-    double s2 = a.s2t[k * A + q];
+    const double an2 = in_an2, rik = in_ri, ridk = in_rid;
+    double s2 = in_s2;
+    fetch(k + 1);
     double ifnofsmall = 0.0;
     if (an2 >= 0.0e0) an = sqrt(an2);
     if (an < fabs(coriol)) ifnofsmall = 1.0;
     double ri1 = rik, rid1 = ridk;
-    const double and2 = ridk / (rik + 1.0e-25) * an2;
-    const double and2on2 = and2 / (an2 + 1.0e-25);
-    const int ifpureshear = (an2 < T.rib[0] * s2) ? 1 : 0;
+    const int ifpureshear = (an2 < T.rib0 * s2) ? 1 : 0;
     if (ifpureshear == 1) {
-      interp1d(and2on2, T, C, amtaun2, sm, sh, ss);
-      slq2 = (-amtaun2) / ((b1 * b1) * rik + 1.0e-25);
+      const double and2 = ridk / (rik + 1.0e-25) * an2;
+      const double and2on2 = and2 / (an2 + 1.0e-25);
+      double v[4];
+      if (interp1d(and2on2, T, C, v)) {
+        amtaun2 = v[0];
+        st.sm = v[1];
+        st.sh = v[2];
+        st.ss = v[3];
+      }
+      st.slq2 = (-amtaun2) / ((b1 * b1) * rik + 1.0e-25);
     } else {
-      interp2d(ri1, rid1, T, C, slq2, sm, sh, ss);
-      if (slq2 < 0.0e0) { quit = true; break; }
-      if (slq2 == 0.0e0) ifbelow = 1.0;
+      interp2d(ri1, rid1, T, C, st);
+      if (st.slq2 < 0.0e0) { quit = true; break; }
+      if (st.slq2 == 0.0e0) ifbelow = 1.0;
     }
-    const bool lifupper = ((ifbelow == 0.0 || ifnofsmall == 1.0 || ((ri1 < 0.0e0) && (k <= 1))) && (slq2 > 0.0e0));
+    const bool lifupper = ((ifbelow == 0.0 || ifnofsmall == 1.0 || ((ri1 < 0.0e0) && (k <= 1))) && (st.slq2 > 0.0e0));
     double epsy = 0.0e0;
-    bool lifepsy = false;
-    if (slq2 == 0.0e0) epsy = 0.0e0;
-    else epsy = -buoytot / ((1.0e0 / ((b1 * b1) * (slq2))) - 0.5e0 * sm);
-    lifepsy = ((epsy >= 0.0e0) && lifupper);
+    if (lifupper) epsy = -buoytot / ((1.0e0 / ((b1 * b1) * (st.slq2))) - 0.5e0 * st.sm);
+    const bool lifepsy = ((epsy >= 0.0e0) && lifupper);
     const double akz = 0.4 * z_0;
     const double al = akz * al0 / (al0 + akz);
     double al2 = al * al;
     if (ifbelow != 1.0 && !lifepsy) {
       if (ri1 > 0.0e0) {
-        const double anlq2 = slq2 * ri1;
+        const double anlq2 = st.slq2 * ri1;
         if (anlq2 > 0.281e0) {
           al2 *= 0.281e0 / anlq2;
-          slq2 = 0.281e0 / (ri1 + 1.0e-20);
+          st.slq2 = 0.281e0 / (ri1 + 1.0e-20);
         }
       }
     }
-    double epson2;
-    if (an2 < 0.0e0) {
-      epson2 = kEpson2;
-    } else {
+    // the latitude factor enters through the background (Ri > 0) and, below
+    // the mixed part, for Ri >= 0 only
+    double epson2 = kEpson2;
+    if (!(an2 < 0.0e0) && (rik > 0.0e0 || ri1 >= 0.0e0)) {
       double ep = ifnofsmall == 1.0 ? 0.0e0 : eplat(C, fabs(coriol), an);
       ep = fmax(ep, kEplatMin);
       epson2 = kEpson2 * ep;
     }
-    double back_ra_r1 = 0.0, back_rit1 = 0.0, back_ric1 = 0.0, back_rid1 = 0.0;
     if (rik > 0.0e0) {
       const double rit = (rik + ridk) / 2.0e0;
       const double ric = (rik - ridk) / 2.0e0;
@@ -380,8 +395,15 @@ __global__ void __launch_bounds__(128, 5) k_turb(Arena a, TurbTabDev T, double n
       if (fabs(rit) <= 0.0e0) theta_r = (fabs(ric) <= 0.0e0) ? C.pi4 : 2.0e0 * C.pi4;
       else theta_r = atan(ric / rit);
       if (fabs(theta_r) > 2.0e0 * C.pi4) { quit = true; break; }
-      if (theta_r < -C.pi4) theta_r += 4.0e0 * C.pi4;
-      const int jt0 = (int)((theta_r + C.pi4) / T.deltheta_r);
+      // cos and sin of the angle from its own components: it points along
+      // (rit, ric), or against it where rit < 0, and is turned by pi below -pi/4
+      double turn = rit < 0.0e0 ? -1.0 : 1.0;
+      if (theta_r < -C.pi4) {
+        theta_r += 4.0e0 * C.pi4;
+        turn = -turn;
+      }
+      bool moved = fabs(rit) <= 0.0e0;
+      const int jt0 = (int)((theta_r + C.pi4) * C.inv_dth);
       int it0 = jt0 - NTH, it1 = it0 + 1;
       double th0 = it0 * T.deltheta_r, th1 = it1 * T.deltheta_r;
       if ((th0 <= T.theta_rcrp) && (theta_r > T.theta_rcrp)) {
@@ -390,17 +412,19 @@ __global__ void __launch_bounds__(128, 5) k_turb(Arena a, TurbTabDev T, double n
         it0 = it1;
         ++it1;
         th1 += T.deltheta_r;
+        moved = true;
       } else if ((th1 >= T.theta_rcrn) && (theta_r < T.theta_rcrn)) {
         theta_r = th0;
         th1 = th0;
         it1 = it0;
         --it0;
         th0 += -T.deltheta_r;
+        moved = true;
       }
       if ((it1 > 3 * NTH) || (it0 < -NTH)) { quit = true; break; }
       double dth = theta_r - th0;
-      const double del = T.back_ra_r[NTH + it1] - T.back_ra_r[NTH + it0];
-      back_ra_r1 = T.back_ra_r[NTH + it0] + dth * (del / T.deltheta_r);
+      const double br0 = T.back_ra_r[NTH + it0];
+      double back_ra_r1 = br0 + dth * ((T.back_ra_r[NTH + it1] - br0) * C.inv_dth);
       int ifrafglt = 0;
       if ((theta_r <= T.theta_rcrp) || (theta_r >= T.theta_rcrn)) {
         if (back_ra_r1 > ra_r) {
@@ -409,38 +433,52 @@ __global__ void __launch_bounds__(128, 5) k_turb(Arena a, TurbTabDev T, double n
         }
       }
       if (back_ra_r1 < 0.0e0) { quit = true; break; }
-      back_rit1 = cos(theta_r) * back_ra_r1;
-      back_ric1 = sin(theta_r) * back_ra_r1;
-      back_ri1 = back_rit1 + back_ric1;
-      back_rid1 = back_rit1 - back_ric1;
-      if (ifrafglt == 1) {
-        interp2d(back_ri1, back_rid1, T, C, slq2_back, sm_back, sh_back, ss_back);
+      double back_rit1, back_ric1;
+      if (moved) {
+        back_rit1 = cos(theta_r) * back_ra_r1;
+        back_ric1 = sin(theta_r) * back_ra_r1;
       } else {
-        dth = theta_r - it0 * T.deltheta_r;
-        sm_back = T.sm_r1[NTH + it0] + dth * ((T.sm_r1[NTH + it1] - T.sm_r1[NTH + it0]) / T.deltheta_r);
-        sh_back = T.sh_r1[NTH + it0] + dth * ((T.sh_r1[NTH + it1] - T.sh_r1[NTH + it0]) / T.deltheta_r);
-        ss_back = T.ss_r1[NTH + it0] + dth * ((T.ss_r1[NTH + it1] - T.ss_r1[NTH + it0]) / T.deltheta_r);
-        slq2_back = T.slq2_r1[NTH + it0] + dth * ((T.slq2_r1[NTH + it1] - T.slq2_r1[NTH + it0]) / T.deltheta_r);
+        const double scale = turn * back_ra_r1 / ra_r;
+        back_rit1 = rit * scale;
+        back_ric1 = ric * scale;
       }
-      if (slq2_back < 0.0e0) { quit = true; break; }
+      back_ri1 = back_rit1 + back_ric1;
+      if (ifrafglt == 1) {
+        double back_rid1 = back_rit1 - back_ric1, bri = back_ri1;
+        Stab b = back;
+        interp2d_back(bri, back_rid1, T, C, b);
+        back_ri1 = bri;
+        back = b;
+      } else {
+        dth = (theta_r - it0 * T.deltheta_r) * C.inv_dth;
+        back.sm = T.sm_r1[NTH + it0] + dth * (T.sm_r1[NTH + it1] - T.sm_r1[NTH + it0]);
+        back.sh = T.sh_r1[NTH + it0] + dth * (T.sh_r1[NTH + it1] - T.sh_r1[NTH + it0]);
+        back.ss = T.ss_r1[NTH + it0] + dth * (T.ss_r1[NTH + it1] - T.ss_r1[NTH + it0]);
+        back.slq2 = T.slq2_r1[NTH + it0] + dth * (T.slq2_r1[NTH + it1] - T.slq2_r1[NTH + it0]);
+      }
+      if (back.slq2 < 0.0e0) { quit = true; break; }
     }
     if (rik <= 0.0e0) back_ri1 = 0.0e0;
     if (ri1 <= 0.0e0) {
-      sm_back = 0.0e0;
-      sh_back = 0.0e0;
-      ss_back = 0.0e0;
+      back.sm = 0.0e0;
+      back.sh = 0.0e0;
+      back.ss = 0.0e0;
     }
-    if ((sm_back < 0.0e0) || (sh_back < 0.0e0) || (ss_back < 0.0e0)) { quit = true; break; }
-    const double tmp_back = 0.5e0 * b1 * b1 * back_ri1 * slq2_back * epson2;
-    const double v_back = tmp_back * sm_back, t_back = tmp_back * sh_back, s_back = tmp_back * ss_back;
+    if ((back.sm < 0.0e0) || (back.sh < 0.0e0) || (back.ss < 0.0e0)) { quit = true; break; }
+    const double tmp_back = 0.5e0 * b1 * b1 * back_ri1 * back.slq2 * epson2;
+    const double v_back = tmp_back * back.sm, t_back = tmp_back * back.sh, s_back = tmp_back * back.ss;
     if ((v_back < 0.0e0) || (t_back < 0.0e0) || (s_back < 0.0e0)) { quit = true; break; }
     if ((rik > 0.0e0) && ((fabs(v_back) <= 0.0e0) || (fabs(t_back) <= 0.0e0) || (fabs(s_back) < 0.0e0))) {
       quit = true;
       break;
     }
+    // the mixing scale: the closure's own where the level is not below the
+    // mixed part, or is unstable there
+    bool shear_scale = ifpureshear != 1;
     if (ifbelow == 1.0) {
       if (ri1 >= 0.0e0) {
-        tmp = 0.5e0 * b1 * b1 * ri1 * slq2 * epson2;
+        tmp = 0.5e0 * b1 * b1 * ri1 * st.slq2 * epson2;
+        shear_scale = false;
       } else if (k >= 2) {
         double delz, delrh, del2rh;
         if (k == n - 1) {
@@ -459,28 +497,17 @@ __global__ void __launch_bounds__(128, 5) k_turb(Arena a, TurbTabDev T, double n
         const double akz2 = 0.4e0 * z_0;
         const double aldeep = akz2 * al0deep / (al0deep + akz2);
         al2 = aldeep * aldeep;
-        if (ifpureshear != 1) {
-          s2 = fmax(s2, kS2min);
-          tmp = 0.5e0 * b1 * al2 * sqrt(s2 / (slq2 + 1.0e-40));
-        }
-      } else {
-        if (ifpureshear != 1) {
-          s2 = fmax(s2, kS2min);
-          if (lifepsy) tmp = 0.5e0 * epsy / (s2 + 1.0e-40);
-          else tmp = 0.5e0 * b1 * al2 * sqrt(s2 / (slq2 + 1.0e-40));
-        }
-      }
-    } else {
-      if (ifpureshear != 1) {
-        s2 = fmax(s2, kS2min);
-        if (lifepsy) tmp = 0.5e0 * epsy / (s2 + 1.0e-40);
-        else tmp = 0.5e0 * b1 * al2 * sqrt(s2 / (slq2 + 1.0e-40));
       }
     }
+    if (shear_scale) {
+      s2 = fmax(s2, kS2min);
+      if (lifepsy && !(ifbelow == 1.0 && k >= 2)) tmp = 0.5e0 * epsy / (s2 + 1.0e-40);
+      else tmp = 0.5e0 * b1 * al2 * sqrt(s2 / (st.slq2 + 1.0e-40));
+    }
     if (ifpureshear == 1) tmp = 0.5e0 * (b1 * b1) * al2 * sqrt(-an2 / amtaun2);
-    const double akm = fmin(tmp * sm + v_back, fricmx);
-    const double akh = fmin(tmp * sh + t_back, fricmx);
-    const double aks = fmin(tmp * ss + s_back, fricmx);
+    const double akm = fmin(tmp * st.sm + v_back, fricmx);
+    const double akh = fmin(tmp * st.sh + t_back, fricmx);
+    const double aks = fmin(tmp * st.ss + s_back, fricmx);
     if (k == 0) {
       km0 = akm;
       kh0 = akh;
@@ -506,15 +533,38 @@ __global__ void __launch_bounds__(128, 5) k_turb(Arena a, TurbTabDev T, double n
     if (ks0 < wndmix) ks0 = wndmix;
   }
   put(0, km0, kh0, ks0);
-  for (int k = done > 1 ? done : 1; k < km - 1; ++k) put(k, 0.0, 0.0, 0.0);
+  for (int k = done > 1 ? done : 1; k < n; ++k) put(k, 0.0, 0.0, 0.0);
+  for (int k = n > 1 ? n : 1; k < km - 1; ++k) {   // below the column: no tide either
+    a.akmt[k * A + q] = 0.0;
+    if (akt_t) akt_t[k * A] = akt_t[F + k * A] = 0.0;
+    else akt_t32[k * A] = akt_t32[F + k * A] = 0.0f;
+  }
   a.akmt[(long)(km - 1) * A + q] = 0.0;
+}
+
+// one table into its place among the interleaved four
+__global__ void k_interleave(const double* __restrict__ x, double* __restrict__ quad, long n) {
+  for (long m = (long)blockIdx.x * blockDim.x + threadIdx.x; m < n; m += (long)gridDim.x * blockDim.x) quad[4 * m] = x[m];
 }
 
 }  // namespace
 
 int launch_turb(const Arena& a, const TurbTabDev& T, int ncc, double dfricmx, cudaStream_t s) {
-  dim3 b(32, 4), g((a.imt + 31) / 32, (a.jmt + 3) / 4);
-  k_turb<<<g, b, 0, s>>>(a, T, (double)(float)ncc, dfricmx * 1.0e+4, a.p.dwndmix * 1.0e+4);
+  TurbConst C;
+  C.pi4 = std::atan(1.0);
+  const double an0 = 5.24e-3, f30 = 4.0 * C.pi4 / 43082.0;
+  C.eplat_den = f30 * std::acosh(an0 / f30);
+  C.inv_ncc = quotient_reciprocal((double)(float)ncc);
+  C.inv_dth = 1.0 / T.deltheta_r;
+  C.inv_dri = 1.0 / T.dri;
+  C.inv_da = 1.0 / T.dand2on2;
+  C.log2_gm = (float)std::log2(T.gm);
+  C.per_log2 = (float)(1.0 / std::log2(T.rri));
+  C.log2_gm1 = (float)std::log2(T.gm1);
+  C.per_log21 = (float)(1.0 / std::log2(T.rnd2on2));
+  // warps of 8 x 4 columns: depths and stability alike, so fewer idle lanes
+  dim3 b(8, 16), g((a.imt + 7) / 8, (a.jmt + 15) / 16);
+  k_turb<<<g, b, 0, s>>>(a, T, C, (double)(float)ncc, dfricmx * 1.0e+4, a.p.dwndmix * 1.0e+4);
   LT_LAUNCHED();
   return LT_OK;
 }
@@ -546,10 +596,11 @@ int lt_turb_tables_create(const lt_turb_tables* h, lt_turb_tab** out) {
   lt_turb_tab* t = new (std::nothrow) lt_turb_tab;
   if (!t) return LT_E_OOM;
   TurbTabDev& T = t->t;
+  std::vector<double> rilim(n1);   // the realizable limit of Ri itself
+  for (int m = 0; m < N1; ++m) rilim[m] = h->rib[MT + h->irimax[m]];
   const Item items[] = {
-      {h->rib, n1 * 8, (const void**)&T.rib},         {h->irimax, n1 * 4, (const void**)&T.irimax},
-      {h->slq2b, n2 * 8, (const void**)&T.slq2b},     {h->smb, n2 * 8, (const void**)&T.smb},
-      {h->shb, n2 * 8, (const void**)&T.shb},         {h->ssb, n2 * 8, (const void**)&T.ssb},
+      {nullptr, 4 * n2 * 8, (const void**)&T.quad},
+      {h->rib, n1 * 8, (const void**)&T.rib},         {rilim.data(), n1 * 8, (const void**)&T.rilim},
       {h->and2on2a1, n1 * 8, (const void**)&T.and2on2a1}, {h->amtaun2a1, n1 * 8, (const void**)&T.amtaun2a1},
       {h->sma1, n1 * 8, (const void**)&T.sma1},       {h->sha1, n1 * 8, (const void**)&T.sha1},
       {h->ssa1, n1 * 8, (const void**)&T.ssa1},       {h->back_ra_r, nb * 8, (const void**)&T.back_ra_r},
@@ -558,23 +609,39 @@ int lt_turb_tables_create(const lt_turb_tables* h, lt_turb_tab** out) {
   size_t total = 0;
   for (const Item& it : items) total += (it.bytes + 255) / 256 * 256;
   char* base = nullptr;
+  double* one = nullptr;   // one 2-D table on its way into the interleaved four
   cudaError_t e = cudaMalloc(&base, total);
+  if (e == cudaSuccess && (e = cudaMalloc(&one, n2 * 8)) != cudaSuccess) cudaFree(base);
   if (e != cudaSuccess) {
     delete t;
-    set_error("lt_turb_tables_create: cudaMalloc(%zu) failed: %s", total, cudaGetErrorString(e));
+    set_error("lt_turb_tables_create: cudaMalloc(%zu) failed: %s", total + n2 * 8, cudaGetErrorString(e));
     return LT_E_OOM;
   }
   size_t off = 0;
   for (const Item& it : items) {
     *it.dst = base + off;
-    e = cudaMemcpy(base + off, it.src, it.bytes, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-      cudaFree(base);
-      delete t;
-      return cuda_fail(e, "lt_turb_tables_create");
-    }
+    if (it.src && e == cudaSuccess) e = cudaMemcpy(base + off, it.src, it.bytes, cudaMemcpyHostToDevice);
     off += (it.bytes + 255) / 256 * 256;
   }
+  const double* tabs[4] = {h->slq2b, h->smb, h->shb, h->ssb};
+  for (int m = 0; m < 4 && e == cudaSuccess; ++m) {
+    e = cudaMemcpy(one, tabs[m], n2 * 8, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) break;
+    k_interleave<<<1184, 256>>>(one, const_cast<double*>(T.quad) + m, (long)n2);
+    lt::count_launches(1);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  }
+  cudaFree(one);
+  if (e != cudaSuccess) {
+    cudaFree(base);
+    delete t;
+    return cuda_fail(e, "lt_turb_tables_create");
+  }
+  T.rib0 = h->rib[0];
+  T.gm = h->rib[MT + MT0];
+  T.gmax = h->rib[2 * MT];
+  T.gm1 = h->and2on2a1[MT + MT0];
   T.rri = h->rri;
   T.rnd2on2 = h->rnd2on2;
   T.dri = h->dri;
