@@ -13,116 +13,164 @@ const lt::Domain* lt_synth_domain(const lt_synth* s);
 namespace lt {
 namespace {
 
-constexpr int KMAX_CONV = 128;
+// The convadj coefficients of every level in shared memory: cc [9][km], to, so
+// [km], dzp [km].
+struct ConvTab {
+  const double *cc, *to, *so, *dz;
+  int km;
+  // density departure of the convadj polynomial at coefficient level l
+  // (convadj.cpp:57-77) of water (t, s)
+  __device__ double rho(double t_, double s_, int l) const {
+    const double t = t_ - to[l], s = s_ - so[l];
+    return (cc[l] + (cc[3 * km + l] + cc[6 * km + l] * s) * s +
+            (cc[2 * km + l] + cc[7 * km + l] * s + cc[5 * km + l] * t) * t) * t +
+           (cc[1 * km + l] + (cc[4 * km + l] + cc[8 * km + l] * s) * s) * s;
+  }
+};
 
-// density departure of the convadj polynomial at coefficient level l
-// (convadj.cpp:57-77)
-__device__ __forceinline__ double conv_rho(const double* cc, int km, double t, double s, int l) {
-  return (cc[l] + (cc[3 * km + l] + cc[6 * km + l] * s) * s +
-          (cc[2 * km + l] + cc[7 * km + l] * s + cc[5 * km + l] * t) * t) * t +
-         (cc[1 * km + l] + (cc[4 * km + l] + cc[8 * km + l] * s) * s) * s;
-}
-
-// convadj_cu (convadj.cpp:29-288): one thread per column; finds the shallowest
-// statically unstable interface, mixes T and S thickness-weighted over the
-// unstable stretch and grows it up and down while unstable, then continues
-// below; finally the tendency diagnostics and atb = at.
-__global__ void k_convadj(Arena a) {
+// convadj_cu (convadj.cpp:29-288) without its last step: one thread per
+// column; finds the shallowest statically unstable interface, mixes T and S
+// thickness-weighted over the unstable stretch and grows it up and down while
+// unstable, then continues below.
+//
+// The reference keeps every interface's two densities in arrays; each is a
+// function of one level's water that is still unmixed when it is used, so
+// here they are formed where they are needed (the same bits) and a column
+// holds two levels in registers instead of 2 x km doubles in local memory,
+// whose traffic was more than the fields' own.  The search loads four levels
+// ahead of their use.  The step over every cell that follows is a kernel of
+// its own, level by level (k_convadj_tend).
+constexpr int kConvAhead = 4;
+constexpr int kConvLevels = 128;   // most levels taken
+__global__ void __launch_bounds__(128) k_convadj(const __grid_constant__ Arena a) {
+  extern __shared__ double s_conv[];
+  const int km = a.km;
+  for (int m = threadIdx.y * blockDim.x + threadIdx.x; m < 12 * km; m += blockDim.x * blockDim.y)
+    s_conv[m] = m < 9 * km ? a.cc[m] : m < 10 * km ? a.to[m - 9 * km] : m < 11 * km ? a.so[m - 10 * km] : a.dzp[m - 11 * km];
+  __syncthreads();
+  const ConvTab C{s_conv, s_conv + 9 * km, s_conv + 10 * km, s_conv + 11 * km, km};
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= a.imt || j >= a.jmt) return;
-  const int km = a.km;
-  const long A = a.A, F = a.F, FB = a.FB;
+  const long A = a.A, F = a.F;
   const long q = (long)j * a.imt + i;
-  double* at = a.at[a.cur];
-  double* atb = a.atb[a.cur];
-  const double* to = a.to;
-  const double* so = a.so;
-  const double* cc = a.cc;
-  const double* dzp = a.dzp;
-  double rhoup[KMAX_CONV], rholo[KMAX_CONV];
-  for (int l = 0; l < km; ++l) { rhoup[l] = 0.0; rholo[l] = 0.0; }
-  auto T = [&](int l) -> double& { return at[(long)l * A + q]; };
-  auto S = [&](int l) -> double& { return at[F + (long)l * A + q]; };
+  double* __restrict__ at = a.at[a.cur] + q;
+  const double* dzp = C.dz;
+  auto T = [&](int l) -> double& { return at[(long)l * A]; };
+  auto S = [&](int l) -> double& { return at[F + (long)l * A]; };
+  // densities across the interface below level l at the coefficients of level l+1
+  auto lower = [&](int l) { return C.rho(T(l), S(l), l + 1); };
+  auto upper = [&](int l) { return C.rho(T(l), S(l), l); };
   const int kcon = a.kmt[q];
-  if (kcon != 0) {
-    int lcon = 0;
-    for (int l = 0; l < km - 1; ++l) {
-      const int l1 = l + 1;
-      rhoup[l1] = conv_rho(cc, km, T(l1) - to[l1], S(l1) - so[l1], l1);
-      rholo[l] = conv_rho(cc, km, T(l) - to[l1], S(l) - so[l1], l1);
-    }
-    for (int k = kcon - 1; k >= 1; --k)
-      if (rholo[k - 1] > rhoup[k]) lcon = k;
-    if (lcon != 0) {
-      for (;;) {
-        int lcona = lcon, lconb = lcon + 1;
-        double dztsum = dzp[lcona - 1] + dzp[lconb - 1];
-        double trasum[2];
-        for (int n = 0; n < 2; ++n) {
-          double* X = at + n * F;
-          trasum[n] = X[(long)(lcona - 1) * A + q] * dzp[lcona - 1] + X[(long)(lconb - 1) * A + q] * dzp[lconb - 1];
-          const double tramix = trasum[n] / dztsum;
-          X[(long)(lcona - 1) * A + q] = tramix;
-          X[(long)(lconb - 1) * A + q] = tramix;
+  int lcon = 0;   // 1-based: the level above the shallowest unstable interface
+  if (kcon > 1) {
+    double t0 = T(0), s0 = S(0);
+    for (int l0 = 0; l0 < kcon - 1 && lcon == 0; l0 += kConvAhead) {
+      double t[kConvAhead], s[kConvAhead];
+#pragma unroll
+      for (int c = 0; c < kConvAhead; ++c) {
+        const int l = min(l0 + c + 1, kcon - 1);
+        t[c] = T(l);
+        s[c] = S(l);
+      }
+#pragma unroll
+      for (int c = 0; c < kConvAhead; ++c) {
+        const int l = l0 + c;
+        if (l < kcon - 1) {
+          if (lcon == 0 && C.rho(t0, s0, l + 1) > C.rho(t[c], s[c], l + 1)) lcon = l + 1;
+          t0 = t[c];
+          s0 = s[c];
         }
-        for (;;) {
-          if (lconb != kcon) {
-            const int l1 = lconb + 1;
-            rholo[lconb - 1] = conv_rho(cc, km, T(lconb - 1) - to[l1 - 1], S(lconb - 1) - so[l1 - 1], l1 - 1);
-            if (rholo[lconb - 1] > rhoup[l1 - 1]) {
-              lconb = lconb + 1;
-              dztsum = dztsum + dzp[lconb - 1];
-              for (int n = 0; n < 2; ++n) {
-                double* X = at + n * F;
-                trasum[n] = trasum[n] + X[(long)(lconb - 1) * A + q] * dzp[lconb - 1];
-                const double tramix = trasum[n] / dztsum;
-                for (int lm = lcona - 1; lm < lconb; ++lm) X[(long)lm * A + q] = tramix;
-              }
-              continue;
-            }
-          }
-          if (lcona > 1) {
-            const int l1 = lcona - 1;
-            rholo[l1 - 1] = conv_rho(cc, km, T(l1 - 1) - to[lcona - 1], S(l1 - 1) - so[lcona - 1], lcona - 1);
-            rhoup[lcona - 1] = conv_rho(cc, km, T(lcona - 1) - to[lcona - 1], S(lcona - 1) - so[lcona - 1], lcona - 1);
-            if (rholo[lcona - 2] > rhoup[lcona - 1]) {
-              lcona = lcona - 1;
-              dztsum = dztsum + dzp[lcona - 1];
-              for (int n = 0; n < 2; ++n) {
-                double* X = at + n * F;
-                trasum[n] = trasum[n] + X[(long)(lcona - 1) * A + q] * dzp[lcona - 1];
-                const double tramix = trasum[n] / dztsum;
-                for (int lm = lcona; lm <= lconb; ++lm) X[(long)(lm - 1) * A + q] = tramix;
-              }
-              continue;
-            }
-          }
-          break;
-        }
-        if (lconb == kcon) break;
-        lcon = lconb;
-        bool done = false;
-        for (;;) {
-          lcon = lcon + 1;
-          if (lcon == kcon) { done = true; break; }
-          if (rholo[lcon - 1] <= rhoup[lcon]) continue;
-          break;
-        }
-        if (done) break;
       }
     }
   }
-  const double c2dtts = a.p.dts;
-  for (int n = 0; n < 2; ++n)
-    for (int k = 0; k < km; ++k) {
-      const long c = n * F + (long)k * A + q;
-      const double vit = (k < kcon) ? 1.0 : 0.0;
-      const double d = (at[c] - atb[n * FB + (long)(k + 1) * A + q]) / c2dtts * vit;
-      a.dt_conv[c] = d;
-      a.tend[c] += d;
-      atb[n * FB + (long)(k + 1) * A + q] = at[c];
+  if (lcon != 0) {
+    for (;;) {
+      int lcona = lcon, lconb = lcon + 1;
+      double dztsum = dzp[lcona - 1] + dzp[lconb - 1];
+      double trasum[2];
+      for (int n = 0; n < 2; ++n) {
+        double* X = at + n * F;
+        trasum[n] = X[(long)(lcona - 1) * A] * dzp[lcona - 1] + X[(long)(lconb - 1) * A] * dzp[lconb - 1];
+        const double tramix = trasum[n] / dztsum;
+        X[(long)(lcona - 1) * A] = tramix;
+        X[(long)(lconb - 1) * A] = tramix;
+      }
+      for (;;) {
+        if (lconb != kcon) {
+          if (lower(lconb - 1) > upper(lconb)) {
+            lconb = lconb + 1;
+            dztsum = dztsum + dzp[lconb - 1];
+            for (int n = 0; n < 2; ++n) {
+              double* X = at + n * F;
+              trasum[n] = trasum[n] + X[(long)(lconb - 1) * A] * dzp[lconb - 1];
+              const double tramix = trasum[n] / dztsum;
+              for (int lm = lcona - 1; lm < lconb; ++lm) X[(long)lm * A] = tramix;
+            }
+            continue;
+          }
+        }
+        if (lcona > 1) {
+          if (lower(lcona - 2) > upper(lcona - 1)) {
+            lcona = lcona - 1;
+            dztsum = dztsum + dzp[lcona - 1];
+            for (int n = 0; n < 2; ++n) {
+              double* X = at + n * F;
+              trasum[n] = trasum[n] + X[(long)(lcona - 1) * A] * dzp[lcona - 1];
+              const double tramix = trasum[n] / dztsum;
+              for (int lm = lcona; lm <= lconb; ++lm) X[(long)(lm - 1) * A] = tramix;
+            }
+            continue;
+          }
+        }
+        break;
+      }
+      if (lconb == kcon) break;
+      lcon = lconb;
+      bool done = false;
+      for (;;) {
+        lcon = lcon + 1;
+        if (lcon == kcon) { done = true; break; }
+        if (lower(lcon - 1) <= upper(lcon)) continue;
+        break;
+      }
+      if (done) break;
     }
+  }
+}
+
+// The tendency diagnostics and atb = at of every cell (convadj.cpp:258-276),
+// level by level (blockIdx.z: tracer and level): 48 B per cell and tracer.
+__global__ void __launch_bounds__(256) k_convadj_tend(const __grid_constant__ Arena a, double dts, double inv_dts) {
+  const long A = a.A;
+  const int k = blockIdx.y, n = blockIdx.z;
+  const double* __restrict__ at = a.at[a.cur] + n * a.F + k * A;
+  double* __restrict__ atb = a.atb[a.cur] + n * a.FB + (k + 1) * A;
+  double* __restrict__ tend = a.tend + n * a.F + k * A;
+  double* __restrict__ conv = a.dt_conv + n * a.F + k * A;
+  const long q0 = (long)blockIdx.x * (4 * 256) + threadIdx.x;
+  double x[4], b[4], d[4];
+  int kz[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const long q = q0 + c * 256;
+    if (q < A) {
+      x[c] = at[q];
+      b[c] = atb[q];
+      d[c] = tend[q];
+      kz[c] = a.kmt[q];
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const long q = q0 + c * 256;
+    if (q < A) {
+      const double dt = quotient(x[c] - b[c], dts, inv_dts) * (k < kz[c] ? 1.0 : 0.0);
+      __stcs(conv + q, dt);
+      tend[q] = d[c] + dt;
+      atb[q] = x[c];
+    }
+  }
 }
 
 // ---------------------------------------------------------------- icesnow
@@ -292,9 +340,11 @@ __global__ void k_synth_vel(CellTables t, double ncc1, double* utf, double* vtf,
 }  // namespace
 
 int launch_convadj(const Arena& a, cudaStream_t s) {
-  if (a.km > KMAX_CONV) { set_error("convadj: km > %d", KMAX_CONV); return LT_E_INVALID; }
-  dim3 b(8, 16), g((a.imt + 7) / 8, (a.jmt + 15) / 16);
-  k_convadj<<<g, b, 0, s>>>(a);
+  if (a.km > kConvLevels) { set_error("convadj: km > %d", kConvLevels); return LT_E_INVALID; }
+  dim3 b(32, 4), g((a.imt + 31) / 32, (a.jmt + 3) / 4);
+  k_convadj<<<g, b, 12 * a.km * sizeof(double), s>>>(a);
+  LT_LAUNCHED();
+  k_convadj_tend<<<dim3((unsigned)((a.A + 1023) / 1024), a.km, 2), 256, 0, s>>>(a, a.p.dts, quotient_reciprocal(a.p.dts));
   LT_LAUNCHED();
   return LT_OK;
 }
