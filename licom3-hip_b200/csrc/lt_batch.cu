@@ -30,7 +30,7 @@ struct lt_batch {
   bool mixed = false;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, evx = nullptr;
-  lt_batch_config cfg{kMixedCtasPerSm, 8, 1};
+  lt_batch_config cfg{kMixedCtasPerSm, kMixedContTileY, 1};
   MemberDesc* d_desc[2] = {nullptr, nullptr};   // per parity
   double* scratch = nullptr;                     // column scratch, kMixedCtasPerSm CTAs per SM
   int km_max = 0, max_imt = 0, max_jmt = 0;
@@ -126,7 +126,7 @@ int enqueue_step(lt_batch* b, int p) {
   if ((rc = launch_small_batch_pre(b->d_desc[p], nmem, b->max_imt, b->max_jmt, b->max_cols, s))) return rc;
   if (b->mixed) {
     if ((rc = launch_continuity_mixed_batch(b->d_desc[p], (int)b->m.size(), b->max_imt, b->max_jmt,
-                                            b->cfg.continuity_tile_y, s)))
+                                            b->km_max, b->cfg.continuity_tile_y, s)))
       return rc;
     if ((rc = launch_tracer_mixed_batch(b->d_desc[p], (int)b->m.size(), b->total_items, b->scratch, b->km_max,
                                         b->sms * b->cfg.column_ctas_per_sm, s)))

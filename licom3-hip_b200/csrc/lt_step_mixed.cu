@@ -276,7 +276,7 @@ struct ContSmem {
 };
 constexpr uint32_t kContLevelBytes = 4 * CRR * CRW * sizeof(float);
 
-__global__ void __launch_bounds__(CBX * kContTileY) k_cont_tma32(Arena a, const __grid_constant__ TracerMaps maps) {
+__device__ __forceinline__ void cont_tma_tile(const Arena& a, const TracerMaps& maps) {
   extern __shared__ __align__(128) unsigned char smem_ct[];
   ContSmem& S = *reinterpret_cast<ContSmem*>(smem_ct);
   constexpr int NT = CBX * kContTileY;
@@ -363,6 +363,11 @@ __global__ void __launch_bounds__(CBX * kContTileY) k_cont_tma32(Arena a, const 
   }
   if (!col_here) return;
   cont_finish(a, qo, kz, P, ps, NT);
+}
+
+__global__ void __launch_bounds__(CBX * kContTileY)
+    k_cont_tma32(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps) {
+  cont_tma_tile(a, maps);
 }
 
 __global__ void __launch_bounds__(CBX * kContTileY) k_cont_march32(Arena a) {
@@ -479,6 +484,23 @@ __global__ void __launch_bounds__(CBX * CBY) k_cont_batch(const MemberDesc* __re
     reinterpret_cast<uint4*>(s_arena)[t] = reinterpret_cast<const uint4*>(&g)[t];
   __syncthreads();
   cont_tile<CBY>(*reinterpret_cast<const Arena*>(s_arena), blockIdx.x, blockIdx.y);
+}
+
+// the same with the TMA-fed march, its tile height, for members whose level
+// boxes come by TMA (the others march by plain loads); km_max levels of
+// partial sums in shared memory
+constexpr size_t cont_smem(int km) { return sizeof(ContSmem) + sizeof(float) * CBX * kContTileY * (size_t)km; }
+__global__ void __launch_bounds__(CBX * kContTileY) k_cont_batch_tma(const MemberDesc* __restrict__ mem) {
+  __shared__ __align__(16) unsigned char s_arena[sizeof(Arena)];
+  const MemberDesc& d = mem[blockIdx.z];
+  if ((int)blockIdx.x * CBX >= d.a.imt || (int)blockIdx.y * kContTileY >= d.a.jmt) return;
+  const int tid = threadIdx.y * CBX + threadIdx.x;
+  for (int t = tid; t < (int)(sizeof(Arena) / 16); t += CBX * kContTileY)
+    reinterpret_cast<uint4*>(s_arena)[t] = reinterpret_cast<const uint4*>(&d.a)[t];
+  __syncthreads();
+  const Arena& a = *reinterpret_cast<const Arena*>(s_arena);
+  if (d.tma) cont_tma_tile(a, d.maps);
+  else cont_tile<kContTileY>(a, blockIdx.x, blockIdx.y);
 }
 
 }  // namespace
@@ -1402,6 +1424,8 @@ int launch_tracer_tma_mixed(const Arena& a, const TracerMaps& maps, bool tma, cu
 }
 
 int prepare_tracer_mixed_batch() {
+  LT_CUDA_OK(cudaFuncSetAttribute(k_cont_batch_tma, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)cont_smem(kMixedMaxLevels)));
   LT_CUDA_OK(cudaFuncSetAttribute(k_tracer_mixed_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)mx_batch_smem(kMixedMaxLevels)));
   return LT_OK;
@@ -1416,11 +1440,13 @@ int launch_tracer_mixed_batch(const MemberDesc* mem, int nmem, long total, doubl
   return LT_OK;
 }
 
-int launch_continuity_mixed_batch(const MemberDesc* mem, int nmem, int max_imt, int max_jmt, int cby,
+int launch_continuity_mixed_batch(const MemberDesc* mem, int nmem, int max_imt, int max_jmt, int km_max, int cby,
                                   cudaStream_t s) {
   const unsigned gx = (max_imt + CBX - 1) / CBX;
   switch (cby) {
-    case 4: k_cont_batch<4><<<dim3(gx, (max_jmt + 3) / 4, nmem), dim3(CBX, 4), 0, s>>>(mem); break;
+    case kContTileY:
+      k_cont_batch_tma<<<dim3(gx, (max_jmt + kContTileY - 1) / kContTileY, nmem), dim3(CBX, kContTileY), cont_smem(km_max), s>>>(mem);
+      break;
     case 8: k_cont_batch<8><<<dim3(gx, (max_jmt + 7) / 8, nmem), dim3(CBX, 8), 0, s>>>(mem); break;
     case 16: k_cont_batch<16><<<dim3(gx, (max_jmt + 15) / 16, nmem), dim3(CBX, 16), 0, s>>>(mem); break;
     default: set_error("continuity tile height %d not built (4, 8, 16)", cby); return LT_E_INVALID;
@@ -1443,13 +1469,12 @@ int launch_continuity_mixed(const Arena& a, const TracerMaps& maps, bool tma, cu
     static int attr_dev = -1;
     int dev = 0;
     LT_CUDA_OK(cudaGetDevice(&dev));
-    const size_t psm = sizeof(float) * CBX * kContTileY;   // partial sums per level
     if (attr_dev != dev) {
       LT_CUDA_OK(cudaFuncSetAttribute(k_cont_tma32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(sizeof(ContSmem) + psm * kMixedMaxLevels)));
+                                      (int)cont_smem(kMixedMaxLevels)));
       attr_dev = dev;
     }
-    k_cont_tma32<<<g, b, sizeof(ContSmem) + psm * a.km, s>>>(a, maps);
+    k_cont_tma32<<<g, b, cont_smem(a.km), s>>>(a, maps);
   } else {
     k_cont_march32<<<g, b, 0, s>>>(a);
   }

@@ -84,10 +84,11 @@ int launch_column_fp64(const Arena& a, const TracerMaps& maps, bool tma, cudaStr
 int prepare_column_fp64();
 // Batched forms (mixed precision): nmem members, total work items, one
 // persistent column launch of `grid` CTAs with per-CTA scratch of km_max
-// levels; continuity over every member's tiles with tiles of 32 x cby columns.
+// levels; continuity over every member's tiles with tiles of 32 x cby columns
+// (the TMA-fed march at its own tile height).
 int launch_tracer_mixed_batch(const MemberDesc* mem, int nmem, long total, double* scratch, int km_max, int grid,
                               cudaStream_t s);
-int launch_continuity_mixed_batch(const MemberDesc* mem, int nmem, int max_imt, int max_jmt, int cby,
+int launch_continuity_mixed_batch(const MemberDesc* mem, int nmem, int max_imt, int max_jmt, int km_max, int cby,
                                   cudaStream_t s);
 // The small kernels of a batch step for every member in one launch each:
 // surface fluxes, the SSS-norm tree (one launch per tree pass; max_cols is
