@@ -312,23 +312,41 @@ __device__ __forceinline__ void laplace_column(const Arena& a, int i, int j, int
   const double dtn = a.dtn[q], dts = a.dts[q], dte = a.dte[q], dtw = a.dtw[q], ahf = a.ahf[q];
   const double* __restrict__ atb = a.atb[a.cur];
   double* __restrict__ d2 = a.atb[a.cur ^ 1];
-#pragma unroll 2
-  for (int k = k0; k < k1; ++k) {
-    const long c0 = (long)(k + 1) * A + q;
-    double h[2] = {0.0, 0.0}, cc = 0.0;
-    auto term = [&](bool there, long at, double cf) {
-      if (there) {
-        h[0] += cf * atb[at];
-        h[1] += cf * atb[FB + at];
-        cc -= cf;
-      }
-    };
-    term(k < kq.n, c0 - imt, dtn);
-    term(k < kq.s, c0 + imt, dts);
-    term(k < kq.e, c0 + 1, dte);
-    term(k < kq.w, c0 - 1, dtw);
+  // two levels' loads together, whatever the masks say
+  constexpr int AH = 2;
+  for (int kb = k0; kb < k1; kb += AH) {
+    double x[AH][2][5];   // here, north, south, east, west
 #pragma unroll
-    for (int n = 0; n < 2; ++n) d2[n * FB + c0] = ahf * (cc * atb[n * FB + c0] + h[n]);
+    for (int d = 0; d < AH; ++d)
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const double* p = atb + n * FB + (long)(min(kb + d, k1 - 1) + 1) * A + q;
+        x[d][n][0] = p[0];
+        x[d][n][1] = p[-imt];
+        x[d][n][2] = p[imt];
+        x[d][n][3] = p[1];
+        x[d][n][4] = p[-1];
+      }
+#pragma unroll
+    for (int d = 0; d < AH; ++d) {
+      const int k = kb + d;
+      if (k >= k1) break;
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        double h = 0.0, cc = 0.0;
+        auto term = [&](bool there, double v, double cf) {
+          if (there) {
+            h += cf * v;
+            cc -= cf;
+          }
+        };
+        term(k < kq.n, x[d][n][1], dtn);
+        term(k < kq.s, x[d][n][2], dts);
+        term(k < kq.e, x[d][n][3], dte);
+        term(k < kq.w, x[d][n][4], dtw);
+        d2[n * FB + (long)(k + 1) * A + q] = ahf * (cc * x[d][n][0] + h);
+      }
+    }
   }
 }
 
