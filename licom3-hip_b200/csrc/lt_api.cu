@@ -193,9 +193,10 @@ void plan_arena(Arena& a, Plan& pl) {
   } else {
     D(&a.utf, F); D(&a.vtf, F); D(&a.utl, F); D(&a.vtl, F); D(&a.akt, 2 * F);
     D(&a.utf_out, F); D(&a.vtf_out, F); D(&a.ws, FB); D(&a.uwf, F); D(&a.vsf, F); D(&a.wka, F);
+    // limiter flags: two tracers, a word per patch of 32 columns
+    pl.add(reinterpret_cast<void**>(&a.flags), sizeof(unsigned) * 2 * km * ((a.imt + kColX - 1) / kColX) *
+                                                   ((a.jmt + kColY - 1) / kColY) * (kColX * kColY / 32));
   }
-  pl.add(reinterpret_cast<void**>(&a.flags), sizeof(unsigned) * 2 * km * ((a.imt + kColX - 1) / kColX) * ((a.jmt + kColY - 1) / kColY) *
-                                               (kColX * kColY / 32));
   D(&a.h0f, A); D(&a.h0l, A); D(&a.h0f_out, A); D(&a.net, 2 * A);
   double** two_d[] = {&a.swv, &a.nswv, &a.sst, &a.sss, &a.fresh, &a.seaice, &a.tarea, &a.tarea_r, &a.htw,
                       &a.hts, &a.hun, &a.hue, &a.dxu, &a.dyu, &a.ahf, &a.dtn, &a.dts, &a.dte, &a.dtw,
@@ -590,10 +591,9 @@ int lt_create(const lt_grid* g, const lt_params* p, lt_domain** out) {
     lt_destroy(d);
     return LT_E_CUDA;
   }
-  // one persistent CTA per resident slot (kFp64CtasPerSm, kMixedCtasPerSm
-  // per SM: the kernels' __launch_bounds__ and shared-memory footprints)
-  const long per_sm = d->a.precision == LT_PREC_MIXED ? kMixedCtasPerSm : kFp64CtasPerSm;
-  d->tma_grid = (int)std::min<long>(d->a.col_scratch_slots, (long)sms * per_sm);
+  // one persistent CTA of the mixed column kernel per resident slot
+  // (kMixedCtasPerSm per SM: its __launch_bounds__ and shared memory)
+  d->tma_grid = (int)std::min<long>(d->a.col_scratch_slots, (long)sms * kMixedCtasPerSm);
   if (cudaStreamSynchronize(d->stream) != cudaSuccess) {
     lt_destroy(d);
     return LT_E_CUDA;

@@ -12,17 +12,22 @@
 //   k_thomas      (lt_thomas.cuh) per column and tracer: the implicit half of
 //                 the vertical mixing, the new state, dry levels copied
 //
-// Why three passes.  Only the implicit sweep runs up and down a column; the
-// rest is a stencil that is free in every direction, limited by instruction
-// issue and the FP64 pipe, not by memory (about 240 FP64 operations per cell
-// and tracer).  As one fused march per tile the whole step was a serial chain
-// of levels with two block barriers each, at 16 warps per SM, with a third of
-// the predictors computed twice on tile halos.  Split, every cell's predictor
-// is formed once, a small grid spreads its levels over the SMs and nothing
-// waits at a barrier; the price is the flags and the Laplacian going through
-// memory (17 B per cell and pass).  The Laplacian lives in the new previous
-// state atb[cur^1] and the explicit value in at[cur^1] until the last pass
-// replaces them, so the passes need one byte per cell of storage.
+// Why passes.  Only the implicit sweep runs up and down a column; the rest is a
+// stencil that is free in every direction and limited by instruction issue and
+// the FP64 pipe, not by memory (about 240 FP64 operations per cell and tracer).
+// As one fused march per tile the whole step was a serial chain of levels with
+// two block barriers each, at 16 warps per SM, with a third of the predictors
+// computed twice on tile halos.  Split, every cell's predictor is formed once,
+// a small grid spreads its levels over the SMs and a level has one barrier;
+// the price is the flags and the Laplacian going through memory (16 B per cell
+// and pass).  The Laplacian lives in the new previous state atb[cur^1] and the
+// explicit value in at[cur^1] until the last pass replaces them, so the passes
+// need a bit per cell and tracer of storage.
+//
+// One step of the fused kernel against these passes, 720 x 460 x 55 on the
+// global area-depth curve: 2.66 ms against 0.14 (Laplacian, 3.3 TB/s) + 0.43
+// (limiter: issue slots 49 % busy, FP64 pipe 35 %) + 0.62 (explicit: 52 %, 35 %)
+// + 0.38 (implicit, 3.8 TB/s); 36 x 40 x 55: 270 us against 52.
 #include <cstdio>
 #include "lt_common.cuh"
 #include "lt_thomas.cuh"
@@ -369,6 +374,10 @@ struct Column {
 __device__ __forceinline__ int patches_x() { return gridDim.x * (CX / PX); }
 __device__ __forceinline__ int patches_y() { return gridDim.y * (CY / PY); }
 
+// Bound by issue and FP64 latency at 16 warps per SM.  Both tracers in one
+// thread: transports, masks, metric terms and the level's bookkeeping are 60 %
+// of a level's instructions (with a tracer per thread and 24 warps per SM it
+// took 557 us instead of 425, 720 x 460 x 55 deep).
 template <bool DIAG>
 __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps,
                                                           int kc, int nch, int tma) {
@@ -431,6 +440,7 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
         const double du = f.ue - f.uw, dv = f.vs - f.vn;
         const bool wn = k < kq.n, wso = k < kq.s, ww = k < kq.w, we = k < kq.e;
         const bool wu = k > 0 && k - 1 < kq.c, wl = k + 1 < kq.c;
+        const bool land = !(wn && wso && ww && we && (wl || last));   // beside or below a wet cell
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
           const double* at = L.at[n] + r;
@@ -464,8 +474,9 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
           // a00 > max or a00 < min over the cell and its wet neighbours,
           // without forming the extrema: beyond a wet cell's own value in one
           // direction, and not short of any wet neighbour in it.  Comparing
-          // with both signs flipped turns "below" into "above".  A dry cell's
-          // own value counts as -1e10 and +1e10, so it is asked in both
+          // with both signs flipped turns "below" into "above".  Land counts
+          // as -1e10 for the maximum and +1e10 for the minimum, either -1e10
+          // when turned; a dry cell's own value too, so it is asked in both
           // directions.
           auto beyond = [&](int flip) {
             auto turned = [&](double t) { return __hiloint2double(__double2hiint(t) ^ flip, __double2loint(t)); };
@@ -478,7 +489,7 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
             seen(we, e);
             seen(wu, up[n]);
             seen(wl, lo[n]);
-            return out;
+            return out && !(land && x <= -1.0e10);
           };
           const int below = (int)0x80000000;
           flag[n] = beyond(a00 < c ? below : 0);
@@ -502,7 +513,9 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
 
 // ----------------------------------------------------------- explicit update
 // Without diagnostics the wet inner cells; with them every ring cell of every
-// level (ax, ay, az) and every inner cell (dz, penetrate, the value).
+// level (ax, ay, az) and every inner cell (dz, penetrate, the value).  Bound as
+// k_limit64: 616 us at 720 x 460 x 55 deep (1216 with neighbours loaded through
+// L1 instead of level slots).
 template <bool DIAG>
 __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_constant__ Arena a,
                                                       const __grid_constant__ TracerMaps maps, int kc, int tma) {
@@ -739,7 +752,8 @@ __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_consta
 // Levels per block: a thread keeps the levels above and below in registers,
 // so long chunks read each level once; short ones give a small grid enough
 // blocks (eight rounds of the resident ones) to fill the GPU evenly although
-// most of a shallow grid's levels are dry.
+// most of a shallow grid's levels are dry (360 x 218 x 30: 181 us of column
+// passes; with four rounds 191).
 static int chunk_levels(long column_blocks, int km) {
   const long want = 148L * kColCtas * 8;
   long chunks = (want + column_blocks - 1) / column_blocks;

@@ -8,15 +8,14 @@
 
 namespace lt {
 
-// Column tile of the fused tracer kernel: TX columns along i (one warp) by TY
+// Column tile of the persistent tracer kernels: TX columns along i (one warp) by TY
 // rows along j; one thread per column.
 constexpr int TX = 32;
 constexpr int TY = 8;
 constexpr int TTHREADS = TX * TY;
-// Persistent CTAs per SM of the column kernels (their shared-memory footprint
-// decides): FP64 2 of 256 threads (its tile's metric and biharmonic
-// coefficients staged in shared memory, no register spills), mixed 2 of 256
-// (both tracers' level boxes per CTA).
+// CTAs per SM of the persistent column kernels: the FP64 plain-load one
+// (centred and flux schemes), and the mixed one, whose shared memory (both
+// tracers' level boxes) takes two of 256 threads.
 constexpr int kFp64CtasPerSm = 2;
 constexpr int kMixedCtasPerSm = 2;
 // The mixed column kernel's tile: TX x kMixedTileY columns, one thread each
@@ -164,7 +163,6 @@ int launch_vtl_clobber(const Arena& a, cudaStream_t s);
 
 int launch_f64_to_f32(const double* x, float* y, long n, cudaStream_t s);
 int launch_f32_to_f64(const float* x, double* y, long n, cudaStream_t s);
-int tracer_slots(const Arena& a);
 size_t tree_sum_part_elems(long n);
 
 // a / h for a divisor that serves many dividends: with y = RN(1/h) and a

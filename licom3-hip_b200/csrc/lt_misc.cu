@@ -39,7 +39,8 @@ struct ConvTab {
 // holds two levels in registers instead of 2 x km doubles in local memory,
 // whose traffic was more than the fields' own.  The search loads four levels
 // ahead of their use.  The step over every cell that follows is a kernel of
-// its own, level by level (k_convadj_tend).
+// its own, level by level (k_convadj_tend).  720 x 460 x 55 deep: 164 us and
+// 256 us (6.9 TB/s) against 904 us as one kernel with the arrays.
 constexpr int kConvAhead = 4;
 constexpr int kConvLevels = 128;   // most levels taken
 __global__ void __launch_bounds__(128) k_convadj(const __grid_constant__ Arena a) {

@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(32 * BY) k_cont_march64(Arena a) {
 // (k_cont_levels64: face transports, scaled velocities, divergence; the
 // neighbours' velocities come through L1), then the two sums of each column
 // (k_cont_columns64).  Same expressions in the same order.
-// Step at 36 x 40 x 55 and 360 x 218 x 30: see launch_continuity_fp64.
+// 36 x 40 x 55: 9 + 17 us against the march's 54.
 constexpr int kContChunk = 4;   // levels per thread of k_cont_levels64
 __global__ void __launch_bounds__(256) k_cont_levels64(const __grid_constant__ Arena a) {
   const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
@@ -525,14 +525,17 @@ __global__ void __launch_bounds__(256) k_cont_levels64(const __grid_constant__ A
   const long A = a.A, q = q2(j, i, imt);
   const lt_params& p = a.p;
   const bool north = j >= 1, east = i < imt - 1;
-  // the free-surface factor at U point (uj, ui), 0 where uk, vk are zero
+  // the free-surface factor at a U point where uk, vk are formed (elsewhere
+  // they are zero)
+  auto formed = [&](int uj, int ui) { return uj >= 0 && uj < jmt - 1 && ui >= 1 && ui < imt; };
   auto factor = [&](int uj, int ui) {
-    if (!(uj >= 0 && uj < jmt - 1 && ui >= 1 && ui < imt)) return 0.0;
+    if (!formed(uj, ui)) return 0.0;
     const long c = q2(uj, ui, imt);
     const double work = a.au0[c] * a.stf_ssh[c] + a.aus[c] * a.stf_ssh[c + imt] + a.auw[c] * a.stf_ssh[c - 1] +
                         a.ausw[c] * a.stf_ssh[c + imt - 1];
     return 1.0 + work * a.ohbu[c];
   };
+  const bool u0 = formed(j, i), un = formed(j - 1, i), u1 = formed(j, i + 1), un1 = formed(j - 1, i + 1);
   const bool div = north && east;
   const int kz = a.kmt[q];
   const double f0 = factor(j, i), fn = factor(j - 1, i), f1 = factor(j, i + 1), fn1 = factor(j - 1, i + 1);
@@ -573,9 +576,10 @@ __global__ void __launch_bounds__(256) k_cont_levels64(const __grid_constant__ A
     }
     double wka = 0.0;
     if (div && k <= kz - 1) {
-      auto times = [](double fac, double w) { return fac == 0.0 ? 0.0 : fac * w; };
-      const double uk0 = times(f0, wd[0]), ukn = times(fn, wd[1]), uk1 = times(f1, wd[2]), ukn1 = times(fn1, wd[3]);
-      const double vk0 = times(f0, wb[0]), vkn = times(fn, wb[1]), vk1 = times(f1, wb[2]), vkn1 = times(fn1, wb[3]);
+      const double uk0 = u0 ? f0 * wd[0] : 0.0, ukn = un ? fn * wd[1] : 0.0;
+      const double uk1 = u1 ? f1 * wd[2] : 0.0, ukn1 = un1 ? fn1 * wd[3] : 0.0;
+      const double vk0 = u0 ? f0 * wb[0] : 0.0, vkn = un ? fn * wb[1] : 0.0;
+      const double vk1 = u1 ? f1 * wb[2] : 0.0, vkn1 = un1 ? fn1 * wb[3] : 0.0;
       const double e = (uk1 + ukn1) * htw_e;
       const double w = (uk0 + ukn) * htw_o;
       const double s = (vk1 + vk0) * hts_o;
@@ -1112,16 +1116,6 @@ int launch_continuity_fp64(const Arena& a, cudaStream_t s) {
   k_cont_march64<BY><<<g, b, 0, s>>>(a);
   LT_LAUNCHED();
   return LT_OK;
-}
-
-int tracer_slots(const Arena& a) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long ntiles = (long)((a.imt + TX - 1) / TX) * ((a.jmt + TY - 1) / TY);
-  long slots = (long)sms * 4;
-  if (slots > 2 * ntiles) slots = 2 * ntiles;
-  return (int)slots;
 }
 
 int launch_tracer_fp64(const Arena& a, cudaStream_t s, int slots) {
