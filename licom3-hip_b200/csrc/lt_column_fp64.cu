@@ -358,6 +358,7 @@ __device__ __forceinline__ void laplace_column(const Arena& a, int i, int j, int
 
 constexpr int kLaplaceLevels = 8;
 __global__ void __launch_bounds__(128) k_laplace64(const __grid_constant__ Arena a) {
+  chain_grid();
   const int k0 = blockIdx.z * kLaplaceLevels;
   laplace_column(a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, k0 + kLaplaceLevels);
 }
@@ -382,6 +383,7 @@ __device__ __forceinline__ int patches_y() { return gridDim.y * (CY / PY); }
 template <bool DIAG>
 __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps,
                                                           int kc, int nch, int tma) {
+  chain_grid();
   extern __shared__ __align__(128) unsigned char smem_col[];
   LimitSmem& S = *reinterpret_cast<LimitSmem*>(smem_col);
   const Column col;
@@ -520,6 +522,7 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
 template <bool DIAG>
 __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_constant__ Arena a,
                                                       const __grid_constant__ TracerMaps maps, int kc, int tma) {
+  chain_grid();
   extern __shared__ __align__(128) unsigned char smem_col[];
   ExplicitSmem& S = *reinterpret_cast<ExplicitSmem*>(smem_col);
   const Column col;
@@ -788,15 +791,16 @@ int launch_column_fp64(const Arena& a, const TracerMaps& maps, bool tma, cudaStr
   // on a large one in a kernel of its own, at three times the occupancy.
   const bool together = (long)gx * gy * nch < 148L * kColCtas * 4;
   if (!together) {
-    k_laplace64<<<dim3(gx, (a.jmt + 3) / 4, (a.km + kLaplaceLevels - 1) / kLaplaceLevels), dim3(CX, 4), 0, s>>>(a);
-    LT_LAUNCHED();
+    if (int rc = launch_chained(k_laplace64, dim3(gx, (a.jmt + 3) / 4, (a.km + kLaplaceLevels - 1) / kLaplaceLevels),
+                                dim3(CX, 4), 0, s, a))
+      return rc;
   }
-  auto kl = a.diagnostics ? k_limit64<true> : k_limit64<false>;
-  kl<<<dim3(gx, gy, together ? 2 * nch : nch), CT, sizeof(LimitSmem), s>>>(a, maps, kc, nch, t);
-  LT_LAUNCHED();
-  auto ke = a.diagnostics ? k_explicit64<true> : k_explicit64<false>;
-  ke<<<grid, CT, sizeof(ExplicitSmem), s>>>(a, maps, kc, t);
-  LT_LAUNCHED();
+  if (int rc = launch_chained(a.diagnostics ? k_limit64<true> : k_limit64<false>,
+                              dim3(gx, gy, together ? 2 * nch : nch), dim3(CT), sizeof(LimitSmem), s, a, maps, kc, nch, t))
+    return rc;
+  if (int rc = launch_chained(a.diagnostics ? k_explicit64<true> : k_explicit64<false>, grid, dim3(CT),
+                              sizeof(ExplicitSmem), s, a, maps, kc, t))
+    return rc;
   return a.diagnostics ? launch_thomas<double, true>(a, maps, tma, s) : launch_thomas<double, false>(a, maps, tma, s);
 }
 

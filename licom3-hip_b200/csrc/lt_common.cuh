@@ -132,6 +132,41 @@ long long launch_counter();
 void count_launches(int n);
 void set_error(const char* fmt, ...);
 
+// The kernels of a small grid's step are launched as a chain (programmatic
+// dependent launch): a kernel's blocks may be placed as soon as every block of
+// the one before it has started, and wait in chain_grid(), their first
+// statement, until it has finished and its writes are visible.  That hides the
+// gaps between launches, which such a step is largely made of.
+__device__ __forceinline__ void chain_grid() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Launches a kernel that begins with chain_grid(): with fewer blocks than SMs
+// as a link of the chain (it finds room beside the one before it; five FP64
+// steps of 36 x 40 x 55 take 418 us instead of 468), else in plain stream order
+// (waiting blocks of a large grid take the places of working ones: 360 x 218 x
+// 30 in FP64 takes 1448 us chained, 1342 in plain order), and so inside a
+// stream capture.
+constexpr long kChainBlocks = 148;
+template <class... P, class... A>
+int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  LT_CUDA_OK(cudaStreamIsCapturing(s, &cap));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = cap == cudaStreamCaptureStatusNone && (long)grid.x * grid.y * grid.z < kChainBlocks ? 1 : 0;
+  LT_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+  count_launches(1);
+  return LT_OK;
+}
+
 // host launchers (defined in the step translation units)
 // the surface kernel in two parts: the SSH mean (h0f_out, stf_ssh), which the
 // continuity needs, and the surface fluxes, net and the mixing floor (which

@@ -115,6 +115,7 @@ __global__ void k_surface_fluxes(Arena a) {
 
 // both, where the forcing is already there
 __global__ void k_surface(const __grid_constant__ Arena a) {
+  chain_grid();
   surface_col(a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
 }
 
@@ -176,6 +177,7 @@ struct PartTerm {   // block sums of other blocks of this launch: past L1
   __device__ double operator()(long m) const { return __ldcg(x + m); }
 };
 __global__ void k_sss_norm(const __grid_constant__ Arena a) {
+  chain_grid();
   long n = (long)a.nx * a.ny, nb = gridDim.x;
   tree_block(SssTerm{a.tarea, a.net + a.A, a.kmt, a.nx, a.imt}, n, a.red_part, blockIdx.x);
   __shared__ int last;
@@ -344,7 +346,8 @@ constexpr int kCont64TileY = 8;   // tile height of the FP64 continuity march (4
 // step).  The column divergence W accumulates in level order during the
 // march; w is integrated upward afterwards from the wka the march wrote.
 template <int BY>
-__global__ void __launch_bounds__(32 * BY) k_cont_march64(Arena a) {
+__global__ void __launch_bounds__(32 * BY) k_cont_march64(const __grid_constant__ Arena a) {
+  chain_grid();
   constexpr int BX = 32, UX = BX + 1, UY = BY + 1, UN = UX * UY, NT = BX * BY;
   constexpr int NPT = (UN + NT - 1) / NT, NST = 3;
   __shared__ double s_st[NST][4][UN];   // staged utf, utl, vtf, vtl of three levels
@@ -519,6 +522,7 @@ __global__ void __launch_bounds__(32 * BY) k_cont_march64(Arena a) {
 // 36 x 40 x 55: 9 + 17 us against the march's 54.
 constexpr int kContChunk = 4;   // levels per thread of k_cont_levels64
 __global__ void __launch_bounds__(256) k_cont_levels64(const __grid_constant__ Arena a) {
+  chain_grid();
   const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
   const int imt = a.imt, jmt = a.jmt;
   if (i >= imt || j >= jmt) return;
@@ -591,6 +595,7 @@ __global__ void __launch_bounds__(256) k_cont_levels64(const __grid_constant__ A
 }
 
 __global__ void __launch_bounds__(128) k_cont_columns64(const __grid_constant__ Arena a) {
+  chain_grid();
   const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
   const int imt = a.imt, km = a.km;
   if (!(j >= 1 && j < a.jmt - 1 && i >= 1 && i < imt - 1)) return;
@@ -999,6 +1004,7 @@ __global__ void k_halo_state(Arena a, int n) {
 // surface flux net (both tracers), whose ghost cells nothing reads within the
 // step.
 __global__ void k_halo_state_parts(const __grid_constant__ Arena a) {
+  chain_grid();
   const int n = blockIdx.z, k = blockIdx.y;
   const int imt = a.imt, jmt = a.jmt;
   if (n == 2) {
@@ -1065,9 +1071,7 @@ int launch_ssh(const Arena& a, cudaStream_t s) {
 
 int launch_surface(const Arena& a, cudaStream_t s) {
   dim3 b(32, 8), g((a.imt + 31) / 32, (a.jmt + 7) / 8);
-  k_surface<<<g, b, 0, s>>>(a);
-  LT_LAUNCHED();
-  return LT_OK;
+  return launch_chained(k_surface, g, b, 0, s, a);
 }
 
 int launch_surface_fluxes(const Arena& a, cudaStream_t s) {
@@ -1088,9 +1092,7 @@ size_t tree_sum_part_elems(long n) {
 
 int launch_interior_sum_sss(const Arena& a, cudaStream_t s) {
   const long n = (long)a.nx * a.ny, nb = (n + 2 * RB - 1) / (2 * RB);
-  k_sss_norm<<<(unsigned)nb, RB, 0, s>>>(a);
-  LT_LAUNCHED();
-  return LT_OK;
+  return launch_chained(k_sss_norm, dim3((unsigned)nb), dim3(RB), 0, s, a);
 }
 
 int launch_tree_sum(const double* x, long n, double* part, double* out, cudaStream_t s) {
@@ -1107,15 +1109,10 @@ int launch_continuity_fp64(const Arena& a, cudaStream_t s) {
   constexpr int BY = kCont64TileY;
   dim3 b(32, BY), g((a.imt + 31) / 32, (a.jmt + BY - 1) / BY);
   if (continuity_by_levels((long)g.x * g.y)) {
-    k_cont_levels64<<<dim3(g.x, g.y, (a.km + kContChunk - 1) / kContChunk), b, 0, s>>>(a);
-    LT_LAUNCHED();
-    k_cont_columns64<<<dim3(g.x, (a.jmt + 3) / 4), dim3(32, 4), 0, s>>>(a);
-    LT_LAUNCHED();
-    return LT_OK;
+    if (int rc = launch_chained(k_cont_levels64, dim3(g.x, g.y, (a.km + kContChunk - 1) / kContChunk), b, 0, s, a)) return rc;
+    return launch_chained(k_cont_columns64, dim3(g.x, (a.jmt + 3) / 4), dim3(32, 4), 0, s, a);
   }
-  k_cont_march64<BY><<<g, b, 0, s>>>(a);
-  LT_LAUNCHED();
-  return LT_OK;
+  return launch_chained(k_cont_march64<BY>, g, b, 0, s, a);
 }
 
 int launch_tracer_fp64(const Arena& a, cudaStream_t s, int slots) {
@@ -1143,9 +1140,7 @@ int launch_tracer_fp64(const Arena& a, cudaStream_t s, int slots) {
 
 int launch_halo_state(const Arena& a, cudaStream_t s) {
   if (!a.diagnostics) {
-    k_halo_state_parts<<<dim3(kHaloParts, a.km, 3), 256, a.imt * sizeof(double), s>>>(a);
-    LT_LAUNCHED();
-    return LT_OK;
+    return launch_chained(k_halo_state_parts, dim3(kHaloParts, a.km, 3), dim3(256), a.imt * sizeof(double), s, a);
   }
   if (int rc = launch_halo_r8(a.net, 2, a.imt, a.jmt, a.ew_cyclic, a.tripole, s)) return rc;
   // with diagnostics, salinity's dt_diff reads temperature's new ghost values

@@ -367,10 +367,12 @@ __device__ __forceinline__ void cont_tma_tile(const Arena& a, const TracerMaps& 
 
 __global__ void __launch_bounds__(CBX * kContTileY)
     k_cont_tma32(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps) {
+  chain_grid();
   cont_tma_tile(a, maps);
 }
 
-__global__ void __launch_bounds__(CBX * kContTileY) k_cont_march32(Arena a) {
+__global__ void __launch_bounds__(CBX * kContTileY) k_cont_march32(const __grid_constant__ Arena a) {
+  chain_grid();
   cont_tile<kContTileY>(a, blockIdx.x, blockIdx.y);
 }
 
@@ -380,6 +382,7 @@ __global__ void __launch_bounds__(CBX * kContTileY) k_cont_march32(Arena a) {
 // the sums of each column, with the roundings of the march's parked sums.
 constexpr int kContChunk32 = 4;
 __global__ void __launch_bounds__(256) k_cont_levels32(const __grid_constant__ Arena a) {
+  chain_grid();
   const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
   const int imt = a.imt, jmt = a.jmt;
   if (i >= imt || j >= jmt) return;
@@ -430,6 +433,7 @@ __global__ void __launch_bounds__(256) k_cont_levels32(const __grid_constant__ A
 }
 
 __global__ void __launch_bounds__(128) k_cont_columns32(const __grid_constant__ Arena a) {
+  chain_grid();
   const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 4 + threadIdx.y;
   const int imt = a.imt, km = a.km;
   if (!(j >= 1 && j < a.jmt - 1 && i >= 1 && i < imt - 1)) return;
@@ -1352,7 +1356,8 @@ __device__ __forceinline__ MxLevel* mixed_levels() {
 // from land (a copy) to the full column, so a fixed deal left the CTAs with
 // the deepest tiles working alone at the end.
 __global__ void __launch_bounds__(MTH, kMixedCtasPerSm)
-    k_tracer_mixed(Arena a, const __grid_constant__ TracerMaps maps, int ntx, long ntiles, int tma) {
+    k_tracer_mixed(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps, int ntx, long ntiles, int tma) {
+  chain_grid();
   MxSmem& S = mixed_smem_init();
   MxLevel* lv = mixed_levels();
   stage_levels(lv, a);
@@ -1418,9 +1423,7 @@ int launch_tracer_tma_mixed(const Arena& a, const TracerMaps& maps, bool tma, cu
                                     (int)mx_smem_bytes(kMixedMaxLevels)));
     attr_dev = dev;
   }
-  k_tracer_mixed<<<grid, MTH, sm, s>>>(a, maps, ntx, ntiles, tma ? 1 : 0);
-  LT_LAUNCHED();
-  return LT_OK;
+  return launch_chained(k_tracer_mixed, dim3(grid), dim3(MTH), sm, s, a, maps, ntx, ntiles, tma ? 1 : 0);
 }
 
 int prepare_tracer_mixed_batch() {
@@ -1459,11 +1462,9 @@ int launch_continuity_mixed(const Arena& a, const TracerMaps& maps, bool tma, cu
   dim3 b(CBX, kContTileY), g((a.imt + CBX - 1) / CBX, (a.jmt + kContTileY - 1) / kContTileY);
   const unsigned rows = (a.jmt + 7) / 8;
   if (continuity_by_levels((long)g.x * rows)) {
-    k_cont_levels32<<<dim3(g.x, rows, (a.km + kContChunk32 - 1) / kContChunk32), dim3(32, 8), 0, s>>>(a);
-    LT_LAUNCHED();
-    k_cont_columns32<<<dim3(g.x, (a.jmt + 3) / 4), dim3(32, 4), 0, s>>>(a);
-    LT_LAUNCHED();
-    return LT_OK;
+    if (int rc = launch_chained(k_cont_levels32, dim3(g.x, rows, (a.km + kContChunk32 - 1) / kContChunk32), dim3(32, 8), 0, s, a))
+      return rc;
+    return launch_chained(k_cont_columns32, dim3(g.x, (a.jmt + 3) / 4), dim3(32, 4), 0, s, a);
   }
   if (tma) {
     static int attr_dev = -1;
@@ -1474,12 +1475,9 @@ int launch_continuity_mixed(const Arena& a, const TracerMaps& maps, bool tma, cu
                                       (int)cont_smem(kMixedMaxLevels)));
       attr_dev = dev;
     }
-    k_cont_tma32<<<g, b, cont_smem(a.km), s>>>(a, maps);
-  } else {
-    k_cont_march32<<<g, b, 0, s>>>(a);
+    return launch_chained(k_cont_tma32, g, b, cont_smem(a.km), s, a, maps);
   }
-  LT_LAUNCHED();
-  return LT_OK;
+  return launch_chained(k_cont_march32, g, b, 0, s, a);
 }
 
 }  // namespace lt

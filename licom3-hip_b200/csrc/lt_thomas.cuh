@@ -219,6 +219,7 @@ __device__ __forceinline__ void copy_dry(const Arena& a, int x0, int y0, int n) 
 template <class AK, bool DIAG>
 __global__ void __launch_bounds__(kThT) k_thomas(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps,
                                                  int tma) {
+  chain_grid();
   // blockIdx.x: the column of tiles and the block's part (the sweep of either
   // tracer, the dry levels of either tracer): the copying blocks only move
   // memory, the sweeping ones mostly wait for their chains of divisions, so
@@ -242,9 +243,9 @@ int prepare_thomas() {
 template <class AK, bool DIAG>
 int launch_thomas(const Arena& a, const TracerMaps& maps, bool tma, cudaStream_t s) {
   const size_t sm = sizeof(ThomasSmem<AK>);
-  k_thomas<AK, DIAG><<<dim3((a.imt + kThX - 1) / kThX * (DIAG ? 2 : 4), (a.jmt + kThY - 1) / kThY), kThT, sm, s>>>(a, maps, tma ? 1 : 0);
-  LT_LAUNCHED();
-  return LT_OK;
+  return launch_chained(k_thomas<AK, DIAG>,
+                        dim3((a.imt + kThX - 1) / kThX * (DIAG ? 2 : 4), (a.jmt + kThY - 1) / kThY), dim3(kThT), sm, s, a,
+                        maps, tma ? 1 : 0);
 }
 
 }  // namespace lt

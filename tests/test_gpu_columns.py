@@ -44,6 +44,33 @@ def test_column_passes_bitexact(lt, nx, ny, km, cyclic, tripole, hyp, diagnostic
         assert g.tobytes() == r.tobytes(), (n, float(np.nanmax(np.abs(g - r))), int((g != r).sum()))
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nx,ny,km", [(8, 8, 3), (36, 40, 55), (130, 90, 7), (300, 130, 12)])
+def test_chained_launches_keep_order(lt, nx, ny, km, precision):
+    """Steps launched without a pause, of two domains in turn on their own
+    streams and of grids on both sides of the chained launches' line, equal
+    steps with the host waiting after each."""
+    syn = lt.Synth(nx, ny, km, seed=5, forced=1)
+    f = syn.all_fields()
+    doms = []
+    for _ in range(3):
+        d = lt.TracerDomain(nx, ny, km, syn.params, precision=lt.PREC_FP64 if precision == "fp64" else lt.PREC_MIXED)
+        for n in lt.INPUT_FIELDS:
+            d.set(n, f[n])
+        doms.append(d)
+    for _ in range(6):
+        doms[0].step(1)
+        doms[0].sync()
+    for _ in range(3):
+        doms[1].step(2)
+        doms[2].step(2)
+    for n in ("AT", "ATB", "NET"):
+        r = doms[0].get(n)
+        for d in doms[1:]:
+            assert d.get(n).tobytes() == r.tobytes(), n
+
+
 def test_quotient_by_reciprocal_is_correctly_rounded():
     """The face divisions' two-step form (a*y, then q - y*(h*q - a) twice, y the
     rounded reciprocal) equals IEEE division for dividends and divisors of the
