@@ -404,13 +404,15 @@ __global__ void __launch_bounds__(128, 5)
       else theta_r = atan(ric / rit);
       if (fabs(theta_r) > 2.0e0 * C.pi4) { quit = true; break; }
       // cos and sin of the angle from its own components: it points along
-      // (rit, ric), or against it where rit < 0, and is turned by pi below -pi/4
+      // (rit, ric), or against it where rit < 0, and is turned by pi below
+      // -pi/4.  Not where the squares in ra_r overflow or lose their bits
+      // below the smallest normal number: there from the angle.
       double turn = rit < 0.0e0 ? -1.0 : 1.0;
       if (theta_r < -C.pi4) {
         theta_r += 4.0e0 * C.pi4;
         turn = -turn;
       }
-      bool moved = fabs(rit) <= 0.0e0;
+      bool moved = fabs(rit) <= 0.0e0 || !(ra_r > 1.0e-130 && ra_r < 1.0e150);
       const int jt0 = (int)((theta_r + C.pi4) * C.inv_dth);
       int it0 = jt0 - NTH, it1 = it0 + 1;
       double th0 = it0 * T.deltheta_r, th1 = it1 * T.deltheta_r;

@@ -88,3 +88,31 @@ def test_turb_then_tracer_step(lt, tab):
 def test_turb_one_degree_tripole(lt, tab):
     syn, f = case(lt, 13, 1, nx=360, ny=218, km=30, dz_top=10.0, dz_bot=250.0)
     compare(gpu_run(lt, syn, f, tab, lt.PREC_FP64), oracle_run(lt, syn, f))
+
+
+def with_ri(f, rng, rit, rid):
+    """The case with Ri and Ri_d replaced at every interface by draws from the
+    given values."""
+    g = dict(f)
+    g["RIT"] = r = rng.choice(rit, size=f["RIT"].shape)
+    g["RICDTTMS"] = d = rid(r)
+    # not at the critical angles, tan = -1/2 and -2, where the background is a
+    # step and an arctangent's last bit decides
+    with np.errstate(all="ignore"):
+        tan = (r - d) / (r + d)
+    d[(np.abs(tan + 0.5) < 1e-6) | (np.abs(tan + 2.0) < 1e-6)] *= 0.9
+    return g
+
+
+def test_turb_ri_beyond_the_squares_range(lt, tab):
+    """Ri and Ri_d whose squares underflow or overflow, zeros and denormals
+    among them: the background's angle keeps its components' ratio."""
+    syn, f = case(lt, 3, 1)
+    rng = np.random.default_rng(5)
+    tiny = np.array([5e-324, 1e-310, 1e-300, 1e-200, 1e-162, 1e-154, 1e-140, 1e-120, 0.0])
+    huge = np.array([1e140, 1e152, 1e155, 1e200, 1e300])
+    for values in (tiny, huge, np.concatenate([-tiny, tiny, [0.1, 0.2]]), np.concatenate([-huge, huge, [0.1, 0.2]])):
+        g = with_ri(f, rng, values, lambda r: r * rng.choice([-1.2, -1.0, -0.4, 0.0, 0.4, 1.0, 1.2], size=r.shape))
+        dom = gpu_run(lt, syn, g, tab, lt.PREC_FP64)
+        assert np.isfinite(dom.get("AKT")).all() and np.isfinite(dom.get("AKMT")).all()
+        compare(dom, oracle_run(lt, syn, g))
