@@ -113,6 +113,7 @@ struct TurbTabDev {
   double rib0, gmax, gm, gm1;   // the first and last Ri; where the two grids turn geometric
 };
 
+  int plain;                    // every entry and step is zero or of a magnitude div_fast takes
 #define LT_CUDA_OK(call)                                   \
   do {                                                     \
     cudaError_t e_ = (call);                               \

@@ -2,9 +2,10 @@
 // step's vertical mixing (turb_cu with turb_device, interp1d_expabs,
 // interp2d_expabs, formld and eplatidepend_fun, readyc.cpp:880-1612, with
 // TIDEMIX as the reference is configured).  Compiled with -fmad=false: the
-// operation order is the reference's term for term; the transcendental
-// functions (atan, acosh, rarely sin, cos) are CUDA's, so results agree with the
-// reference to a few units in the last place, not bit for bit.
+// operation order is the reference's term for term but for the cosine and sine
+// of the background's angle; the transcendental functions (atan, acosh, rarely
+// sin, cos, log) are CUDA's, so results agree with the reference to a few units
+// in the last place, not bit for bit.
 //
 // One thread per column.  Where the reference first fills per-column work
 // arrays (wp1, wp3, wp7, wp8 in [i][j][k] order) and then walks them, this
@@ -20,11 +21,14 @@
 //
 // Bound by latency: a long chain per level (square roots, atan, acosh,
 // quotients, table gathers) at 20 warps per SM, instruction fetch across its
-// branches, and idle lanes where neighbours differ in stability.  4.00 -> 2.14
+// branches, and idle lanes where neighbours differ in stability.  4.00 -> 2.23
 // ms at 720 x 460 x 55 on the global area-depth curve with interleaved tables,
 // brackets found without logarithms and the angle's cosine and sine taken from
-// its components; four, six or eight blocks per SM instead of five: 2.29, 2.42,
-// 2.27 ms.
+// its components, which are nearer the exact ones than those of the rounded
+// angle (root mean square 0.9e-16 against 6e-11 for the cosine).  Quotients
+// that share a divisor are formed from its reciprocal and rounded as divisions
+// (ratio).  Four, six or eight blocks per SM instead of five were slower by
+// 7, 13 and 6 %.
 #include <cmath>
 #include <new>
 #include <vector>
@@ -54,9 +58,7 @@ __device__ __forceinline__ double sgn(double x, double y) { return y >= 0.0 ? fa
 struct TurbConst {
   double pi4;               // atan(1.0)
   double eplat_den;         // wavelat(f_30, an0)
-  double inv_ncc;           // 1/ncc (0: divide)
-  double inv_dth;           // 1/deltheta_r
-  double inv_dri, inv_da;   // 1/dri, 1/dand2on2
+  double inv_ncc, inv_dth, inv_dri, inv_da;   // reciprocals: ncc (0: divide), deltheta_r, dri, dand2on2
   float log2_gm, per_log2;     // 2-D tables: log2(rib[mt + mt0]), 1/log2(rri)
   float log2_gm1, per_log21;   // zero-shear table
 };
@@ -67,30 +69,60 @@ __device__ __forceinline__ double eplat(const TurbConst& C, double f, double an)
   return anum / C.eplat_den;
 }
 
+// a / h with y = 1/h: where the tables allow it (TurbTabDev::plain: every entry
+// and grid step within 1e-100 .. 1e100 or zero) the division's bits without its
+// code, which this kernel has no room for in the instruction cache (thirteen
+// quotients a level with the general form's test and division: 3.54 ms)
+template <bool PLAIN>
+__device__ __forceinline__ double ratio(double a, double h, double y) {
+  return PLAIN ? div_fast(a, h, y) : a / h;
+}
+
 // Indices (offset by MT) of the entries that bracket x on an "expabs" grid
-// (linear spacing delta up to grid[mt + mt0] = gm, geometric beyond), which
-// interp1d_expabs and interp2d_expabs find from a quotient or a logarithm and
-// a correction (readyc.cpp:922-941, 1014-1031).  Here the first guess is a
-// single-precision one and the grid itself decides: lo towards zero, an entry
-// that x meets counts as lo.
+// (linear spacing delta up to grid[mt + mt0] = gm, geometric ratio rat beyond),
+// lo towards zero, which interp1d_expabs and interp2d_expabs find from a
+// quotient or a logarithm and a correction by one (readyc.cpp:922-941,
+// 1014-1031).  The linear part takes the same quotient.  In the geometric part
+// the first guess is a single-precision logarithm and the grid itself decides;
+// where x meets an entry, which side of it counts is left to the logarithm's
+// rounding, so there (rarely) it is formed as the reference does: the tables'
+// interpolation and the realizable limit are steps at an entry.
 struct Bracket {
   int lo, hi;
 };
-__device__ __forceinline__ Bracket bracket(double x, const double* __restrict__ g, double gm, double inv_delta,
-                                           float log2_gm, float per_log2) {
+__device__ __noinline__ int met_entry(double ax, const double* __restrict__ g, int s, double gm, double rat) {
+  const double ti = (double)MT0 + ((log(ax) - log(gm)) / log(rat));
+  int m = max(1, min(MT, (int)ti + 1));
+  if (fabs(g[MT + s * m]) < ax) m = min(MT, m + 1);
+  else if (m > 1 && fabs(g[MT + s * (m - 1)]) > ax) --m;
+  return m;
+}
+template <bool PLAIN>
+__device__ __forceinline__ Bracket bracket(double x, const double* __restrict__ g, double gm, double delta,
+                                           double inv_delta, double rat, float log2_gm, float per_log2) {
   const double ax = fabs(x);
   const int s = x >= 0.0 ? 1 : -1;
+  const bool linear = ax < gm;
   int m;
-  if (ax < gm) m = 1 + (int)(ax * inv_delta);
+  if (linear) m = 1 + (int)ratio<PLAIN>(ax, delta, inv_delta);
   else m = 1 + MT0 + (int)((__log2f((float)ax) - log2_gm) * per_log2);
   m = max(1, min(MT, m));
-  while (m < MT && fabs(g[MT + s * m]) <= ax) ++m;
-  while (m > 1 && fabs(g[MT + s * (m - 1)]) > ax) --m;
+  double above = fabs(g[MT + s * m]), below = fabs(g[MT + s * (m - 1)]);
+  while (m < MT && above < ax) {
+    below = above;
+    above = fabs(g[MT + s * ++m]);
+  }
+  while (m > 1 && below > ax) {
+    above = below;
+    below = fabs(g[MT + s * (--m - 1)]);
+  }
+  if (!linear && (above == ax || below == ax)) m = met_entry(ax, g, s, gm, rat);
   return {MT + s * (m - 1), MT + s * m};
 }
 
 // interp1d_expabs (readyc.cpp:915-973): false, outputs left as they were, when
 // x falls outside the bracketing entries
+template <bool PLAIN>
 __device__ __noinline__ bool interp1d(double x, const TurbTabDev& T, const TurbConst& C, double out[4]) {
   const double* x1 = T.and2on2a1;
   if (x > x1[2 * MT]) x = x1[2 * MT];
@@ -98,7 +130,7 @@ __device__ __noinline__ bool interp1d(double x, const TurbTabDev& T, const TurbC
   const double gm = x1[MT + MT0], gmax = x1[2 * MT];
   Bracket b;
   if (fabs(x) >= gm && fabs(x) >= gmax) b.lo = b.hi = x >= 0.0 ? 2 * MT : 0;
-  else b = bracket(x, x1, gm, C.inv_da, C.log2_gm1, C.per_log21);
+  else b = bracket<PLAIN>(x, x1, gm, T.dand2on2, C.inv_da, T.rnd2on2, C.log2_gm1, C.per_log21);
   const double x0 = x1[b.lo], xh = x1[b.hi];
   if ((x > 0.0e0 && (x < x0 || x > xh)) || (x < 0.0e0 && (x > x0 || x < xh))) return false;
   const double dta = xh - x0;
@@ -126,6 +158,7 @@ __device__ __forceinline__ Stab quad_at(const TurbTabDev& T, long c) {
   return {u.x, u.y, v.x, v.y};
 }
 
+template <bool PLAIN>
 __device__ __forceinline__ bool interp2d(double& ri, double& rid, const TurbTabDev& T, const TurbConst& C, Stab& out) {
   const double* rib = T.rib;
   const double rmax = T.gmax, rmin = T.rib0, gm = T.gm;
@@ -163,7 +196,7 @@ __device__ __forceinline__ bool interp2d(double& ri, double& rid, const TurbTabD
   const double x_ri = ri, x_rid = rid;
   Bracket d, r;
   if (fabs(x_rid) >= gm && fabs(x_rid) >= rmax) d.lo = d.hi = x_rid >= 0.0 ? 2 * MT : 0;
-  else d = bracket(x_rid, rib, gm, C.inv_dri, C.log2_gm, C.per_log2);
+  else d = bracket<PLAIN>(x_rid, rib, gm, T.dri, C.inv_dri, T.rri, C.log2_gm, C.per_log2);
   const double d0 = rib[d.lo], d1 = rib[d.hi];
   if ((x_rid > 0.0e0 && (x_rid < d0 || x_rid > d1)) || (x_rid < 0.0e0 && (x_rid > d0 || x_rid < d1))) return false;
   if (x_ri > fmin(T.rilim[d.lo], T.rilim[d.hi])) {
@@ -171,25 +204,31 @@ __device__ __forceinline__ bool interp2d(double& ri, double& rid, const TurbTabD
     return true;
   }
   if (fabs(x_ri) >= gm && fabs(x_ri) >= rmax) r.lo = r.hi = x_ri >= 0.0 ? 2 * MT : 0;
-  else r = bracket(x_ri, rib, gm, C.inv_dri, C.log2_gm, C.per_log2);
+  else r = bracket<PLAIN>(x_ri, rib, gm, T.dri, C.inv_dri, T.rri, C.log2_gm, C.per_log2);
   const double r0 = rib[r.lo], r1 = rib[r.hi];
   if ((x_ri > 0.0e0 && (x_ri < r0 || x_ri > r1)) || (x_ri < 0.0e0 && (x_ri > r0 || x_ri < r1))) return false;
   const Stab t00 = quad_at(T, (long)N1 * d.lo + r.lo);
   out = t00;
   if (d.hi != d.lo) {
     const Stab t10 = quad_at(T, (long)N1 * d.hi + r.lo), t01 = quad_at(T, (long)N1 * d.lo + r.hi);
-    const double gd = 1.0 / (d1 - d0), gr = 1.0 / (r1 - r0);
+    // one reciprocal per direction serves four quotients, rounded as divisions
+    const double dridta = d1 - d0, drita = r1 - r0;
+    const double gd = 1.0 / dridta, gr = 1.0 / drita;
     const double drid = x_rid - d0, dri = x_ri - r0;
-    out.slq2 = t00.slq2 + (t01.slq2 - t00.slq2) * gr * dri + (t10.slq2 - t00.slq2) * gd * drid;
-    out.sm = t00.sm + (t01.sm - t00.sm) * gr * dri + (t10.sm - t00.sm) * gd * drid;
-    out.sh = t00.sh + (t01.sh - t00.sh) * gr * dri + (t10.sh - t00.sh) * gd * drid;
-    out.ss = t00.ss + (t01.ss - t00.ss) * gr * dri + (t10.ss - t00.ss) * gd * drid;
+    auto plane = [&](double v00, double v10, double v01) {
+      return v00 + ratio<PLAIN>(v01 - v00, drita, gr) * dri + ratio<PLAIN>(v10 - v00, dridta, gd) * drid;
+    };
+    out.slq2 = plane(t00.slq2, t10.slq2, t01.slq2);
+    out.sm = plane(t00.sm, t10.sm, t01.sm);
+    out.sh = plane(t00.sh, t10.sh, t01.sh);
+    out.ss = plane(t00.ss, t10.ss, t01.ss);
   }
   return true;
 }
 // the background's second look-up (rare), kept out of the level loop's code
+template <bool PLAIN>
 __device__ __noinline__ bool interp2d_back(double& ri, double& rid, const TurbTabDev& T, const TurbConst& C, Stab& out) {
-  return interp2d(ri, rid, T, C, out);
+  return interp2d<PLAIN>(ri, rid, T, C, out);
 }
 
 // The column's interface values (the reference's wp1, wp3, wp8 at level k,
@@ -212,6 +251,7 @@ struct Iface {
 
 constexpr int kTurbLevels = 256;   // most levels a domain may have
 
+template <bool PLAIN>
 __global__ void __launch_bounds__(128, 5)
     k_turb(const __grid_constant__ Arena a, const __grid_constant__ TurbTabDev T, const __grid_constant__ TurbConst C,
            double ncc_f, double fricmx, double wndmix) {
@@ -359,7 +399,7 @@ __global__ void __launch_bounds__(128, 5)
       const double and2 = ridk / (rik + 1.0e-25) * an2;
       const double and2on2 = and2 / (an2 + 1.0e-25);
       double v[4];
-      if (interp1d(and2on2, T, C, v)) {
+      if (interp1d<PLAIN>(and2on2, T, C, v)) {
         amtaun2 = v[0];
         st.sm = v[1];
         st.sh = v[2];
@@ -367,7 +407,7 @@ __global__ void __launch_bounds__(128, 5)
       }
       st.slq2 = (-amtaun2) / ((b1 * b1) * rik + 1.0e-25);
     } else {
-      interp2d(ri1, rid1, T, C, st);
+      interp2d<PLAIN>(ri1, rid1, T, C, st);
       if (st.slq2 < 0.0e0) { quit = true; break; }
       if (st.slq2 == 0.0e0) ifbelow = 1.0;
     }
@@ -390,7 +430,7 @@ __global__ void __launch_bounds__(128, 5)
     // the latitude factor enters through the background (Ri > 0) and, below
     // the mixed part, for Ri >= 0 only
     double epson2 = kEpson2;
-    if (!(an2 < 0.0e0) && (rik > 0.0e0 || ri1 >= 0.0e0)) {
+    if (!(an2 < 0.0e0) && (!(rik <= 0.0e0) || ri1 >= 0.0e0)) {
       double ep = ifnofsmall == 1.0 ? 0.0e0 : eplat(C, fabs(coriol), an);
       ep = fmax(ep, kEplatMin);
       epson2 = kEpson2 * ep;
@@ -406,14 +446,16 @@ __global__ void __launch_bounds__(128, 5)
       // cos and sin of the angle from its own components: it points along
       // (rit, ric), or against it where rit < 0, and is turned by pi below
       // -pi/4.  Not where the squares in ra_r overflow or lose their bits
-      // below the smallest normal number: there from the angle.
+      // below the smallest normal number, nor where Ri is small beside Ri_d:
+      // there cos + sin is mostly the angle's rounding, which decides whether
+      // the column goes on.
       double turn = rit < 0.0e0 ? -1.0 : 1.0;
       if (theta_r < -C.pi4) {
         theta_r += 4.0e0 * C.pi4;
         turn = -turn;
       }
-      bool moved = fabs(rit) <= 0.0e0 || !(ra_r > 1.0e-130 && ra_r < 1.0e150);
-      const int jt0 = (int)((theta_r + C.pi4) * C.inv_dth);
+      bool moved = fabs(rit) <= 0.0e0 || !(ra_r > 1.0e-130 && ra_r < 1.0e150 && rik > 1.0e-3 * ra_r);
+      const int jt0 = (int)ratio<PLAIN>(theta_r + C.pi4, T.deltheta_r, C.inv_dth);
       int it0 = jt0 - NTH, it1 = it0 + 1;
       double th0 = it0 * T.deltheta_r, th1 = it1 * T.deltheta_r;
       if ((th0 <= T.theta_rcrp) && (theta_r > T.theta_rcrp)) {
@@ -434,7 +476,7 @@ __global__ void __launch_bounds__(128, 5)
       if ((it1 > 3 * NTH) || (it0 < -NTH)) { quit = true; break; }
       double dth = theta_r - th0;
       const double br0 = T.back_ra_r[NTH + it0];
-      double back_ra_r1 = br0 + dth * ((T.back_ra_r[NTH + it1] - br0) * C.inv_dth);
+      double back_ra_r1 = br0 + dth * ratio<PLAIN>(T.back_ra_r[NTH + it1] - br0, T.deltheta_r, C.inv_dth);
       int ifrafglt = 0;
       if ((theta_r <= T.theta_rcrp) || (theta_r >= T.theta_rcrn)) {
         if (back_ra_r1 > ra_r) {
@@ -443,8 +485,11 @@ __global__ void __launch_bounds__(128, 5)
         }
       }
       if (back_ra_r1 < 0.0e0) { quit = true; break; }
+      // where the second look-up takes them, from the angle too: small Ri are
+      // their own components, and one that meets a table entry would go to a
+      // side of it that the angle's rounding decides
       double back_rit1, back_ric1;
-      if (moved) {
+      if (moved || ifrafglt == 1) {
         back_rit1 = cos(theta_r) * back_ra_r1;
         back_ric1 = sin(theta_r) * back_ra_r1;
       } else {
@@ -456,15 +501,18 @@ __global__ void __launch_bounds__(128, 5)
       if (ifrafglt == 1) {
         double back_rid1 = back_rit1 - back_ric1, bri = back_ri1;
         Stab b = back;
-        interp2d_back(bri, back_rid1, T, C, b);
+        interp2d_back<PLAIN>(bri, back_rid1, T, C, b);
         back_ri1 = bri;
         back = b;
       } else {
-        dth = (theta_r - it0 * T.deltheta_r) * C.inv_dth;
-        back.sm = T.sm_r1[NTH + it0] + dth * (T.sm_r1[NTH + it1] - T.sm_r1[NTH + it0]);
-        back.sh = T.sh_r1[NTH + it0] + dth * (T.sh_r1[NTH + it1] - T.sh_r1[NTH + it0]);
-        back.ss = T.ss_r1[NTH + it0] + dth * (T.ss_r1[NTH + it1] - T.ss_r1[NTH + it0]);
-        back.slq2 = T.slq2_r1[NTH + it0] + dth * (T.slq2_r1[NTH + it1] - T.slq2_r1[NTH + it0]);
+        dth = theta_r - it0 * T.deltheta_r;
+        auto between = [&](const double* tab) {
+          return tab[NTH + it0] + dth * ratio<PLAIN>(tab[NTH + it1] - tab[NTH + it0], T.deltheta_r, C.inv_dth);
+        };
+        back.sm = between(T.sm_r1);
+        back.sh = between(T.sh_r1);
+        back.ss = between(T.ss_r1);
+        back.slq2 = between(T.slq2_r1);
       }
       if (back.slq2 < 0.0e0) { quit = true; break; }
     }
@@ -552,9 +600,21 @@ __global__ void __launch_bounds__(128, 5)
   a.akmt[(long)(km - 1) * A + q] = 0.0;
 }
 
-// one table into its place among the interleaved four
-__global__ void k_interleave(const double* __restrict__ x, double* __restrict__ quad, long n) {
-  for (long m = (long)blockIdx.x * blockDim.x + threadIdx.x; m < n; m += (long)gridDim.x * blockDim.x) quad[4 * m] = x[m];
+// zero, or a magnitude ratio's quick form may divide
+__host__ __device__ inline bool plain_entry(double x) {
+  const double v = fabs(x);
+  return v == 0.0 || (v > 1.0e-100 && v < 1.0e100);
+}
+
+// one table into its place among the interleaved four; odd: set where an
+// entry is not plain_entry
+__global__ void k_interleave(const double* __restrict__ x, double* __restrict__ quad, long n, int* odd) {
+  bool plain = true;
+  for (long m = (long)blockIdx.x * blockDim.x + threadIdx.x; m < n; m += (long)gridDim.x * blockDim.x) {
+    quad[4 * m] = x[m];
+    plain = plain && plain_entry(x[m]);
+  }
+  if (!plain) *odd = 1;
 }
 
 }  // namespace
@@ -575,7 +635,8 @@ int launch_turb(const Arena& a, const TurbTabDev& T, int ncc, double dfricmx, cu
   // warps of 8 x 4 columns: depths and stability alike, so fewer idle lanes
   // (720 x 460 x 55 deep: 2.14 ms, rows of 32 2.38)
   dim3 b(8, 16), g((a.imt + 7) / 8, (a.jmt + 15) / 16);
-  k_turb<<<g, b, 0, s>>>(a, T, C, (double)(float)ncc, dfricmx * 1.0e+4, a.p.dwndmix * 1.0e+4);
+  (T.plain ? k_turb<true> : k_turb<false>)<<<g, b, 0, s>>>(a, T, C, (double)(float)ncc, dfricmx * 1.0e+4,
+                                                           a.p.dwndmix * 1.0e+4);
   LT_LAUNCHED();
   return LT_OK;
 }
@@ -607,10 +668,11 @@ int lt_turb_tables_create(const lt_turb_tables* h, lt_turb_tab** out) {
   lt_turb_tab* t = new (std::nothrow) lt_turb_tab;
   if (!t) return LT_E_OOM;
   TurbTabDev& T = t->t;
+  const int* odd = nullptr;        // set while the 2-D tables are interleaved
   std::vector<double> rilim(n1);   // the realizable limit of Ri itself
   for (int m = 0; m < N1; ++m) rilim[m] = h->rib[MT + h->irimax[m]];
   const Item items[] = {
-      {nullptr, 4 * n2 * 8, (const void**)&T.quad},
+      {nullptr, 4 * n2 * 8, (const void**)&T.quad}, {nullptr, sizeof(int), (const void**)&odd},
       {h->rib, n1 * 8, (const void**)&T.rib},         {rilim.data(), n1 * 8, (const void**)&T.rilim},
       {h->and2on2a1, n1 * 8, (const void**)&T.and2on2a1}, {h->amtaun2a1, n1 * 8, (const void**)&T.amtaun2a1},
       {h->sma1, n1 * 8, (const void**)&T.sma1},       {h->sha1, n1 * 8, (const void**)&T.sha1},
@@ -634,21 +696,32 @@ int lt_turb_tables_create(const lt_turb_tables* h, lt_turb_tab** out) {
     if (it.src && e == cudaSuccess) e = cudaMemcpy(base + off, it.src, it.bytes, cudaMemcpyHostToDevice);
     off += (it.bytes + 255) / 256 * 256;
   }
+  if (e == cudaSuccess) e = cudaMemset(const_cast<int*>(odd), 0, sizeof(int));
   const double* tabs[4] = {h->slq2b, h->smb, h->shb, h->ssb};
   for (int m = 0; m < 4 && e == cudaSuccess; ++m) {
     e = cudaMemcpy(one, tabs[m], n2 * 8, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) break;
-    k_interleave<<<1184, 256>>>(one, const_cast<double*>(T.quad) + m, (long)n2);
+    k_interleave<<<1184, 256>>>(one, const_cast<double*>(T.quad) + m, (long)n2, const_cast<int*>(odd));
     lt::count_launches(1);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
   }
   cudaFree(one);
+  int any_odd = 0;
+  if (e == cudaSuccess) e = cudaMemcpy(&any_odd, odd, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) {
     cudaFree(base);
     delete t;
     return cuda_fail(e, "lt_turb_tables_create");
   }
+  // the grids' steps and the 1-D tables on the host
+  bool plain = !any_odd && plain_entry(h->dri) && plain_entry(h->dand2on2) && plain_entry(h->deltheta_r);
+  for (size_t m = 0; m < n1 && plain; ++m)
+    plain = plain_entry(h->rib[m]) && (m == 0 || (h->rib[m] != h->rib[m - 1] && plain_entry(h->rib[m] - h->rib[m - 1])));
+  const double* angle[] = {h->back_ra_r, h->sm_r1, h->sh_r1, h->ss_r1, h->slq2_r1};
+  for (const double* tab : angle)
+    for (size_t m = 0; m < nb && plain; ++m) plain = plain_entry(tab[m]);
+  T.plain = plain ? 1 : 0;
   T.rib0 = h->rib[0];
   T.gm = h->rib[MT + MT0];
   T.gmax = h->rib[2 * MT];

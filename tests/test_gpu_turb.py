@@ -116,3 +116,36 @@ def test_turb_ri_beyond_the_squares_range(lt, tab):
         dom = gpu_run(lt, syn, g, tab, lt.PREC_FP64)
         assert np.isfinite(dom.get("AKT")).all() and np.isfinite(dom.get("AKMT")).all()
         compare(dom, oracle_run(lt, syn, g))
+
+
+@pytest.mark.parametrize("part", ["linear", "geometric_rid", "geometric_ri", "ends"])
+def test_turb_ri_on_table_entries(lt, tab, part):
+    """Ri and Ri_d that meet table entries, lie one rounding off them, on both
+    sides of the linear part's last entry, at the ends and beyond them.  Where
+    an entry of the geometric part is met, the side is left to a logarithm's
+    rounding, so the other of the two stays off the entries there (the
+    realizable limit is a step)."""
+    import turb_synth
+    t = tables(lt)
+    rib, mt, mt0 = t["rib"], turb_synth.MT, turb_synth.MT0
+    syn, f = case(lt, 8, 1)
+    rng = np.random.default_rng(9)
+    i = np.arange(-mt, mt + 1)
+    lin, geo = rib[np.abs(i) < mt0], rib[np.abs(i) > mt0]
+    near = np.concatenate([lin, np.nextafter(lin, -np.inf), np.nextafter(lin, np.inf)])
+    near = np.concatenate([near, lin[np.abs(lin) < 0.5], lin[np.abs(lin) < 0.5]])   # about the realizable limit
+    free = lambda r: rng.uniform(-3.0, 3.0, size=r.shape)
+    if part == "linear":
+        g = with_ri(f, rng, near, lambda r: rng.choice(near, size=r.shape))
+    elif part == "geometric_rid":
+        off = rng.uniform(-1.0, 1.0, 4000)
+        off = off[np.abs(np.abs(off) - 0.2) > 0.12]          # clear of the realizable limits, 0.1 .. 0.3
+        g = with_ri(f, rng, off, lambda r: rng.choice(geo, size=r.shape))
+    elif part == "geometric_ri":
+        g = with_ri(f, rng, geo, free)
+    else:
+        ends = [rib[0], rib[-1], np.nextafter(rib[-1], 0.0), np.nextafter(rib[-1], np.inf), 3.0 * rib[-1],
+                rib[mt + mt0], np.nextafter(rib[mt + mt0], 0.0), np.nextafter(rib[mt + mt0], np.inf), 0.0, -0.0]
+        ends = np.array(ends + [-e for e in ends])
+        g = with_ri(f, rng, ends, lambda r: rng.choice(np.concatenate([ends, [0.3, -0.3]]), size=r.shape))
+    compare(gpu_run(lt, syn, g, tab, lt.PREC_FP64), oracle_run(lt, syn, g))
