@@ -111,9 +111,9 @@ struct TurbTabDev {
   const double *back_ra_r, *sm_r1, *sh_r1, *ss_r1, *slq2_r1;
   double rri, rnd2on2, dri, deltheta_r, b1, theta_rcrp, theta_rcrn, dand2on2;
   double rib0, gmax, gm, gm1;   // the first and last Ri; where the two grids turn geometric
+  int plain;                    // every entry and step is zero or of a magnitude div_fast takes
 };
 
-  int plain;                    // every entry and step is zero or of a magnitude div_fast takes
 #define LT_CUDA_OK(call)                                   \
   do {                                                     \
     cudaError_t e_ = (call);                               \
