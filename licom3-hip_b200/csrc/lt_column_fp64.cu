@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
   int k1 = k0;   // end of this thread's levels
   if (ring) {
     kq = load_kmt5(a, q);
-    k1 = min(k0 + kc, DIAG ? km : kq.deepest());
+    k1 = min(k0 + kc, DIAG ? flow_end(a, q, kq.c) : kq.deepest());
   }
   init_bars<kLimitDepth>(S, tma != 0);
   const int kend = block_max(S, k1);
@@ -515,8 +515,9 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
 }
 
 // ----------------------------------------------------------- explicit update
-// Without diagnostics the wet inner cells; with them every ring cell of every
-// level (ax, ay, az) and every inner cell (dz, penetrate, the value).  Bound as
+// Without diagnostics the wet inner cells; with them every ring cell (ax, ay,
+// az) and every inner cell (dz, penetrate, the value) above the block's
+// dry_from.  Bound as
 // k_limit64: 616 us at 720 x 460 x 55 deep (1216 with neighbours loaded through
 // L1 instead of level slots).
 template <bool DIAG>
@@ -538,12 +539,13 @@ __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_consta
   int k1 = k0;
   if (DIAG ? ring : inner) {
     kq = load_kmt5(a, q);
-    k1 = min(k0 + kc, DIAG ? km : kq.c);
+    k1 = min(k0 + kc, DIAG ? flow_end(a, q, kq.c) : kq.c);
   }
   const int kz = kq.c;
   init_bars<kExplicitDepth>(S, tma != 0);
   const int kend = block_max(S, k1);
   if (k0 >= kend) return;
+  if (DIAG && ring) k1 = kend;   // the block's columns alike: the last pass takes them from there
   start_levels<true, kExplicitDepth>(S, a, maps, tma != 0, x0, y0, k0, kend);
   load_block(S, a, x0, y0, k0, kc);
   const lt_params& p = a.p;

@@ -86,6 +86,8 @@ struct alignas(16) Arena {   // copied into shared memory as 16-byte words
   double *uwf, *vsf;          // face transports u_wface, v_sface [km][jmt][imt]
   double *wka;                // horizontal divergence [km][jmt][imt]
   unsigned* flags;            // [2][km] limiter flags, one word per patch of 8 x 4 columns
+  int* kflow;                 // [jmt][imt] one past the deepest level with a transport through the column's west or
+                              // south face or w (diagnostics on grids whose continuity marches, else null)
   // mixed precision: f32 storage of the dynamics inputs, mixing and the
   // derived fields (the f64 pointers above are null for these; the
   // horizontal divergence lives only in registers of the continuity march)
@@ -182,6 +184,7 @@ int launch_continuity_fp64(const Arena& a, cudaStream_t s);
 // march, which reads and writes each field once (360 x 218 x 30: 60 against
 // 79 us in FP64, 39 against 60 us in mixed precision).
 inline bool continuity_by_levels(long tiles) { return tiles < 74; }
+inline long continuity_tiles(const Arena& a) { return (long)((a.imt + 31) / 32) * ((a.jmt + 7) / 8); }
 int launch_tracer_fp64(const Arena& a, cudaStream_t s, int slots);
 int launch_assm_dt_restore(const Arena& a, cudaStream_t s);
 int launch_halo_state(const Arena& a, cudaStream_t s);

@@ -448,6 +448,7 @@ __global__ void __launch_bounds__(32 * BY) k_cont_march64(const __grid_constant_
   const double trr = own ? a.tarea_r[qo] : 0.0;
   const int m0 = (ty + 1) * UX + tx, mn = ty * UX + tx;
   double W = 0.0;
+  int kf = 0;   // one past the deepest level with a nonzero west or south face transport or w here
   double dzp_k = a.dzp[0];
   for (int k = 0; k < km; ++k) {
     const int b = k & 1;
@@ -466,13 +467,15 @@ __global__ void __launch_bounds__(32 * BY) k_cont_march64(const __grid_constant_
       __stcs(a.utf_out + c, own_utf * p.oncc);
       __stcs(a.vtf_out + c, own_vtf * p.oncc);
       // the faces outside these ranges stay zero
+      double uwv = 0.0, vsv = 0.0;
       if (flux) {
-        if (j >= 1 && j < jmt - 1) __stcs(a.uwf + c, (wd[mn] * dyu_n + wd[m0] * dyu_o) * 0.25);
-        if (i >= 1 && i < imt - 1) __stcs(a.vsf + c, (wb[m0] * dxu_o + wb[m0 + 1] * dxu_e) * 0.25);
+        if (j >= 1 && j < jmt - 1) __stcs(a.uwf + c, uwv = (wd[mn] * dyu_n + wd[m0] * dyu_o) * 0.25);
+        if (i >= 1 && i < imt - 1) __stcs(a.vsf + c, vsv = (wb[m0] * dxu_o + wb[m0 + 1] * dxu_e) * 0.25);
       } else {
-        if (j >= 1 && j < jmt - 1) __stcs(a.uwf + c, (wd[mn] + wd[m0]) * htw_o * 0.25);
-        if (i >= 1 && i < imt - 1) __stcs(a.vsf + c, (wb[m0] + wb[m0 + 1]) * hts_o * 0.25);
+        if (j >= 1 && j < jmt - 1) __stcs(a.uwf + c, uwv = (wd[mn] + wd[m0]) * htw_o * 0.25);
+        if (i >= 1 && i < imt - 1) __stcs(a.vsf + c, vsv = (wb[m0] + wb[m0 + 1]) * hts_o * 0.25);
       }
+      if (uwv != 0.0 || vsv != 0.0) kf = k + 1;
       double wka = 0.0;
       if (j >= 1 && i < imt - 1 && k <= kz - 1) {
         const double east = (uk[m0 + 1] + uk[mn + 1]) * htw_e;
@@ -490,7 +493,10 @@ __global__ void __launch_bounds__(32 * BY) k_cont_march64(const __grid_constant_
     }
   }
   cp_async_wait<0>();
-  if (!col) return;
+  if (!col) {
+    if (a.kflow && own) a.kflow[qo] = kf;
+    return;
+  }
   const double ohbt = a.ohbt[qo];
   const double fac = 1.0 / (1.0 + a.stf_ssh[qo] * ohbt);
   double wsp = a.ws[qo];
@@ -508,10 +514,13 @@ __global__ void __launch_bounds__(32 * BY) k_cont_march64(const __grid_constant_
       const int k = k0 + c;
       if (k >= km) break;
       const double raw = (k < kz ? 1.0 : 0.0) * (wsp + a.dzp[k - 1] * (W * ohbt + wk[c]));
-      __stcs(a.ws + (long)k * A + qo, raw * fac);
+      const double wv = raw * fac;
+      __stcs(a.ws + (long)k * A + qo, wv);
+      if (wv != 0.0) kf = max(kf, k + 1);
       wsp = raw;
     }
   }
+  if (a.kflow) a.kflow[qo] = kf;
 }
 
 // The same continuity for grids whose tiles do not fill the GPU, where the
@@ -1107,8 +1116,9 @@ int launch_halo_r8(double* f, int nz, int imt, int jmt, int ew_cyclic, int tripo
 
 int launch_continuity_fp64(const Arena& a, cudaStream_t s) {
   constexpr int BY = kCont64TileY;
+  static_assert(BY == 8, "continuity_tiles");
   dim3 b(32, BY), g((a.imt + 31) / 32, (a.jmt + BY - 1) / BY);
-  if (continuity_by_levels((long)g.x * g.y)) {
+  if (continuity_by_levels(continuity_tiles(a))) {
     if (int rc = launch_chained(k_cont_levels64, dim3(g.x, g.y, (a.km + kContChunk - 1) / kContChunk), b, 0, s, a)) return rc;
     return launch_chained(k_cont_columns64, dim3(g.x, (a.jmt + 3) / 4), dim3(32, 4), 0, s, a);
   }

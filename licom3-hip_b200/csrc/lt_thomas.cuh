@@ -38,6 +38,30 @@ struct ThomasSmem {
   int wmax[kThT / 32];
 };
 
+// With diagnostics a column's levels from here down are below its bottom and
+// carry no transport through its four faces or w (kflow of its own column
+// covers its west and south faces and w, that of its east and north neighbours
+// the other two).  They need no flags: a zero transport gives the same signed
+// zero in the upwind and the Lax-Wendroff form of a flux.  The passes leave the
+// levels below the deepest such column of a block of 32 x 4 (dry_from) to
+// dry_levels.
+__device__ __forceinline__ int flow_end(const Arena& a, long q, int kmt) {
+  if (!a.kflow) return a.km;
+  return max(max(kmt, a.kflow[q]), max(a.kflow[q + 1], a.kflow[q - a.imt]));
+}
+// The block's dry_from: one past the deepest flow_end of its ring cells (this
+// thread's at q).  wmax: a word per warp.
+__device__ __forceinline__ int dry_from(const Arena& a, bool ring, long q, int* wmax) {
+  if (!a.kflow) return a.km;
+  int v = __reduce_max_sync(0xffffffffu, ring ? flow_end(a, q, a.kmt[q]) : 0);
+  __syncthreads();   // wmax is free
+  if (threadIdx.x % 32 == 0) wmax[threadIdx.x / 32] = v;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kThT / 32; ++w) v = max(v, wmax[w]);
+  return v;
+}
+
 // Columns of one block: x0.., y0.., tracer n.  DIAG: with the diagnostics of
 // tracer_9 (tend, dt_diff) and the pre-fold values of the top row.
 template <class AK, bool DIAG>
@@ -62,6 +86,13 @@ __device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& m
   int kmax = 0;
 #pragma unroll
   for (int w = 0; w < kThT / 32; ++w) kmax = max(kmax, S.wmax[w]);
+
+  int kout = kz;   // levels of this column the pass writes
+  if (DIAG) {
+    static_assert(kThX == kColX && kThY == kColY, "the passes' blocks");
+    const bool ring = i >= 1 && i < imt - 1 && j >= 1 && j < jmt - 1;
+    kout = dry_from(a, ring, (long)j * imt + i, S.wmax);
+  }
 
   double* __restrict__ at_out = a.at[a.cur ^ 1] + n * a.F;
   double* __restrict__ atb_out = a.atb[a.cur ^ 1] + n * a.FB;
@@ -153,7 +184,7 @@ __device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& m
   constexpr int SUB = 8;
   const uint64_t once = l2_evict_first();
   double x = 0.0;
-  const int kend = DIAG ? km : kz;
+  const int kend = kout;
   double ev[SUB], fv[SUB];
   auto load = [&](int k0) {
 #pragma unroll
@@ -194,7 +225,7 @@ __device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& m
 }
 
 // The dry levels of a block's columns keep their values (with diagnostics the
-// sweep writes them): eight levels' loads ahead of their stores.
+// sweep and dry_levels write them): eight levels' loads ahead of their stores.
 __device__ __forceinline__ void copy_dry(const Arena& a, int x0, int y0, int n) {
   const int i = x0 + threadIdx.x % kThX, j = y0 + threadIdx.x / kThX;
   if (!(i >= 2 && i < a.imt - 2 && j >= 2 && j < a.jmt - 2)) return;
@@ -216,18 +247,138 @@ __device__ __forceinline__ void copy_dry(const Arena& a, int x0, int y0, int n) 
   }
 }
 
+// The levels of a block of columns from dry_from down (every ring cell below
+// its bottom, no transport): the diagnostics of advection_tracer_3 (the upwind
+// form of each flux), of tracer_5 (penetrate, dz) and of tracer_9 (tend,
+// dt_diff, with the value kept: every term is masked) and the new state.
+// All signed zeros and copies: bound by memory, so a block takes a chunk of
+// levels of both tracers, whose transports it reads once, and nothing is written
+// twice.  With such levels in all three passes instead (each read them, the last
+// one wrote the explicit pass's value again) a step with diagnostics took 45.1 ms
+// at 3600 x 2302 x 55 on the linear depth map and 54.4 on the global area-depth
+// curve, now 33.0 and 50.4; 360 x 218 x 30: 496 and 549 us, now 405 and 541.  As
+// a launch of its own: 31.4 and 49.9 ms, but 419 and 567 us.
+constexpr int kDryLevels = 16;
+__device__ __forceinline__ void dry_levels(const Arena& a, int x0, int y0, int chunk, int* wmax) {
+  const int i = x0 + threadIdx.x % kThX, j = y0 + threadIdx.x / kThX;
+  const int imt = a.imt, jmt = a.jmt, km = a.km;
+  const bool ring = i >= 1 && i < imt - 1 && j >= 1 && j < jmt - 1;
+  const bool inner = i >= 2 && i < imt - 2 && j >= 2 && j < jmt - 2;
+  const long A = a.A, F = a.F, FB = a.FB;
+  const long q = (long)j * imt + i;
+  const int from = dry_from(a, ring, q, wmax);
+  int k = max(from, chunk * kDryLevels);
+  const int kend = min(km, (chunk + 1) * kDryLevels);
+  if (!ring || k >= kend) return;
+  const double* __restrict__ at_in = a.at[a.cur] + q;
+  const double* __restrict__ atb_in = a.atb[a.cur] + A + q;   // level 0
+  const double* __restrict__ akt = a.akt + q;
+  const double* __restrict__ uwf = a.uwf + q;
+  const double* __restrict__ vsf = a.vsf + q;
+  const double* __restrict__ ws = a.ws + q;
+  double* __restrict__ at_out = a.at[a.cur ^ 1] + q;
+  double* __restrict__ atb_out = a.atb[a.cur ^ 1] + A + q;
+  const double tr = a.tarea_r[q], swv = inner ? a.swv[q] : 0.0;
+  const double inv = 1.0 / a.p.dts, none = 0.0;   // none: the mask below the bottom
+  long c = (long)k * A;
+  double wk = ws[c];
+  double up[2], x[2], bx[2], mix[2];   // at of levels k-1 and k; atb of level k; mixing flux from above
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    x[n] = at_in[n * F + c];
+    up[n] = k > 0 ? at_in[n * F + c - A] : 0.0;
+    bx[n] = inner ? atb_in[n * FB + c] : 0.0;
+    mix[n] = inner && k > 0 ? akt[n * F + c - A] * (atb_in[n * FB + c - A] - bx[n]) * a.odzt[k] * none : 0.0;
+  }
+  for (; k < kend; ++k, c += A) {
+    const bool last = k == km - 1;
+    const double odzp = a.odzp[k];
+    const double ue = uwf[c + 1], uw = uwf[c], vs = vsf[c], vn = vsf[c - imt];
+    const double w1 = last ? 0.0 : ws[c + A];
+    double lo[2], e[2], w[2], s[2], nn[2], bl[2], ak[2];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const double* p = at_in + n * F + c;
+      e[n] = p[1];
+      w[n] = p[-1];
+      s[n] = p[imt];
+      nn[n] = p[-imt];
+      lo[n] = last ? 0.0 : p[A];
+      bl[n] = inner && !last ? atb_in[n * FB + c + A] : 0.0;
+      ak[n] = inner && !last ? akt[n * F + c] : 0.0;
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const double v = x[n];
+      const long cg = n * F + c + q;
+      const double xe = -(e[n] - v) * fabs(ue) * tr, xw = (v - w[n]) * fabs(uw) * tr;
+      const double ys = -(s[n] - v) * fabs(vs) * tr, yn = (v - nn[n]) * fabs(vn) * tr;
+      const double x0v = (e[n] + v) * ue * tr - (v + w[n]) * uw * tr;
+      const double y0v = ((s[n] + v) * vs - (v + nn[n]) * vn) * tr;
+      const double cx = -v * (ue - uw) * tr * 2.0, cy = -v * (vs - vn) * tr * 2.0;
+      double za, zb1 = 0.0, zb2 = 0.0, zc;
+      if (k > 0) zb1 = -0.5 * fabs(wk) * odzp * (up[n] - v);
+      if (!last) zb2 = 0.5 * fabs(w1) * odzp * (v - lo[n]);
+      if (k == 0) {
+        za = -0.5 * odzp * w1 * (lo[n] + v);
+        zc = odzp * v * w1;
+      } else if (last) {
+        za = 0.5 * odzp * wk * (v + up[n]);
+        zc = -odzp * v * wk;
+      } else {
+        za = 0.5 * odzp * wk * (v + up[n]) - 0.5 * odzp * w1 * (v + lo[n]);
+        zc = -odzp * v * (wk - w1);
+      }
+      __stcs(a.ax + cg, -(x0v + xe + xw + cx));
+      __stcs(a.ay + cg, -(y0v + ys + yn + cy));
+      __stcs(a.az + cg, -(za + zb1 + zb2 + zc));
+      up[n] = v;
+      x[n] = lo[n];
+      if (!inner) continue;
+      if (n == 0) {
+        double pen;
+        if (k == 0) pen = -(swv * a.pen[0] * none) * odzp;
+        else if (last) pen = swv * a.pen[km - 2] * none * odzp;
+        else pen = (swv * a.pen[k - 1] * none - swv * a.pen[k] * none) * odzp;
+        __stcs(a.penetrate + c + q, pen);
+      }
+      const double below = last ? 0.0 : ak[n] * (bx[n] - bl[n]) * a.odzt[k + 1] * none;
+      double dz;
+      if (k == 0) dz = -odzp * below * 0.5;
+      else if (last) dz = odzp * mix[n] * 0.5;
+      else dz = odzp * (mix[n] - below) * 0.5;
+      __stcs(a.dzd + cg, dz);
+      mix[n] = below;
+      bx[n] = bl[n];
+      const double kept = (v - v) * inv * none;   // no change
+      __stcs(a.tend + cg, kept);
+      __stcs(a.dt_diff + cg, k == 0 ? kept - a.stf_n[n * A + q] * 0.5 * odzp : kept);
+      if (j == 2 && a.tripole) a.fold_save[((long)(n * km + k)) * imt + i] = v;
+      __stcs(at_out + n * F + c, v);
+      __stcs(atb_out + n * FB + c, v);
+    }
+    wk = w1;
+  }
+}
+
 template <class AK, bool DIAG>
 __global__ void __launch_bounds__(kThT) k_thomas(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps,
-                                                 int tma) {
+                                                 int tma, int parts) {
   chain_grid();
   // blockIdx.x: the column of tiles and the block's part (the sweep of either
-  // tracer, the dry levels of either tracer): the copying blocks only move
-  // memory, the sweeping ones mostly wait for their chains of divisions, so
-  // the two kinds run side by side
-  constexpr int PARTS = DIAG ? 2 : 4;
-  const int part = blockIdx.x % PARTS, x0 = blockIdx.x / PARTS * kThX, y0 = blockIdx.y * kThY;
-  if (part < 2) thomas_block<AK, DIAG>(a, maps, tma != 0, x0, y0, part);
-  else copy_dry(a, x0, y0, part - 2);
+  // tracer, then the dry levels: of either tracer, with diagnostics a chunk of
+  // levels of both): the copying blocks only move memory, the sweeping ones
+  // mostly wait for their chains of divisions, so the two kinds run side by side
+  if (!DIAG) parts = 4;
+  const int part = blockIdx.x % parts, x0 = blockIdx.x / parts * kThX, y0 = blockIdx.y * kThY;
+  if (part < 2) {
+    thomas_block<AK, DIAG>(a, maps, tma != 0, x0, y0, part);
+  } else if (DIAG) {
+    extern __shared__ __align__(128) unsigned char smem_th[];
+    dry_levels(a, x0, y0, part - 2, reinterpret_cast<ThomasSmem<AK>*>(smem_th)->wmax);
+  } else {
+    copy_dry(a, x0, y0, part - 2);
+  }
 }
 
 // shared-memory size of the pass on the current device (not inside a capture)
@@ -243,9 +394,9 @@ int prepare_thomas() {
 template <class AK, bool DIAG>
 int launch_thomas(const Arena& a, const TracerMaps& maps, bool tma, cudaStream_t s) {
   const size_t sm = sizeof(ThomasSmem<AK>);
-  return launch_chained(k_thomas<AK, DIAG>,
-                        dim3((a.imt + kThX - 1) / kThX * (DIAG ? 2 : 4), (a.jmt + kThY - 1) / kThY), dim3(kThT), sm, s, a,
-                        maps, tma ? 1 : 0);
+  const int parts = !DIAG ? 4 : a.kflow ? 2 + (a.km + kDryLevels - 1) / kDryLevels : 2;
+  return launch_chained(k_thomas<AK, DIAG>, dim3((a.imt + kThX - 1) / kThX * parts, (a.jmt + kThY - 1) / kThY), dim3(kThT),
+                        sm, s, a, maps, tma ? 1 : 0, parts);
 }
 
 }  // namespace lt

@@ -1,14 +1,13 @@
-"""The FP64 column passes (limiter flags, explicit update, implicit sweep) at
-the sizes where their blocks, patches, level chunks and stages can go wrong,
-bit for bit against the oracle: grids one column short of, at and beyond the
-32 x 4 blocks and 8 x 4 patches, level counts around the chunk and stage
-lengths, row pitches with and without TMA boxes, closed and folded boundaries."""
+"""The FP64 column passes (limiter flags, explicit update, implicit sweep, dry
+levels with diagnostics) at the sizes where their blocks, patches, level chunks
+and stages can go wrong, bit for bit against the oracle: grids one column short
+of, at and beyond the 32 x 4 blocks and 8 x 4 patches, chunks of up to 4 levels
+on small grids and of up to 56 on large ones, level counts around the stages'
+eight, row pitches with and without TMA boxes, closed and folded boundaries."""
 import numpy as np
 import pytest
 
 import pyoracle
-
-
 
 CASES = [
     # nx, ny, km, cyclic, tripole, hypsometry
@@ -22,6 +21,23 @@ CASES = [
 ]
 
 
+def compare(lt, syn, f, steps, diagnostics):
+    dom = lt.TracerDomain(syn.nx, syn.ny, syn.km, syn.params, precision=lt.PREC_FP64, diagnostics=diagnostics,
+                          ew_cyclic=bool(syn.cfg.ew_cyclic), tripole=bool(syn.cfg.tripole))
+    o = pyoracle.Oracle(syn.nx, syn.ny, syn.km, syn.params, ew_cyclic=syn.cfg.ew_cyclic, tripole=syn.cfg.tripole)
+    o.load(f)
+    o.sum_order(1)
+    for n in lt.INPUT_FIELDS:
+        dom.set(n, f[n])
+    dom.step(steps)
+    dom.sync()
+    o.step(steps)
+    for n in ("AT", "ATB", "WS", "NET") + (("AX", "AY", "AZ", "DZ", "PENETRATE", "TEND", "DT_DIFF") if diagnostics else ()):
+        g, r = dom.get(n), o.get(n)
+        assert g.tobytes() == r.tobytes(), (n, float(np.nanmax(np.abs(g - r))), int((g != r).sum()))
+    dom.close()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("diagnostics", [False, True])
 @pytest.mark.parametrize("nx,ny,km,cyclic,tripole,hyp", CASES)
@@ -29,19 +45,59 @@ def test_column_passes_bitexact(lt, nx, ny, km, cyclic, tripole, hyp, diagnostic
     syn = lt.Synth(nx, ny, km, seed=17 + nx, forced=1, ew_cyclic=cyclic, tripole=tripole, hypsometry=hyp,
                    cap_north=0 if tripole else 2, cap_south=2)
     f = syn.all_fields()
-    dom = lt.TracerDomain(nx, ny, km, syn.params, precision=lt.PREC_FP64, diagnostics=diagnostics,
-                          ew_cyclic=bool(cyclic), tripole=bool(tripole))
-    o = pyoracle.Oracle(nx, ny, km, syn.params, ew_cyclic=cyclic, tripole=tripole)
-    o.load(f)
-    o.sum_order(1)
-    for n in lt.INPUT_FIELDS:
-        dom.set(n, f[n])
-    dom.step(3)
-    dom.sync()
-    o.step(3)
-    for n in ("AT", "ATB", "WS", "NET") + (("AX", "AY", "AZ", "DZ", "PENETRATE", "TEND", "DT_DIFF") if diagnostics else ()):
-        g, r = dom.get(n), o.get(n)
-        assert g.tobytes() == r.tobytes(), (n, float(np.nanmax(np.abs(g - r))), int((g != r).sum()))
+    compare(lt, syn, f, 3, diagnostics)
+
+
+def large(lt, nx, ny, km, cyclic, tripole, hyp):
+    return lt.Synth(nx, ny, km, seed=3 + km, forced=1, ew_cyclic=cyclic, tripole=tripole, hypsometry=hyp,
+                    cap_north=0 if tripole else 2, cap_south=2)
+
+
+# Grids whose continuity marches (74 tiles and more), with and without TMA row
+# pitches; the larger ones run the Laplacian in a launch of its own and long
+# chunks of levels, whose slots and barriers are used again and again: 28 levels
+# a block at 720 x 460 x 55, 20 at 721 x 461 x 40, 56 at 1180 x 508 x 56.
+LARGE = [
+    (260, 90, 8, 1, 1, 1),
+    (261, 93, 17, 0, 0, 0),
+    (720, 460, 55, 1, 1, 0),
+    (721, 461, 40, 0, 0, 1),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("diagnostics", [False, True])
+@pytest.mark.parametrize("nx,ny,km,cyclic,tripole,hyp", LARGE)
+def test_large_grids_bitexact(lt, nx, ny, km, cyclic, tripole, hyp, diagnostics):
+    syn = large(lt, nx, ny, km, cyclic, tripole, hyp)
+    compare(lt, syn, syn.all_fields(), 2 if nx < 300 else 1, diagnostics)
+
+
+@pytest.mark.gpu
+def test_longest_chunk_bitexact(lt):
+    syn = large(lt, 1180, 508, 56, 1, 1, 1)
+    compare(lt, syn, syn.all_fields(), 1, False)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,km,cyclic,tripole", [(260, 90, 37, 1, 1), (261, 93, 16, 0, 0), (322, 61, 3, 1, 0)])
+def test_dry_levels_with_diagnostics_bitexact(lt, nx, ny, km, cyclic, tripole):
+    """The diagnostics of dry cells, zeros of either sign that depend on every
+    input there: velocities down to a level of each U point's own, above or
+    below the bottom, zeros of both signs beneath; a quarter of the grid and the
+    land in it without any flow."""
+    syn = large(lt, nx, ny, km, cyclic, tripole, 1)
+    f = syn.all_fields()
+    rng = np.random.default_rng(km)
+    jmt, imt = f["KMT"].shape
+    depth = rng.integers(0, km + 1, size=(jmt, imt))
+    depth[:, : imt // 4] = 0
+    depth[jmt // 2 :, imt // 2 :] = np.minimum(depth, 1)[jmt // 2 :, imt // 2 :]
+    flow = np.arange(km)[:, None, None] < depth
+    for n in ("UTF", "VTF", "UTL", "VTL"):
+        v = rng.normal(0.0, 0.1, size=f[n].shape)
+        f[n] = np.where(flow, v, np.copysign(0.0, v))
+    compare(lt, syn, f, 2, True)
 
 
 @pytest.mark.gpu
