@@ -321,11 +321,14 @@ int lt_last_step_ms(lt_domain* dom, float* ms);
 int lt_mark(lt_domain* dom, int which);
 /* Per-phase device timing: lt_profile(dom, 1) records CUDA events around the
  * six launch phases of each step; lt_phase_ms sums them over the recorded
- * steps into ms[0..5] = surface fluxes, SSS-norm sum, net halo, continuity
- * (with the SSH mean it needs), tracer column kernel, state halo, and returns
- * the number of steps.  The continuity is launched first (it needs no
- * forcing); with lt_step_host, the surface-flux phase includes any wait for
- * the forcing copies still in flight after it. */
+ * steps into ms[0..5] = surface fluxes, SSS-norm sum, net halo, continuity,
+ * tracer column kernels, state halo, and returns the number of steps.  The SSH
+ * mean is formed with the surface fluxes; with lt_step_host the continuity
+ * (and the SSH mean before it) is launched first, as it needs no forcing, and
+ * the surface phase includes any wait for the forcing copies still in flight
+ * after it.  The net halo is a launch of its own only with diagnostics: without
+ * them the state halo's launch fills net's ghost cells too and ms[2] is 0 but
+ * for the events. */
 int lt_profile(lt_domain* dom, int on);
 int lt_phase_ms(lt_domain* dom, float* ms, int nphase);
 /* How the column kernels' level slots are filled: 1 = TMA boxes (the default

@@ -318,26 +318,33 @@ int run_step(lt_domain* d, cudaEvent_t forcing_ready) {
   cudaEvent_t* ev = nullptr;
   if (d->profile && d->prof_steps < LT_PROF_STEPS) {
     ev = &d->prof_ev[(size_t)d->prof_steps * (LT_NPHASE + 1)];
+    d->prof_order[d->prof_steps] = forcing_ready ? 1 : 0;
     d->prof_steps++;
   }
   // events bound the phases in launch order (LT_PHASE_ORDER)
   auto mark = [&](int ph) { if (ev) cudaEventRecord(ev[ph], s); };
+  auto continuity = [&] {
+    return a.precision == LT_PREC_MIXED ? launch_continuity_mixed(a, d->maps, d->use_tma, s) : launch_continuity_fp64(a, s);
+  };
   mark(0);
   // the continuity reads the SSH mean and the velocities, not the surface
   // forcing: with a forcing still on its way it comes before the fluxes
-  if ((rc = forcing_ready ? launch_ssh(a, s) : launch_surface(a, s))) return rc;
-  if (a.precision == LT_PREC_MIXED) rc = launch_continuity_mixed(a, d->maps, d->use_tma, s);
-  else rc = launch_continuity_fp64(a, s);
-  if (rc) return rc;
-  mark(1);
   if (forcing_ready) {
+    if ((rc = launch_ssh(a, s)) || (rc = continuity())) return rc;
+    mark(1);
     LT_CUDA_OK(cudaStreamWaitEvent(s, forcing_ready, 0));
     if ((rc = launch_surface_fluxes(a, s))) return rc;
+  } else {
+    if ((rc = launch_surface(a, s))) return rc;
+    mark(1);
+    if ((rc = continuity())) return rc;
   }
   mark(2);
   if ((rc = launch_interior_sum_sss(a, s))) return rc;
   mark(3);
-  mark(4);   // net's ghost cells are filled with the state's
+  // without diagnostics net's ghost cells are filled in the state halo's launch
+  if (a.diagnostics && (rc = launch_halo_r8(a.net, 2, a.imt, a.jmt, a.ew_cyclic, a.tripole, s))) return rc;
+  mark(4);
   if (a.precision == LT_PREC_MIXED) {
     if ((rc = launch_tracer_tma_mixed(a, d->maps, d->use_tma, s, d->tma_grid))) return rc;
   } else if (a.p.adv_tracer == LT_ADV_TSPAS) {
@@ -481,7 +488,7 @@ int lt_phase_ms(lt_domain* d, float* ms, int nphase) {
     for (int p = 0; p < LT_NPHASE; ++p) {
       float t = 0.0f;
       LT_CUDA_OK(cudaEventElapsedTime(&t, ev[p], ev[p + 1]));
-      ms[LT_PHASE_ORDER[p]] += t;
+      ms[LT_PHASE_ORDER[d->prof_order[st]][p]] += t;
     }
   }
   return d->prof_steps;

@@ -6,9 +6,9 @@
 #include "lt_tracer_tma.cuh"
 
 constexpr int LT_NPHASE = 6;       // surface, sss sum, net halo, continuity, tracer, state halo
-// launch order of the phases in a step (continuity first: it needs no
-// forcing, so it runs while lt_step_host's forcing copies are in flight)
-constexpr int LT_PHASE_ORDER[LT_NPHASE] = {3, 0, 1, 2, 4, 5};
+// launch order of the phases in a step: the surface first, or with forcing
+// copies still in flight (lt_step_host) the continuity, which needs no forcing
+constexpr int LT_PHASE_ORDER[2][LT_NPHASE] = {{0, 3, 1, 2, 4, 5}, {3, 0, 1, 2, 4, 5}};
 constexpr int LT_PROF_STEPS = 512;  // steps whose phase events are kept
 
 struct lt_domain {
@@ -26,6 +26,7 @@ struct lt_domain {
   int profile = 0;
   int prof_steps = 0;
   std::vector<cudaEvent_t> prof_ev;   // [LT_PROF_STEPS][LT_NPHASE + 1]
+  unsigned char prof_order[LT_PROF_STEPS];   // the step's row of LT_PHASE_ORDER
   std::vector<void*> allocations;
   int slots = 0;
   int steps_done = 0;

@@ -1152,7 +1152,6 @@ int launch_halo_state(const Arena& a, cudaStream_t s) {
   if (!a.diagnostics) {
     return launch_chained(k_halo_state_parts, dim3(kHaloParts, a.km, 3), dim3(256), a.imt * sizeof(double), s, a);
   }
-  if (int rc = launch_halo_r8(a.net, 2, a.imt, a.jmt, a.ew_cyclic, a.tripole, s)) return rc;
   // with diagnostics, salinity's dt_diff reads temperature's new ghost values
   for (int n = 0; n < 2; ++n) {
     k_halo_state<true><<<a.km, 256, a.imt * sizeof(double), s>>>(a, n);
