@@ -121,9 +121,9 @@ def test_multistep_medium_grid(lt):
 
 @pytest.mark.parametrize("diagnostics", [False, True])
 def test_deep_ocean_bitexact(lt, diagnostics):
-    """Depths from the global ocean's area-depth curve: the column march
-    starts at the bottom level in most tiles and the deep-level paths (copies
-    below the tile's bottom, the diagnostics' deep kernel) see few levels."""
+    """Depths from the global ocean's area-depth curve: most blocks of the
+    column passes have wet levels to the bottom, and the paths of dry levels
+    (copies, zeros of the diagnostics) see few."""
     syn, f = make(lt, 120, 80, 30, forced=1, cap_north=0, hypsometry=1)
     dom = gpu_domain(lt, syn, f, diagnostics=diagnostics)
     dom.step(10)

@@ -79,6 +79,20 @@ def test_scheme_step_bitexact(lt, scheme, size, kw, nsteps, diagnostics):
     dom.close()
 
 
+# grids of 74 tiles and more, whose continuity (with the flux scheme's weighted
+# faces) is the march; smaller ones form it level by level
+@pytest.mark.parametrize("scheme", ["centered", "flux"])
+@pytest.mark.parametrize("size,kw,diagnostics", [
+    ((260, 90, 8), dict(cap_north=0), False),
+    ((261, 93, 9), dict(cap_north=2, ew_cyclic=0, tripole=0), True),
+])
+def test_scheme_step_on_marched_grids(lt, scheme, size, kw, diagnostics):
+    syn, p, f = scheme_case.case(lt, scheme, forced=1, seed=7, nx=size[0], ny=size[1], km=size[2], **kw)
+    dom, o = run_pair(lt, syn, p, f, 3, diagnostics)
+    check(dom, o, STATE + (DIAG if diagnostics else []))
+    dom.close()
+
+
 @pytest.mark.parametrize("scheme", ["centered", "flux"])
 def test_scheme_through_shim(lt, scheme):
     """tracer_ (the reference-named shim) on a domain with the scheme set:

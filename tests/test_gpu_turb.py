@@ -149,3 +149,22 @@ def test_turb_ri_on_table_entries(lt, tab, part):
         ends = np.array(ends + [-e for e in ends])
         g = with_ri(f, rng, ends, lambda r: rng.choice(np.concatenate([ends, [0.3, -0.3]]), size=r.shape))
     compare(gpu_run(lt, syn, g, tab, lt.PREC_FP64), oracle_run(lt, syn, g))
+
+
+@pytest.mark.parametrize("name,value", [("ssb", 1e-150), ("smb", np.inf), ("sm_r1", 1e-101)])
+def test_turb_tables_that_are_divided(lt, name, value):
+    """A table entry beyond the quick quotient's range (the tables' far corner,
+    or the background's last angle, which no level reaches): every quotient is
+    a division, with the same results."""
+    t = {k: v.copy() if isinstance(v, np.ndarray) else v for k, v in tables(lt).items()}
+    t[name].flat[-1] = value
+    syn, f = case(lt, 21, 1)
+    odd = lt.TurbTab(t)
+    dom = gpu_run(lt, syn, f, odd, lt.PREC_FP64)
+    plain = lt.TurbTab(tables(lt))
+    same = gpu_run(lt, syn, f, plain, lt.PREC_FP64)
+    for n in EXACT + CLOSE:
+        assert dom.get(n).tobytes() == same.get(n).tobytes(), n
+    compare(dom, oracle_run(lt, syn, f))
+    odd.close()
+    plain.close()
