@@ -274,41 +274,42 @@ bool make_tensor_map_3d(CUtensorMap* map, const void* base, int esize, long nx, 
 
 bool build_tracer_maps(const Arena& a, TracerMaps* m) {
   const long imt = a.imt, jmt = a.jmt, km = a.km;
-  const bool mx = a.precision == LT_PREC_MIXED;
-  const int es = mx ? 4 : 8;
+  const int ty = kMixedTileY;   // tile rows of the column kernel
   bool ok = true;
-  if (mx) {
-    const int ty = kMixedTileY;   // tile rows of the column kernel
-    for (int b = 0; b < 2; ++b) {
-      ok = ok && make_tensor_map_3d(&m->at[b], a.at[b], 8, imt, jmt, 2 * km, kMixedBoxW64, ty + 4);
-      ok = ok && make_tensor_map_3d(&m->atb[b], a.atb[b], 8, imt, jmt, 2 * (km + 1), kMixedBoxW64, ty + 4);
-    }
-    ok = ok && make_tensor_map_3d(&m->ws, a.ws32, es, imt, jmt, km + 1, SW, ty + 2);
-    // the U-point means wkd, wkb (rows y0-2..), faces formed in the kernel
-    ok = ok && make_tensor_map_3d(&m->uw, a.wkd32, es, imt, jmt, km, SW, ty + 3);
-    ok = ok && make_tensor_map_3d(&m->vs, a.wkb32, es, imt, jmt, km, SW, ty + 3);
-    ok = ok && make_tensor_map_3d(&m->akt, a.akt32, es, imt, jmt, 2 * km, TX, ty);
-  } else {
-    for (int b = 0; b < 2; ++b) {
-      ok = ok && make_tensor_map_3d(&m->at[b], a.at[b], 8, imt, jmt, 2 * km, kColX + 8, kColY + 2);
-      ok = ok && make_tensor_map_3d(&m->atb[b], a.atb[b], 8, imt, jmt, 2 * (km + 1), kColX + 8, kColY + 2);
-      ok = ok && make_tensor_map_3d(&m->atb_own[b], a.atb[b], 8, imt, jmt, 2 * (km + 1), kColX, kColY);
-    }
-    ok = ok && make_tensor_map_3d(&m->ws, a.ws, es, imt, jmt, km + 1, kColX, kColY);
-    ok = ok && make_tensor_map_3d(&m->uw, a.uwf, es, imt, jmt, km, kColX + 8, kColY);
-    ok = ok && make_tensor_map_3d(&m->vs, a.vsf, es, imt, jmt, km, kColX, kColY + 1);
-    ok = ok && make_tensor_map_3d(&m->akt, a.akt, es, imt, jmt, 2 * km, kColX, kColY);
+  for (int b = 0; b < 2; ++b) {
+    ok = ok && make_tensor_map_3d(&m->at[b], a.at[b], 8, imt, jmt, 2 * km, kMixedBoxW64, ty + 4);
+    ok = ok && make_tensor_map_3d(&m->atb[b], a.atb[b], 8, imt, jmt, 2 * (km + 1), kMixedBoxW64, ty + 4);
   }
-  for (int b = 0; b < 2; ++b)
-    ok = ok && make_tensor_map_3d(&m->th_at[b], a.at[b], 8, imt, jmt, 2 * km, kThomasX, kThomasY, kThomasLevels);
-  ok = ok && make_tensor_map_3d(&m->th_akt, mx ? (const void*)a.akt32 : a.akt, es, imt, jmt, 2 * km, kThomasX,
-                                kThomasY, kThomasLevels);
-  if (mx) {
-    const float* vel[4] = {a.utf32, a.vtf32, a.utl32, a.vtl32};
-    for (int v = 0; v < 4; ++v)
-      ok = ok && make_tensor_map_3d(&m->vel[v], vel[v], 4, imt, jmt, km, kMixedContBoxW, kMixedContTileY + 1);
-  }
+  ok = ok && make_tensor_map_3d(&m->ws, a.ws32, 4, imt, jmt, km + 1, SW, ty + 2);
+  // the U-point means wkd, wkb (rows y0-2..), faces formed in the kernel
+  ok = ok && make_tensor_map_3d(&m->uw, a.wkd32, 4, imt, jmt, km, SW, ty + 3);
+  ok = ok && make_tensor_map_3d(&m->vs, a.wkb32, 4, imt, jmt, km, SW, ty + 3);
+  ok = ok && make_tensor_map_3d(&m->akt, a.akt32, 4, imt, jmt, 2 * km, TX, ty);
+  const float* vel[4] = {a.utf32, a.vtf32, a.utl32, a.vtl32};
+  for (int v = 0; v < 4; ++v)
+    ok = ok && make_tensor_map_3d(&m->vel[v], vel[v], 4, imt, jmt, km, kMixedContBoxW, kMixedContTileY + 1);
   return ok;
+}
+
+bool build_column_maps(const Arena& a, ColumnMaps* m) {
+  const long imt = a.imt, jmt = a.jmt, km = a.km;
+  bool ok = true;
+  for (int b = 0; b < 2; ++b) {
+    ok = ok && make_tensor_map_3d(&m->at[b], a.at[b], 8, imt, jmt, 2 * km, kColX + 8, kColY + 2);
+    ok = ok && make_tensor_map_3d(&m->atb[b], a.atb[b], 8, imt, jmt, 2 * (km + 1), kColX + 8, kColY + 2);
+    ok = ok && make_tensor_map_3d(&m->atb_own[b], a.atb[b], 8, imt, jmt, 2 * (km + 1), kColX, kColY);
+    ok = ok && make_tensor_map_3d(&m->th_at[b], a.at[b], 8, imt, jmt, 2 * km, kThomasX, kThomasY, kThomasLevels);
+  }
+  ok = ok && make_tensor_map_3d(&m->ws, a.ws, 8, imt, jmt, km + 1, kColX, kColY);
+  ok = ok && make_tensor_map_3d(&m->uw, a.uwf, 8, imt, jmt, km, kColX + 8, kColY);
+  ok = ok && make_tensor_map_3d(&m->vs, a.vsf, 8, imt, jmt, km, kColX, kColY + 1);
+  ok = ok && make_tensor_map_3d(&m->akt, a.akt, 8, imt, jmt, 2 * km, kColX, kColY);
+  ok = ok && make_tensor_map_3d(&m->th_akt, a.akt, 8, imt, jmt, 2 * km, kThomasX, kThomasY, kThomasLevels);
+  return ok;
+}
+
+static bool build_maps(lt_domain* d) {
+  return d->a.precision == LT_PREC_MIXED ? build_tracer_maps(d->a, &d->maps) : build_column_maps(d->a, &d->column_maps);
 }
 
 int run_step(lt_domain* d, cudaEvent_t forcing_ready) {
@@ -348,7 +349,7 @@ int run_step(lt_domain* d, cudaEvent_t forcing_ready) {
   if (a.precision == LT_PREC_MIXED) {
     if ((rc = launch_tracer_tma_mixed(a, d->maps, d->use_tma, s, d->tma_grid))) return rc;
   } else if (a.p.adv_tracer == LT_ADV_TSPAS) {
-    if ((rc = launch_column_fp64(a, d->maps, d->use_tma, s))) return rc;
+    if ((rc = launch_column_fp64(a, d->column_maps, d->use_tma, s))) return rc;
   } else {
     if ((rc = launch_tracer_fp64(a, s, d->slots))) return rc;
   }
@@ -594,7 +595,7 @@ int lt_create(const lt_grid* g, const lt_params* p, lt_domain** out) {
   cudaEventCreateWithFlags(&d->ev_forcing, cudaEventDisableTiming);
   cudaStreamCreateWithFlags(&d->copy_stream, cudaStreamNonBlocking);
   // TMA-fed tracer kernel where the row pitch is a multiple of 16 bytes
-  d->use_tma = build_tracer_maps(d->a, &d->maps);
+  d->use_tma = build_maps(d);
   if (d->a.precision == LT_PREC_FP64 && prepare_column_fp64() != LT_OK) {
     lt_destroy(d);
     return LT_E_CUDA;
@@ -885,7 +886,7 @@ int lt_last_step_ms(lt_domain* d, float* ms) {
 
 int lt_use_tma(lt_domain* d, int on) {
   if (!d) return LT_E_INVALID;
-  if (on && !build_tracer_maps(d->a, &d->maps)) {
+  if (on && !build_maps(d)) {
     set_error("lt_use_tma: row pitch of this domain does not allow TMA boxes");
     return LT_E_INVALID;
   }

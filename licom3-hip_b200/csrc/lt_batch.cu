@@ -137,7 +137,7 @@ int enqueue_step(lt_batch* b, int p) {
       Arena a = d->a;
       a.cur = b->base_cur[i] ^ p;
       if ((rc = launch_continuity_fp64(a, s))) return rc;
-      rc = a.p.adv_tracer == LT_ADV_TSPAS ? launch_column_fp64(a, d->maps, d->use_tma, s)
+      rc = a.p.adv_tracer == LT_ADV_TSPAS ? launch_column_fp64(a, d->column_maps, d->use_tma, s)
                                           : launch_tracer_fp64(a, s, d->slots);
       if (rc) return rc;
     }

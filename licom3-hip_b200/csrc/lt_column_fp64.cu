@@ -96,7 +96,7 @@ __device__ __forceinline__ void copy_box(double* dst, const double* lvl, const A
 }
 
 template <bool EXPLICIT, class Slot>
-__device__ __forceinline__ void fill_slot(Slot& sl, uint64_t* bar, const Arena& a, const TracerMaps& m, bool tma, int L,
+__device__ __forceinline__ void fill_slot(Slot& sl, uint64_t* bar, const Arena& a, const ColumnMaps& m, bool tma, int L,
                                           int x0, int y0) {
   const int km = a.km;
   if (tma) {
@@ -135,7 +135,7 @@ __device__ __forceinline__ void fill_slot(Slot& sl, uint64_t* bar, const Arena& 
 
 // The first D levels of the block's march on their way.
 template <bool EXPLICIT, int D, class Smem>
-__device__ __forceinline__ void start_levels(Smem& S, const Arena& a, const TracerMaps& maps, bool tma, int x0, int y0,
+__device__ __forceinline__ void start_levels(Smem& S, const Arena& a, const ColumnMaps& maps, bool tma, int x0, int y0,
                                              int k0, int kend) {
   const int kdata = min(kend + 1, a.km);
   for (int L = k0; L < k0 + D && L < kdata; ++L)
@@ -147,7 +147,7 @@ __device__ __forceinline__ void start_levels(Smem& S, const Arena& a, const Trac
 // is refilled D-1 levels ahead.  One barrier per level.  kdata: levels below
 // kend read (kend itself for the level below the last, where there is one).
 template <bool EXPLICIT, int D, class Smem, class Body>
-__device__ __forceinline__ void march(Smem& S, const Arena& a, const TracerMaps& maps, bool tma, int x0, int y0, int k0,
+__device__ __forceinline__ void march(Smem& S, const Arena& a, const ColumnMaps& maps, bool tma, int x0, int y0, int k0,
                                       int kend, Body body) {
   const int kdata = min(kend + 1, a.km);
   auto slot_of = [&](int L) { return (L - k0) % D; };
@@ -381,7 +381,7 @@ __device__ __forceinline__ int patches_y() { return gridDim.y * (CY / PY); }
 // of a level's instructions (with a tracer per thread and 24 warps per SM it
 // took 557 us instead of 425, 720 x 460 x 55 deep).
 template <bool DIAG>
-__global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps,
+__global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant__ Arena a, const __grid_constant__ ColumnMaps maps,
                                                           int kc, int nch, int tma) {
   chain_grid();
   extern __shared__ __align__(128) unsigned char smem_col[];
@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
 // L1 instead of level slots).
 template <bool DIAG>
 __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_constant__ Arena a,
-                                                      const __grid_constant__ TracerMaps maps, int kc, int tma) {
+                                                      const __grid_constant__ ColumnMaps maps, int kc, int tma) {
   chain_grid();
   extern __shared__ __align__(128) unsigned char smem_col[];
   ExplicitSmem& S = *reinterpret_cast<ExplicitSmem*>(smem_col);
@@ -771,7 +771,7 @@ static int chunk_levels(long column_blocks, int km) {
 // Raises the column kernels' shared-memory limit on the current device (not
 // inside a stream capture).
 int prepare_column_fp64() {
-  if (int rc = prepare_thomas<double>()) return rc;
+  if (int rc = prepare_thomas()) return rc;
   const void* lim[] = {(const void*)k_limit64<false>, (const void*)k_limit64<true>};
   const void* ex[] = {(const void*)k_explicit64<false>, (const void*)k_explicit64<true>};
   for (const void* k : lim)
@@ -781,7 +781,7 @@ int prepare_column_fp64() {
   return LT_OK;
 }
 
-int launch_column_fp64(const Arena& a, const TracerMaps& maps, bool tma, cudaStream_t s) {
+int launch_column_fp64(const Arena& a, const ColumnMaps& maps, bool tma, cudaStream_t s) {
   if (int rc = launch_assm_dt_restore(a, s)) return rc;
   const unsigned gx = (a.imt + CX - 1) / CX, gy = (a.jmt + CY - 1) / CY;
   const int kc = chunk_levels((long)gx * gy, a.km);
@@ -803,7 +803,7 @@ int launch_column_fp64(const Arena& a, const TracerMaps& maps, bool tma, cudaStr
   if (int rc = launch_chained(a.diagnostics ? k_explicit64<true> : k_explicit64<false>, grid, dim3(CT),
                               sizeof(ExplicitSmem), s, a, maps, kc, t))
     return rc;
-  return a.diagnostics ? launch_thomas<double, true>(a, maps, tma, s) : launch_thomas<double, false>(a, maps, tma, s);
+  return a.diagnostics ? launch_thomas<true>(a, maps, tma, s) : launch_thomas<false>(a, maps, tma, s);
 }
 
 }  // namespace lt

@@ -34,7 +34,8 @@ struct lt_domain {
   bool owns_stream = false;
   bool use_tma = false;       // tracer kernel fed by TMA boxes (needs 16-byte row pitch)
   int tma_grid = 0;           // persistent CTAs of the TMA tracer kernel
-  lt::TracerMaps maps;
+  lt::TracerMaps maps;           // of a mixed domain
+  lt::ColumnMaps column_maps;    // of an FP64 domain
 };
 
 namespace lt {

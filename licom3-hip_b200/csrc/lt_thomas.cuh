@@ -1,4 +1,4 @@
-// lt_thomas.cuh - the last pass over the columns, both precision forms: the
+// lt_thomas.cuh - the last pass over the columns of the FP64 tspas step: the
 // implicit half of the vertical mixing (invtrit, tracer.cpp:923-978), the new
 // state, and the dry levels.
 //
@@ -28,11 +28,10 @@ constexpr int kThX = kThomasX, kThY = kThomasY, kThT = kThX * kThY;
 constexpr int kThLevels = kThomasLevels;
 constexpr int kThStages = 2;
 
-template <class AK>
 struct ThomasSmem {
   struct alignas(128) Slot {
     alignas(128) double d8[kThLevels * kThT];   // levels l0 .. l0+kThLevels-1 of the explicit values
-    alignas(128) AK akt[kThLevels * kThT];      // levels l0-1 .. of the mixing coefficient
+    alignas(128) double akt[kThLevels * kThT];      // levels l0-1 .. of the mixing coefficient
   } slot[kThStages];
   uint64_t bar[kThStages];
   int wmax[kThT / 32];
@@ -64,11 +63,10 @@ __device__ __forceinline__ int dry_from(const Arena& a, bool ring, long q, int* 
 
 // Columns of one block: x0.., y0.., tracer n.  DIAG: with the diagnostics of
 // tracer_9 (tend, dt_diff) and the pre-fold values of the top row.
-template <class AK, bool DIAG>
-__device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& maps, bool tma, int x0, int y0, int n) {
+template <bool DIAG>
+__device__ __forceinline__ void thomas_block(const Arena& a, const ColumnMaps& maps, bool tma, int x0, int y0, int n) {
   extern __shared__ __align__(128) unsigned char smem_th[];
-  ThomasSmem<AK>& S = *reinterpret_cast<ThomasSmem<AK>*>(smem_th);
-  constexpr bool F64 = sizeof(AK) == 8;
+  ThomasSmem& S = *reinterpret_cast<ThomasSmem*>(smem_th);
   const int tid = threadIdx.x, tx = tid % kThX, ty = tid / kThX;
   const int i = x0 + tx, j = y0 + ty;
   const int imt = a.imt, jmt = a.jmt, km = a.km;
@@ -97,15 +95,15 @@ __device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& m
   double* __restrict__ at_out = a.at[a.cur ^ 1] + n * a.F;
   double* __restrict__ atb_out = a.atb[a.cur ^ 1] + n * a.FB;
   const double* __restrict__ at_in = a.at[a.cur] + n * a.F;
-  const AK* __restrict__ akt = (F64 ? (const AK*)a.akt : (const AK*)a.akt32) + n * a.F;
+  const double* __restrict__ akt = a.akt + n * a.F;
   // stage t holds levels l0(t) .. l0(t)+kThLevels-1, l0(t) = (stages-1-t)*kThLevels
   const int stages = (kmax + kThLevels - 1) / kThLevels;
   auto issue = [&](int t) {
     const int l0 = (stages - 1 - t) * kThLevels, r = t % kThStages;
-    typename ThomasSmem<AK>::Slot& sl = S.slot[r];
+    ThomasSmem::Slot& sl = S.slot[r];
     if (tma) {
       if (tid == 0) {
-        mbar_expect_tx(&S.bar[r], (uint32_t)(kThLevels * kThT * (sizeof(double) + sizeof(AK))));
+        mbar_expect_tx(&S.bar[r], (uint32_t)(kThLevels * kThT * 2 * sizeof(double)));
         // boxes of both tracers' levels: beyond a tracer's last level the box
         // reads its neighbour's levels or zeros, which no column uses
         tma_load_3d(sl.d8, &maps.th_at[a.cur ^ 1], x0, y0, n * km + l0, &S.bar[r]);
@@ -120,9 +118,7 @@ __device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& m
         const bool in = inner && k < kz;
         cp_async8z(&sl.d8[c * kThT + tid], at_out + (in ? (long)k * A + q : 0), in);
         const bool ia = in && k >= 1;
-        const AK* src = akt + (ia ? (long)(k - 1) * A + q : 0);
-        if (F64) cp_async8z(&sl.akt[c * kThT + tid], src, ia);
-        else cp_async4z(&sl.akt[c * kThT + tid], src, ia);
+        cp_async8z(&sl.akt[c * kThT + tid], akt + (ia ? (long)(k - 1) * A + q : 0), ia);
       }
       cp_async_mbar_arrive(&S.bar[r]);
     }
@@ -149,12 +145,12 @@ __device__ __forceinline__ void thomas_block(const Arena& a, const TracerMaps& m
       __syncthreads();
       return;
     }
-    const typename ThomasSmem<AK>::Slot& sl = S.slot[r];
+    const ThomasSmem::Slot& sl = S.slot[r];
 #pragma unroll
     for (int c = kThLevels - 1; c >= 0; --c) {
       const int k = l0 + c;
       if (k >= kz) continue;
-      const double d8 = sl.d8[c * kThT + tid], au = (double)sl.akt[c * kThT + tid];
+      const double d8 = sl.d8[c * kThT + tid], au = sl.akt[c * kThT + tid];
       double a8, c8, b8;
       if (k >= 1) a8 = au * odzt[k] * odzp[k] * dts * 0.5;
       else a8 = odzp[0] * dts * 0.5;
@@ -361,8 +357,8 @@ __device__ __forceinline__ void dry_levels(const Arena& a, int x0, int y0, int c
   }
 }
 
-template <class AK, bool DIAG>
-__global__ void __launch_bounds__(kThT) k_thomas(const __grid_constant__ Arena a, const __grid_constant__ TracerMaps maps,
+template <bool DIAG>
+__global__ void __launch_bounds__(kThT) k_thomas(const __grid_constant__ Arena a, const __grid_constant__ ColumnMaps maps,
                                                  int tma, int parts) {
   chain_grid();
   // blockIdx.x: the column of tiles and the block's part (the sweep of either
@@ -372,30 +368,28 @@ __global__ void __launch_bounds__(kThT) k_thomas(const __grid_constant__ Arena a
   if (!DIAG) parts = 4;
   const int part = blockIdx.x % parts, x0 = blockIdx.x / parts * kThX, y0 = blockIdx.y * kThY;
   if (part < 2) {
-    thomas_block<AK, DIAG>(a, maps, tma != 0, x0, y0, part);
+    thomas_block<DIAG>(a, maps, tma != 0, x0, y0, part);
   } else if (DIAG) {
     extern __shared__ __align__(128) unsigned char smem_th[];
-    dry_levels(a, x0, y0, part - 2, reinterpret_cast<ThomasSmem<AK>*>(smem_th)->wmax);
+    dry_levels(a, x0, y0, part - 2, reinterpret_cast<ThomasSmem*>(smem_th)->wmax);
   } else {
     copy_dry(a, x0, y0, part - 2);
   }
 }
 
 // shared-memory size of the pass on the current device (not inside a capture)
-template <class AK>
-int prepare_thomas() {
-  const int sm = (int)sizeof(ThomasSmem<AK>);
-  LT_CUDA_OK(cudaFuncSetAttribute(k_thomas<AK, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-  if (sizeof(AK) == 8)
-    LT_CUDA_OK(cudaFuncSetAttribute(k_thomas<AK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+inline int prepare_thomas() {
+  const int sm = (int)sizeof(ThomasSmem);
+  LT_CUDA_OK(cudaFuncSetAttribute(k_thomas<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+  LT_CUDA_OK(cudaFuncSetAttribute(k_thomas<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
   return LT_OK;
 }
 
-template <class AK, bool DIAG>
-int launch_thomas(const Arena& a, const TracerMaps& maps, bool tma, cudaStream_t s) {
-  const size_t sm = sizeof(ThomasSmem<AK>);
+template <bool DIAG>
+int launch_thomas(const Arena& a, const ColumnMaps& maps, bool tma, cudaStream_t s) {
+  const size_t sm = sizeof(ThomasSmem);
   const int parts = !DIAG ? 4 : a.kflow ? 2 + (a.km + kDryLevels - 1) / kDryLevels : 2;
-  return launch_chained(k_thomas<AK, DIAG>, dim3((a.imt + kThX - 1) / kThX * parts, (a.jmt + kThY - 1) / kThY), dim3(kThT),
+  return launch_chained(k_thomas<DIAG>, dim3((a.imt + kThX - 1) / kThX * parts, (a.jmt + kThY - 1) / kThY), dim3(kThT),
                         sm, s, a, maps, tma ? 1 : 0, parts);
 }
 

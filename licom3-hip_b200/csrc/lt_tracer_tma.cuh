@@ -25,11 +25,17 @@ namespace lt {
 constexpr int SW = 40;      // row width of loaded boxes: columns x0-4 .. x0+35
 constexpr int HQX = TX + 2;   // a row of the tile plus a 1-cell halo
 
+// Mixed precision: the column kernel's boxes and those of the continuity march
+// (vel: utf, vtf, utl, vtl).
 struct TracerMaps {
   CUtensorMap at[2], atb[2], ws, uw, vs, akt;
-  CUtensorMap vel[4];   // mixed: utf, vtf, utl, vtl (f32) in the continuity march's boxes
-  CUtensorMap atb_own[2];         // FP64: the previous state of a block's own columns
-  CUtensorMap th_at[2], th_akt;   // the state and the mixing in the implicit pass's boxes
+  CUtensorMap vel[4];
+};
+// The FP64 tspas passes: the limiter's and the explicit pass's boxes (atb_own:
+// the previous state of a block's own columns) and the implicit pass's (th_*).
+struct ColumnMaps {
+  CUtensorMap at[2], atb[2], atb_own[2], ws, uw, vs, akt;
+  CUtensorMap th_at[2], th_akt;
 };
 
 // One member of a batched launch, in device memory.  The tensor maps come
@@ -43,9 +49,9 @@ struct alignas(64) MemberDesc {
   int tma;       // 1: level boxes by TMA; 0: by per-thread copies (row pitch TMA cannot take)
 };
 
-// The FP64 tspas passes over the columns (lt_column_fp64.cu); tma: the
-// implicit pass's level data by TMA boxes (else per-thread copies)
-int launch_column_fp64(const Arena& a, const TracerMaps& maps, bool tma, cudaStream_t s);
+// The FP64 tspas passes over the columns (lt_column_fp64.cu); tma: their level
+// data by TMA boxes (else per-thread copies)
+int launch_column_fp64(const Arena& a, const ColumnMaps& maps, bool tma, cudaStream_t s);
 // sets its kernels' shared-memory size on the current device
 int prepare_column_fp64();
 // Batched forms (mixed precision): nmem members, total work items, one
@@ -70,9 +76,10 @@ int launch_tracer_tma_mixed(const Arena& a, const TracerMaps& maps, bool tma, cu
 // The mixed continuity: TMA-fed when the domain has its maps (tma), else
 // plain loads.
 int launch_continuity_mixed(const Arena& a, const TracerMaps& maps, bool tma, cudaStream_t s);
-// Build the tensor maps of a domain; false if the layout does not allow TMA
-// (row pitch not a multiple of 16 bytes for some field).
+// Build the tensor maps of a mixed or FP64 domain; false if the layout does not
+// allow TMA (row pitch not a multiple of 16 bytes for some field).
 bool build_tracer_maps(const Arena& a, TracerMaps* maps);
+bool build_column_maps(const Arena& a, ColumnMaps* maps);
 
 // Records a timed-out wait and drains this CTA's outstanding loads (bounded).
 template <class SM>
