@@ -158,7 +158,10 @@ typedef struct lt_domain lt_domain;
 int lt_create(const lt_grid* grid, const lt_params* params, lt_domain** out);
 int lt_destroy(lt_domain* dom);
 int lt_set_params(lt_domain* dom, const lt_params* params);
-/* Bytes one domain of this grid holds on the device (admission control). */
+/* Bytes one domain of this grid holds on the device (admission control), with
+ * the tspas scheme; the centred and flux schemes add a column scratch when they
+ * are chosen (lt_create, lt_set_params): at most 2 blocks per SM of 256 threads
+ * x km x 16 bytes (24 with diagnostics). */
 size_t lt_domain_bytes(const lt_grid* grid);
 
 /* --- data movement (host pointers; synchronous on the domain's stream) --- */

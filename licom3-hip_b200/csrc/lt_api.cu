@@ -181,6 +181,17 @@ struct Plan {
   void add(void** p, size_t bytes) { items.push_back({p, bytes}); off += (bytes + 255) / 256 * 256; }
 };
 
+// The Thomas sweep's per-level coefficients of each resident CTA: of the mixed
+// column kernel and of the FP64 one of the centred and flux schemes (the tspas
+// passes keep theirs in the new state's buffers).
+bool uses_col_scratch(int precision, const lt_params& p) {
+  return precision == LT_PREC_MIXED || p.adv_tracer != LT_ADV_TSPAS;
+}
+size_t col_scratch_bytes(const Arena& a) {
+  const size_t cta_threads = a.precision == LT_PREC_MIXED ? kMixedThreads : TTHREADS;
+  return sizeof(double) * a.col_scratch_slots * a.km * a.nv_scratch * cta_threads;
+}
+
 void plan_arena(Arena& a, Plan& pl) {
   const size_t A = a.A, F = a.F, FB = a.FB, km = a.km;
   auto D = [&](double** p, size_t n) { pl.add(reinterpret_cast<void**>(p), n * sizeof(double)); };
@@ -221,9 +232,7 @@ void plan_arena(Arena& a, Plan& pl) {
     D(&a.dt_conv, 2 * F);  // convadj writes it
     D(&a.tend, 2 * F);     // convadj accumulates into it
   }
-  // the Thomas sweep's per-level coefficients of each resident CTA
-  const size_t cta_threads = a.precision == LT_PREC_MIXED ? kMixedThreads : TTHREADS;
-  D(&a.col_scratch, (size_t)a.col_scratch_slots * km * a.nv_scratch * cta_threads);
+  if (uses_col_scratch(a.precision, a.p)) pl.add(reinterpret_cast<void**>(&a.col_scratch), col_scratch_bytes(a));
 }
 
 void init_arena_dims(Arena& a, const lt_grid* g, const lt_params* p) {
@@ -347,7 +356,7 @@ int run_step(lt_domain* d, cudaEvent_t forcing_ready) {
   if (a.diagnostics && (rc = launch_halo_r8(a.net, 2, a.imt, a.jmt, a.ew_cyclic, a.tripole, s))) return rc;
   mark(4);
   if (a.precision == LT_PREC_MIXED) {
-    if ((rc = launch_tracer_tma_mixed(a, d->maps, d->use_tma, s, d->tma_grid))) return rc;
+    if ((rc = launch_tracer_tma_mixed(a, d->maps, d->use_tma, s, d->slots))) return rc;
   } else if (a.p.adv_tracer == LT_ADV_TSPAS) {
     if ((rc = launch_column_fp64(a, d->column_maps, d->use_tma, s))) return rc;
   } else {
@@ -600,9 +609,6 @@ int lt_create(const lt_grid* g, const lt_params* p, lt_domain** out) {
     lt_destroy(d);
     return LT_E_CUDA;
   }
-  // one persistent CTA of the mixed column kernel per resident slot
-  // (kMixedCtasPerSm per SM: its __launch_bounds__ and shared memory)
-  d->tma_grid = (int)std::min<long>(d->a.col_scratch_slots, (long)sms * kMixedCtasPerSm);
   if (cudaStreamSynchronize(d->stream) != cudaSuccess) {
     lt_destroy(d);
     return LT_E_CUDA;
@@ -642,6 +648,16 @@ int lt_set_params(lt_domain* d, const lt_params* p) {
   if (p->simple_assm && !d->a.restore_at) {
     set_error("lt_set_params: simple_assm needs a domain created with it");
     return LT_E_STATE;
+  }
+  if (uses_col_scratch(d->a.precision, *p) && !d->a.col_scratch) {
+    const size_t bytes = col_scratch_bytes(d->a);
+    const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&d->a.col_scratch), bytes);
+    if (e != cudaSuccess) {
+      d->a.col_scratch = nullptr;
+      set_error("lt_set_params: cudaMalloc(%zu) for the scheme's column scratch failed: %s", bytes, cudaGetErrorString(e));
+      return LT_E_OOM;
+    }
+    d->allocations.push_back(d->a.col_scratch);
   }
   d->a.p = *p;
   return LT_OK;

@@ -28,12 +28,11 @@ struct lt_domain {
   std::vector<cudaEvent_t> prof_ev;   // [LT_PROF_STEPS][LT_NPHASE + 1]
   unsigned char prof_order[LT_PROF_STEPS];   // the step's row of LT_PHASE_ORDER
   std::vector<void*> allocations;
-  int slots = 0;
+  int slots = 0;              // persistent CTAs of the mixed or the plain-load FP64 column kernel
   int steps_done = 0;
   bool have_state = false;
   bool owns_stream = false;
   bool use_tma = false;       // tracer kernel fed by TMA boxes (needs 16-byte row pitch)
-  int tma_grid = 0;           // persistent CTAs of the TMA tracer kernel
   lt::TracerMaps maps;           // of a mixed domain
   lt::ColumnMaps column_maps;    // of an FP64 domain
 };

@@ -137,6 +137,29 @@ def test_scheme_switched_between_steps(lt):
     dom.close()
 
 
+def test_column_scratch_only_with_the_scheme(lt):
+    """A tspas domain does not hold the centred and flux schemes' column scratch
+    (296 blocks x 256 threads x 16 B a level and here 75 levels: 91 MB); a switch
+    takes it, once, and the memory goes with the domain."""
+    import torch
+    syn = lt.Synth(720, 460, 75, forced=1)
+    free = lambda: torch.cuda.mem_get_info()[0]
+    dom = syn.domain(precision=lt.PREC_FP64)
+    dom.step(1)
+    dom.sync()
+    held = free()
+    p = type(syn.params).from_buffer_copy(syn.params)
+    for scheme in ("centered", "flux", "tspas", "flux"):
+        p.adv_tracer = lt.ADV_SCHEMES[scheme]
+        dom.set_params(p)
+        dom.step(1)
+        dom.sync()
+    scratch = 296 * 256 * 16 * 75
+    assert 0.9 * scratch < held - free() < 1.1 * scratch + (8 << 20)
+    dom.close()
+    assert free() > held
+
+
 def test_mixed_refuses_scheme(lt):
     syn, p, _ = scheme_case.case(lt, "flux", forced=0, seed=1, nx=40, ny=24, km=10)
     with pytest.raises(lt.LtError) as e:
