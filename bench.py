@@ -139,10 +139,16 @@ class ClockSampler:
     def __enter__(self):
         try:
             self.proc = subprocess.Popen(["nvidia-smi", "-i", str(self.idx), "--query-gpu=" + self.FIELDS,
-                                          "--format=csv,noheader,nounits", "-lms", "100"],
+                                          "--format=csv,noheader,nounits", "-lms", "20"],
                                          stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
             self.t = threading.Thread(target=self._read, daemon=True)
             self.t.start()
+            # the region may be shorter than nvidia-smi's start: begin once it
+            # samples, without the samples from before the region
+            t0 = time.time()
+            while not self.lines and self.proc.poll() is None and time.time() - t0 < 10.0:
+                time.sleep(0.005)
+            del self.lines[:]
         except OSError:
             self.proc = None
         return self
