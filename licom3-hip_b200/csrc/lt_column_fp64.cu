@@ -236,7 +236,7 @@ __device__ __forceinline__ void load_block(Smem& S, const Arena& a, int x0, int 
 // One column's faces and metric in the block's level-free data.
 struct Faces {
   const double2 *e, *w, *s, *n;
-  double tr, tr2;       // tarea_r, 2*tarea_r (the reference's *2.0*tarea_r: a power of two scales exactly)
+  double tr, tr2;       // tarea_r, 2*tarea_r (the reference's *2.0*tarea_r; not its *tarea_r*2.0, rounded before it doubles)
   bool fast;
 };
 
@@ -451,8 +451,8 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
           const double x0v = (e + c) * f.ue * g.tr - (c + w) * f.uw * g.tr;
           const double y0v = ((s + c) * f.vs - (c + nn) * f.vn) * g.tr;
           const Lw lw = lax_wendroff(g, f, dts, e - c, c - w, s - c, c - nn);
-          const double cx = -c * du * g.tr2;
-          const double cy = -c * dv * g.tr2;
+          const double cx = -c * du * g.tr * 2.0;
+          const double cy = -c * dv * g.tr * 2.0;
           double za, zb1, zb2, zc;
           if (k == 0) {
             za = -f.B * (lo[n] + c);
@@ -666,8 +666,8 @@ __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_consta
           za = f.A * (c + up[n]) - f.B * (c + lo);
           zc = -odzp * c * (f.wk - f.w1);
         }
-        const double cx = -c * du * g.tr2;
-        const double cy = -c * dv * g.tr2;
+        const double cx = -c * du * g.tr * 2.0;
+        const double cy = -c * dv * g.tr * 2.0;
         const double x0v = (e + c) * f.ue * g.tr - (c + w) * f.uw * g.tr;
         const double y0v = ((s + c) * f.vs - (c + nn) * f.vn) * g.tr;
         const double xx = -(x0v + xy.e + xy.w + cx);

@@ -251,9 +251,10 @@ __device__ __forceinline__ void copy_dry(const Arena& a, int x0, int y0, int n) 
 // levels of both tracers, whose transports it reads once, and nothing is written
 // twice.  With such levels in all three passes instead (each read them, the last
 // one wrote the explicit pass's value again) a step with diagnostics took 45.1 ms
-// at 3600 x 2302 x 55 on the linear depth map and 54.4 on the global area-depth
-// curve, now 33.0 and 50.4; 360 x 218 x 30: 496 and 549 us, now 405 and 541.  As
-// a launch of its own: 31.4 and 49.9 ms, but 419 and 567 us.
+// at 3600 x 2302 x 55 on the linear depth map and 54.1 on the global area-depth
+// curve, with these blocks 33.2 and 50.8; 360 x 218 x 30: 496 and 550 us, 411 and
+// 551.  As a launch of its own (six blocks per SM): 32.6 and 51.1 ms, but 428 and
+// 581 us; chunks of eight levels: 33.6 and 51.1 ms, 414 and 553 us.
 constexpr int kDryLevels = 16;
 __device__ __forceinline__ void dry_levels(const Arena& a, int x0, int y0, int chunk, int* wmax) {
   const int i = x0 + threadIdx.x % kThX, j = y0 + threadIdx.x / kThX;
