@@ -208,13 +208,16 @@ __device__ __forceinline__ bool interp2d(double& ri, double& rid, const TurbTabD
   const double r0 = rib[r.lo], r1 = rib[r.hi];
   if ((x_ri > 0.0e0 && (x_ri < r0 || x_ri > r1)) || (x_ri < 0.0e0 && (x_ri > r0 || x_ri < r1))) return false;
   const Stab t00 = quad_at(T, (long)N1 * d.lo + r.lo);
-  out = t00;
-  if (d.hi != d.lo) {
+  const double drid = x_rid - d0, dri = x_ri - r0;
+  if (d.hi == d.lo) {
+    // at an end: no slopes, but a NaN in Ri stays one
+    const double gone = 0.0e0 * dri, none = 0.0e0 * drid;
+    out = {t00.slq2 + gone + none, t00.sm + gone + none, t00.sh + gone + none, t00.ss + gone + none};
+  } else {
     const Stab t10 = quad_at(T, (long)N1 * d.hi + r.lo), t01 = quad_at(T, (long)N1 * d.lo + r.hi);
     // one reciprocal per direction serves four quotients, rounded as divisions
     const double dridta = d1 - d0, drita = r1 - r0;
     const double gd = 1.0 / dridta, gr = 1.0 / drita;
-    const double drid = x_rid - d0, dri = x_ri - r0;
     auto plane = [&](double v00, double v10, double v01) {
       return v00 + ratio<PLAIN>(v01 - v00, drita, gr) * dri + ratio<PLAIN>(v10 - v00, dridta, gd) * drid;
     };

@@ -151,6 +151,19 @@ def test_turb_ri_on_table_entries(lt, tab, part):
     compare(gpu_run(lt, syn, g, tab, lt.PREC_FP64), oracle_run(lt, syn, g))
 
 
+def test_turb_ri_nan(lt, tab):
+    """Some Ri not a number, beside an Ri_d within the table and beyond either
+    end of it: as in the reference, the level takes the largest diffusivity."""
+    syn, f = case(lt, 8, 1)
+    rng = np.random.default_rng(2)
+    g = dict(f)
+    g["RIT"] = np.where(rng.random(f["RIT"].shape) < 0.1, np.nan, f["RIT"])
+    beyond = 3.0 * tables(lt)["rib"][-1]
+    at = np.isnan(g["RIT"])
+    g["RICDTTMS"] = np.where(at, rng.choice([beyond, -beyond, 0.3, -2.0], size=at.shape), f["RICDTTMS"])
+    compare(gpu_run(lt, syn, g, tab, lt.PREC_FP64), oracle_run(lt, syn, g))
+
+
 @pytest.mark.parametrize("name,value", [("ssb", 1e-150), ("smb", np.inf), ("sm_r1", 1e-101)])
 def test_turb_tables_that_are_divided(lt, name, value):
     """A table entry beyond the quick quotient's range (the tables' far corner,
