@@ -21,7 +21,7 @@
 //
 // Bound by latency: a long chain per level (square roots, atan, acosh,
 // quotients, table gathers) at 20 warps per SM, instruction fetch across its
-// branches, and idle lanes where neighbours differ in stability.  4.00 -> 2.23
+// branches, and idle lanes where neighbours differ in stability.  4.00 -> 2.22
 // ms at 720 x 460 x 55 on the global area-depth curve with interleaved tables,
 // brackets found without logarithms and the angle's cosine and sine taken from
 // its components, which are nearer the exact ones than those of the rounded
@@ -69,10 +69,10 @@ __device__ __forceinline__ double eplat(const TurbConst& C, double f, double an)
   return anum / C.eplat_den;
 }
 
-// a / h with y = 1/h: where the tables allow it (TurbTabDev::plain: every entry
-// and grid step within 1e-100 .. 1e100 or zero) the division's bits without its
-// code, which this kernel has no room for in the instruction cache (thirteen
-// quotients a level with the general form's test and division: 3.54 ms)
+// a / h with y = 1/h: where the tables allow it (TurbTabDev::plain: entries and
+// steps within 1e-100 .. 1e100, entries also zero) the division's bits without
+// its code, which this kernel has no room for in the instruction cache (with the
+// general form's test and division at thirteen quotients a level 3.54 ms)
 template <bool PLAIN>
 __device__ __forceinline__ double ratio(double a, double h, double y) {
   return PLAIN ? div_fast(a, h, y) : a / h;
@@ -82,29 +82,28 @@ __device__ __forceinline__ double ratio(double a, double h, double y) {
 // (linear spacing delta up to grid[mt + mt0] = gm, geometric ratio rat beyond),
 // lo towards zero, which interp1d_expabs and interp2d_expabs find from a
 // quotient or a logarithm and a correction by one (readyc.cpp:922-941,
-// 1014-1031).  The linear part takes the same quotient.  In the geometric part
-// the first guess is a single-precision logarithm and the grid itself decides;
-// where x meets an entry, which side of it counts is left to the logarithm's
-// rounding, so there (rarely) it is formed as the reference does: the tables'
-// interpolation and the realizable limit are steps at an entry.
+// 1014-1031).  Here the first guess is a product or a single-precision logarithm
+// and the grid itself decides; where x meets an entry, which side of it counts is
+// left to the quotient's or logarithm's rounding, so there (rarely) it is formed
+// as the reference does: the tables' interpolation and the realizable limit are
+// steps at an entry.
 struct Bracket {
   int lo, hi;
 };
-__device__ __noinline__ int met_entry(double ax, const double* __restrict__ g, int s, double gm, double rat) {
-  const double ti = (double)MT0 + ((log(ax) - log(gm)) / log(rat));
+__device__ __noinline__ int met_entry(double ax, const double* __restrict__ g, int s, double gm, double delta,
+                                      double rat) {
+  const double ti = ax < gm ? ax / delta : (double)MT0 + ((log(ax) - log(gm)) / log(rat));
   int m = max(1, min(MT, (int)ti + 1));
   if (fabs(g[MT + s * m]) < ax) m = min(MT, m + 1);
   else if (m > 1 && fabs(g[MT + s * (m - 1)]) > ax) --m;
   return m;
 }
-template <bool PLAIN>
 __device__ __forceinline__ Bracket bracket(double x, const double* __restrict__ g, double gm, double delta,
                                            double inv_delta, double rat, float log2_gm, float per_log2) {
   const double ax = fabs(x);
   const int s = x >= 0.0 ? 1 : -1;
-  const bool linear = ax < gm;
   int m;
-  if (linear) m = 1 + (int)ratio<PLAIN>(ax, delta, inv_delta);
+  if (ax < gm) m = 1 + (int)(ax * inv_delta);
   else m = 1 + MT0 + (int)((__log2f((float)ax) - log2_gm) * per_log2);
   m = max(1, min(MT, m));
   double above = fabs(g[MT + s * m]), below = fabs(g[MT + s * (m - 1)]);
@@ -116,13 +115,12 @@ __device__ __forceinline__ Bracket bracket(double x, const double* __restrict__ 
     above = below;
     below = fabs(g[MT + s * (--m - 1)]);
   }
-  if (!linear && (above == ax || below == ax)) m = met_entry(ax, g, s, gm, rat);
+  if (above == ax || below == ax) m = met_entry(ax, g, s, gm, delta, rat);
   return {MT + s * (m - 1), MT + s * m};
 }
 
 // interp1d_expabs (readyc.cpp:915-973): false, outputs left as they were, when
 // x falls outside the bracketing entries
-template <bool PLAIN>
 __device__ __noinline__ bool interp1d(double x, const TurbTabDev& T, const TurbConst& C, double out[4]) {
   const double* x1 = T.and2on2a1;
   if (x > x1[2 * MT]) x = x1[2 * MT];
@@ -130,7 +128,7 @@ __device__ __noinline__ bool interp1d(double x, const TurbTabDev& T, const TurbC
   const double gm = x1[MT + MT0], gmax = x1[2 * MT];
   Bracket b;
   if (fabs(x) >= gm && fabs(x) >= gmax) b.lo = b.hi = x >= 0.0 ? 2 * MT : 0;
-  else b = bracket<PLAIN>(x, x1, gm, T.dand2on2, C.inv_da, T.rnd2on2, C.log2_gm1, C.per_log21);
+  else b = bracket(x, x1, gm, T.dand2on2, C.inv_da, T.rnd2on2, C.log2_gm1, C.per_log21);
   const double x0 = x1[b.lo], xh = x1[b.hi];
   if ((x > 0.0e0 && (x < x0 || x > xh)) || (x < 0.0e0 && (x > x0 || x < xh))) return false;
   const double dta = xh - x0;
@@ -196,7 +194,7 @@ __device__ __forceinline__ bool interp2d(double& ri, double& rid, const TurbTabD
   const double x_ri = ri, x_rid = rid;
   Bracket d, r;
   if (fabs(x_rid) >= gm && fabs(x_rid) >= rmax) d.lo = d.hi = x_rid >= 0.0 ? 2 * MT : 0;
-  else d = bracket<PLAIN>(x_rid, rib, gm, T.dri, C.inv_dri, T.rri, C.log2_gm, C.per_log2);
+  else d = bracket(x_rid, rib, gm, T.dri, C.inv_dri, T.rri, C.log2_gm, C.per_log2);
   const double d0 = rib[d.lo], d1 = rib[d.hi];
   if ((x_rid > 0.0e0 && (x_rid < d0 || x_rid > d1)) || (x_rid < 0.0e0 && (x_rid > d0 || x_rid < d1))) return false;
   if (x_ri > fmin(T.rilim[d.lo], T.rilim[d.hi])) {
@@ -204,7 +202,7 @@ __device__ __forceinline__ bool interp2d(double& ri, double& rid, const TurbTabD
     return true;
   }
   if (fabs(x_ri) >= gm && fabs(x_ri) >= rmax) r.lo = r.hi = x_ri >= 0.0 ? 2 * MT : 0;
-  else r = bracket<PLAIN>(x_ri, rib, gm, T.dri, C.inv_dri, T.rri, C.log2_gm, C.per_log2);
+  else r = bracket(x_ri, rib, gm, T.dri, C.inv_dri, T.rri, C.log2_gm, C.per_log2);
   const double r0 = rib[r.lo], r1 = rib[r.hi];
   if ((x_ri > 0.0e0 && (x_ri < r0 || x_ri > r1)) || (x_ri < 0.0e0 && (x_ri > r0 || x_ri < r1))) return false;
   const Stab t00 = quad_at(T, (long)N1 * d.lo + r.lo);
@@ -232,6 +230,13 @@ __device__ __forceinline__ bool interp2d(double& ri, double& rid, const TurbTabD
 template <bool PLAIN>
 __device__ __noinline__ bool interp2d_back(double& ri, double& rid, const TurbTabDev& T, const TurbConst& C, Stab& out) {
   return interp2d<PLAIN>(ri, rid, T, C, out);
+}
+
+// One of the background's five tables (back_ra_r, sm_r1, sh_r1, ss_r1, slq2_r1)
+// at dth beyond angle it0, with the slope to the next angle
+__device__ __forceinline__ double angle(const TurbTabDev& T, int tab, int it0, double dth) {
+  const double2 e = __ldg(T.angle + tab * LT_TURB_NB + NTH + it0);
+  return e.x + dth * e.y;
 }
 
 // The column's interface values (the reference's wp1, wp3, wp8 at level k,
@@ -402,7 +407,7 @@ __global__ void __launch_bounds__(128, 5)
       const double and2 = ridk / (rik + 1.0e-25) * an2;
       const double and2on2 = and2 / (an2 + 1.0e-25);
       double v[4];
-      if (interp1d<PLAIN>(and2on2, T, C, v)) {
+      if (interp1d(and2on2, T, C, v)) {
         amtaun2 = v[0];
         st.sm = v[1];
         st.sh = v[2];
@@ -478,8 +483,7 @@ __global__ void __launch_bounds__(128, 5)
       }
       if ((it1 > 3 * NTH) || (it0 < -NTH)) { quit = true; break; }
       double dth = theta_r - th0;
-      const double br0 = T.back_ra_r[NTH + it0];
-      double back_ra_r1 = br0 + dth * ratio<PLAIN>(T.back_ra_r[NTH + it1] - br0, T.deltheta_r, C.inv_dth);
+      double back_ra_r1 = angle(T, 0, it0, dth);
       int ifrafglt = 0;
       if ((theta_r <= T.theta_rcrp) || (theta_r >= T.theta_rcrn)) {
         if (back_ra_r1 > ra_r) {
@@ -509,13 +513,10 @@ __global__ void __launch_bounds__(128, 5)
         back = b;
       } else {
         dth = theta_r - it0 * T.deltheta_r;
-        auto between = [&](const double* tab) {
-          return tab[NTH + it0] + dth * ratio<PLAIN>(tab[NTH + it1] - tab[NTH + it0], T.deltheta_r, C.inv_dth);
-        };
-        back.sm = between(T.sm_r1);
-        back.sh = between(T.sh_r1);
-        back.ss = between(T.ss_r1);
-        back.slq2 = between(T.slq2_r1);
+        back.sm = angle(T, 1, it0, dth);
+        back.sh = angle(T, 2, it0, dth);
+        back.ss = angle(T, 3, it0, dth);
+        back.slq2 = angle(T, 4, it0, dth);
       }
       if (back.slq2 < 0.0e0) { quit = true; break; }
     }
@@ -636,7 +637,7 @@ int launch_turb(const Arena& a, const TurbTabDev& T, int ncc, double dfricmx, cu
   C.log2_gm1 = (float)std::log2(T.gm1);
   C.per_log21 = (float)(1.0 / std::log2(T.rnd2on2));
   // warps of 8 x 4 columns: depths and stability alike, so fewer idle lanes
-  // (720 x 460 x 55 deep: 2.14 ms, rows of 32 2.38)
+  // (720 x 460 x 55 deep: rows of 32 were 11 % slower)
   dim3 b(8, 16), g((a.imt + 7) / 8, (a.jmt + 15) / 16);
   (T.plain ? k_turb<true> : k_turb<false>)<<<g, b, 0, s>>>(a, T, C, (double)(float)ncc, dfricmx * 1.0e+4,
                                                            a.p.dwndmix * 1.0e+4);
@@ -674,14 +675,17 @@ int lt_turb_tables_create(const lt_turb_tables* h, lt_turb_tab** out) {
   const int* odd = nullptr;        // set while the 2-D tables are interleaved
   std::vector<double> rilim(n1);   // the realizable limit of Ri itself
   for (int m = 0; m < N1; ++m) rilim[m] = h->rib[MT + h->irimax[m]];
+  std::vector<double2> angle(5 * nb);
+  const double* angles[] = {h->back_ra_r, h->sm_r1, h->sh_r1, h->ss_r1, h->slq2_r1};
+  for (size_t t = 0; t < 5; ++t)
+    for (size_t m = 0; m < nb; ++m)
+      angle[t * nb + m] = {angles[t][m], m + 1 < nb ? (angles[t][m + 1] - angles[t][m]) / h->deltheta_r : 0.0};
   const Item items[] = {
       {nullptr, 4 * n2 * 8, (const void**)&T.quad}, {nullptr, sizeof(int), (const void**)&odd},
       {h->rib, n1 * 8, (const void**)&T.rib},         {rilim.data(), n1 * 8, (const void**)&T.rilim},
       {h->and2on2a1, n1 * 8, (const void**)&T.and2on2a1}, {h->amtaun2a1, n1 * 8, (const void**)&T.amtaun2a1},
       {h->sma1, n1 * 8, (const void**)&T.sma1},       {h->sha1, n1 * 8, (const void**)&T.sha1},
-      {h->ssa1, n1 * 8, (const void**)&T.ssa1},       {h->back_ra_r, nb * 8, (const void**)&T.back_ra_r},
-      {h->sm_r1, nb * 8, (const void**)&T.sm_r1},     {h->sh_r1, nb * 8, (const void**)&T.sh_r1},
-      {h->ss_r1, nb * 8, (const void**)&T.ss_r1},     {h->slq2_r1, nb * 8, (const void**)&T.slq2_r1}};
+      {h->ssa1, n1 * 8, (const void**)&T.ssa1},       {angle.data(), 5 * nb * 16, (const void**)&T.angle}};
   size_t total = 0;
   for (const Item& it : items) total += (it.bytes + 255) / 256 * 256;
   char* base = nullptr;
@@ -717,13 +721,9 @@ int lt_turb_tables_create(const lt_turb_tables* h, lt_turb_tab** out) {
     delete t;
     return cuda_fail(e, "lt_turb_tables_create");
   }
-  // the grids' steps and the 1-D tables on the host
-  bool plain = !any_odd && plain_entry(h->dri) && plain_entry(h->dand2on2) && plain_entry(h->deltheta_r);
+  bool plain = !any_odd && plain_entry(h->deltheta_r);
   for (size_t m = 0; m < n1 && plain; ++m)
     plain = plain_entry(h->rib[m]) && (m == 0 || (h->rib[m] != h->rib[m - 1] && plain_entry(h->rib[m] - h->rib[m - 1])));
-  const double* angle[] = {h->back_ra_r, h->sm_r1, h->sh_r1, h->ss_r1, h->slq2_r1};
-  for (const double* tab : angle)
-    for (size_t m = 0; m < nb && plain; ++m) plain = plain_entry(tab[m]);
   T.plain = plain ? 1 : 0;
   T.rib0 = h->rib[0];
   T.gm = h->rib[MT + MT0];

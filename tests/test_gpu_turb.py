@@ -164,11 +164,11 @@ def test_turb_ri_nan(lt, tab):
     compare(gpu_run(lt, syn, g, tab, lt.PREC_FP64), oracle_run(lt, syn, g))
 
 
-@pytest.mark.parametrize("name,value", [("ssb", 1e-150), ("smb", np.inf), ("sm_r1", 1e-101)])
+@pytest.mark.parametrize("name,value", [("ssb", 1e-150), ("smb", np.inf), ("slq2b", 1e-101)])
 def test_turb_tables_that_are_divided(lt, name, value):
     """A table entry beyond the quick quotient's range (the tables' far corner,
-    or the background's last angle, which no level reaches): every quotient is
-    a division, with the same results."""
+    which no level reaches): every quotient is a division, with the same
+    results."""
     t = {k: v.copy() if isinstance(v, np.ndarray) else v for k, v in tables(lt).items()}
     t[name].flat[-1] = value
     syn, f = case(lt, 21, 1)
