@@ -268,6 +268,10 @@ __device__ __forceinline__ void vertical_factors(Flow& f, double odzp, double od
   f.C2 = f.B * f.w1 * odzt1;
 }
 
+// s + x*2.0: doubling is exact, so the fused sum is rounded as the separate one
+// (where 2x overflows it is not, and the sum is at the end of the range)
+__device__ __forceinline__ double plus_twice(double s, double x) { return __fma_rn(2.0, x, s); }
+
 // unlimited (Lax-Wendroff) parts of the horizontal face fluxes
 struct Lw {
   double e, w, s, n;
@@ -451,8 +455,8 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
           const double x0v = (e + c) * f.ue * g.tr - (c + w) * f.uw * g.tr;
           const double y0v = ((s + c) * f.vs - (c + nn) * f.vn) * g.tr;
           const Lw lw = lax_wendroff(g, f, dts, e - c, c - w, s - c, c - nn);
-          const double cx = -c * du * g.tr * 2.0;
-          const double cy = -c * dv * g.tr * 2.0;
+          const double cx = -c * du * g.tr;
+          const double cy = -c * dv * g.tr;
           double za, zb1, zb2, zc;
           if (k == 0) {
             za = -f.B * (lo[n] + c);
@@ -470,8 +474,8 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
             zb2 = f.C2 * (c - lo[n]) * dts;
             zc = -odzp * c * (f.wk - f.w1);
           }
-          const double xx = -(x0v + lw.e + lw.w + cx);
-          const double yy = -(y0v + lw.s + lw.n + cy);
+          const double xx = -plus_twice(x0v + lw.e + lw.w, cx);
+          const double yy = -plus_twice(y0v + lw.s + lw.n, cy);
           const double zz = -(zb1 + zb2 + za + zc);
           const double a00 = c + (xx + yy + zz) * dts;
           // a00 > max or a00 < min over the cell and its wet neighbours,
@@ -666,12 +670,12 @@ __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_consta
           za = f.A * (c + up[n]) - f.B * (c + lo);
           zc = -odzp * c * (f.wk - f.w1);
         }
-        const double cx = -c * du * g.tr * 2.0;
-        const double cy = -c * dv * g.tr * 2.0;
+        const double cx = -c * du * g.tr;
+        const double cy = -c * dv * g.tr;
         const double x0v = (e + c) * f.ue * g.tr - (c + w) * f.uw * g.tr;
         const double y0v = ((s + c) * f.vs - (c + nn) * f.vn) * g.tr;
-        const double xx = -(x0v + xy.e + xy.w + cx);
-        const double yy = -(y0v + xy.s + xy.n + cy);
+        const double xx = -plus_twice(x0v + xy.e + xy.w, cx);
+        const double yy = -plus_twice(y0v + xy.s + xy.n, cy);
         const double zz = -(za + zb1 + zb2 + zc);
         adv = xx + yy + zz;
         if (DIAG) {
