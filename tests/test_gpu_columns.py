@@ -101,6 +101,26 @@ def test_dry_levels_with_diagnostics_bitexact(lt, nx, ny, km, cyclic, tripole):
 
 
 @pytest.mark.gpu
+def test_batch_members_with_diagnostics(lt):
+    """Members with diagnostics, one whose continuity marches (and so leaves its
+    dry levels to the last launch's blocks) and one whose does not, in a batch's
+    graph: as stepped alone."""
+    sizes = [(260, 90, 17), (61, 33, 9)]
+    kw = dict(tripole=0, ew_cyclic=0, cap_north=2, cap_south=2, forced=1)
+    alone, both = ([lt.Synth(*s, seed=k, **kw).domain(precision=lt.PREC_FP64, diagnostics=True)
+                    for k, s in enumerate(sizes)] for _ in range(2))
+    b = lt.Batch(both)
+    b.step(3)
+    b.sync()
+    for x, y in zip(alone, both):
+        x.step(3)
+        x.sync()
+        for n in ("AT", "ATB", "NET", "AX", "AY", "AZ", "DZ", "PENETRATE", "TEND", "DT_DIFF"):
+            assert x.get(n).tobytes() == y.get(n).tobytes(), n
+    b.close()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("nx,ny,km,cyclic,tripole", [(40, 30, 9, 1, 1), (261, 93, 9, 0, 0)])
 def test_diagnostics_of_denormal_values_bitexact(lt, nx, ny, km, cyclic, tripole):
     """Values and velocities whose products are below the smallest normal
