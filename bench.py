@@ -47,11 +47,11 @@ FALLBACK_HBM_GBS = 6650.0
 # U-point means wkd, wkb (8), akt (16 | 8)
 STEP_BYTES = {"fp64": 136.0, "mixed": 100.0}
 TRACER_KERNEL_BYTES = {"fp64": 104.0, "mixed": 84.0}
-# DRAM bytes per cell (read + write) of the column kernel, from one ncu
-# --set full capture of a 720x460x55 launch (profiles/); traffic grows with
-# the cells, so it scales to the bench's launch
-TRACER_KERNEL_TRAFFIC = {"fp64": (1.106355e9 + 0.653346e9) / (720 * 460 * 55),
-                         "mixed": (0.963681e9 + 0.646199e9) / (720 * 460 * 55)}
+# DRAM bytes per cell (read + write) of the column kernel (FP64: of the four
+# passes together), from ncu captures of one 720x460x55 launch each (profiles/);
+# traffic grows with the cells, so it scales to the bench's launch
+TRACER_KERNEL_TRAFFIC = {"fp64": (1.496851e9 + 0.592589e9) / (720 * 460 * 55),
+                         "mixed": (0.769636e9 + 0.613676e9) / (720 * 460 * 55)}
 
 
 def ICESNOW_BYTES_PER_POINT(km):
@@ -598,7 +598,7 @@ def measure_readyc(lt, args, precision):
     d_bytes = 56.0 * cells
     turb = {"grid": "%dx%dx%d patch of the bench grid" % (nx, ny, km), "ms_per_launch": ms,
             "cells_per_s": cells / (ms * 1e-3), "ms_scaled_to_bench_grid": ms * full / cells,
-            "bound": "fp64 arithmetic (table-index logarithms, atan, sin, cos, acosh, divisions)",
+            "bound": "latency of a column's chain of levels (square roots, atan, acosh, quotients, table gathers)",
             "tables": "stand-ins on the reference's table grids"}
     del4u = {"grid": turb["grid"], "ms_per_launch": ms_d, "cells_per_s": cells / (ms_d * 1e-3),
              "ms_scaled_to_bench_grid": ms_d * full / cells, "algorithmic_bytes_per_launch": d_bytes,

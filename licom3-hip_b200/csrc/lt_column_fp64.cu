@@ -1,4 +1,4 @@
-// lt_column_fp64.cu - the FP64 tspas step of both tracers as three passes
+// lt_column_fp64.cu - the FP64 tspas step of both tracers as four passes
 // over the columns, each expression in the reference's operation order
 // (advection_tracer_2/3 with tracer_del4_1/2, tracer_5..9 and invtrit;
 // tracer.cpp:291-978, 1238-1699).  Compiled with -fmad=false.
@@ -10,7 +10,8 @@
 //                 Laplacian, shortwave, explicit vertical mixing, surface
 //                 terms; leaves the explicitly updated value in the new state
 //   k_thomas      (lt_thomas.cuh) per column and tracer: the implicit half of
-//                 the vertical mixing, the new state, dry levels copied
+//                 the vertical mixing, the new state, dry levels copied (with
+//                 diagnostics also their zeros)
 //
 // Why passes.  Only the implicit sweep runs up and down a column; the rest is a
 // stencil that is free in every direction and limited by instruction issue and
@@ -25,9 +26,9 @@
 // need a bit per cell and tracer of storage.
 //
 // One step of the fused kernel against these passes, 720 x 460 x 55 on the
-// global area-depth curve: 2.66 ms against 0.14 (Laplacian, 3.3 TB/s) + 0.43
-// (limiter: issue slots 49 % busy, FP64 pipe 35 %) + 0.62 (explicit: 52 %, 35 %)
-// + 0.38 (implicit, 3.8 TB/s); 36 x 40 x 55: 270 us against 52.
+// global area-depth curve: 2.66 ms against 0.13 (Laplacian, 3.4 TB/s) + 0.43
+// (limiter: issue slots 49 % busy, FP64 pipe 35 %) + 0.60 (explicit: 52 %, 35 %)
+// + 0.37 (implicit, 3.8 TB/s); 36 x 40 x 55: 270 us against 50.
 #include <cstdio>
 #include "lt_common.cuh"
 #include "lt_thomas.cuh"
@@ -46,8 +47,11 @@ constexpr int PX = 8, PY = 4;
 constexpr int HW = CX + 8;
 constexpr int HB = ((CY + 2) * HW * 8 + 127) / 128 * 16; // doubles of such a box, to a 128-byte boundary
 constexpr int kColCtas = 512 / CT;                      // blocks per SM: 16 warps of 128 registers
-constexpr int kChunkMax = 56;                           // levels of one block (all 55 at once: 5.29 -> 5.19 ms
-                                                        // of column passes at 1440 x 920 x 55 against two chunks)
+// Most levels of one block, whose level constants sit in shared memory; more
+// levels are cut into equal chunks, each of which reads the levels above and
+// below it again (1440 x 920 x 55 in two chunks: 5.29 ms of column passes, in
+// one 5.19).
+constexpr int kChunkMax = 56;
 
 // ------------------------------------------------------------ level pipeline
 // One level of a block's columns in shared memory: T and S with a one-point
@@ -383,7 +387,7 @@ __device__ __forceinline__ int patches_y() { return gridDim.y * (CY / PY); }
 // Bound by issue and FP64 latency at 16 warps per SM.  Both tracers in one
 // thread: transports, masks, metric terms and the level's bookkeeping are 60 %
 // of a level's instructions (with a tracer per thread and 24 warps per SM it
-// took 557 us instead of 425, 720 x 460 x 55 deep).
+// took 557 us instead of 432, 720 x 460 x 55 deep).
 template <bool DIAG>
 __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant__ Arena a, const __grid_constant__ ColumnMaps maps,
                                                           int kc, int nch, int tma) {
@@ -522,7 +526,7 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
 // Without diagnostics the wet inner cells; with them every ring cell (ax, ay,
 // az) and every inner cell (dz, penetrate, the value) above the block's
 // dry_from.  Bound as
-// k_limit64: 616 us at 720 x 460 x 55 deep (1216 with neighbours loaded through
+// k_limit64: 605 us at 720 x 460 x 55 deep (1216 with neighbours loaded through
 // L1 instead of level slots).
 template <bool DIAG>
 __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_constant__ Arena a,

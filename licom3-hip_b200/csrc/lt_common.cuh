@@ -145,11 +145,11 @@ __device__ __forceinline__ void chain_grid() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 // Launches a kernel that begins with chain_grid(): with fewer blocks than SMs
-// as a link of the chain (it finds room beside the one before it; five FP64
-// steps of 36 x 40 x 55 take 418 us instead of 468), else in plain stream order
-// (waiting blocks of a large grid take the places of working ones: 360 x 218 x
-// 30 in FP64 takes 1448 us chained, 1342 in plain order), and so inside a
-// stream capture.
+// as a link of the chain (they find room beside the kernel before), else in plain
+// stream order (waiting blocks of a larger grid take the places of working ones),
+// and so inside a stream capture.  Five steps of 36 x 40 x 55 in FP64 and of 360 x
+// 218 x 30 in FP64 and mixed precision, us: no links 468, 1277, 975; below 148
+// blocks 418, 1288, 915; below 600 418, 1343, 909; below 2400 447, 1356, 915.
 constexpr long kChainBlocks = 148;
 template <class... P, class... A>
 int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
@@ -180,7 +180,7 @@ int launch_surface_fluxes(const Arena& a, cudaStream_t s);
 int launch_continuity_fp64(const Arena& a, cudaStream_t s);
 // Which form of the continuity: below this many 32 x 8 tiles (half an SM each)
 // every level at once, where the march would be a chain of km levels on a few
-// SMs (36 x 40 x 55, FP64: 60 us per step against 28 us); from there on the
+// SMs (36 x 40 x 55, FP64: 59 us of a step against 21); from there on the
 // march, which reads and writes each field once (360 x 218 x 30: 60 against
 // 79 us in FP64, 39 against 60 us in mixed precision).
 inline bool continuity_by_levels(long tiles) { return tiles < 74; }

@@ -5,20 +5,24 @@
 // results match the FP64 CPU oracle bit for bit.
 //
 // Launch sequence of one step (replacing tracer.cpp:1701-1903):
-//   k_ssh           SSH mean (h0f*onbc, stf)                    (tracer_1_0)
-//   k_cont_march64  uk/vk, divergence, w by upward integration,
-//                   face transports, scaled utf/vtf             (tracer_1, upwell_2..4, advection_tracer_1_0)
-//   k_surface_fluxes surface fluxes of both tracers, net, the
-//                   surface mixing floor, SSS-norm terms       (tracer_5/6 surface parts)
-//   tree sum        deterministic SSS-normalisation sum         (tracer.cpp:1849-1868)
-//   halo(net)       in-GPU ghost fill                           (pop_haloupdate_tracer1)
-//   k_limit64, k_explicit64, k_thomas (lt_column_fp64.cu; k_tracer64 for the
-//                   centred and flux schemes), both tracers: tspas
-//                   predictor/limiter, biharmonic diffusion, shortwave,
-//                   explicit and implicit vertical diffusion, surface
-//                   terms, update                               (advection_tracer_2/3, tracer_del4_1/2,
+//   k_surface       SSH mean (h0f*onbc, stf), surface fluxes of
+//                   both tracers, net, the surface mixing floor (tracer_1_0, tracer_5/6 surface parts)
+//   k_cont_march64  (small grids: k_cont_levels64, k_cont_columns64) uk/vk,
+//                   divergence, w by upward integration, face
+//                   transports, scaled utf/vtf                  (tracer_1, upwell_2..4, advection_tracer_1_0)
+//   k_sss_norm      deterministic SSS-normalisation sum         (tracer.cpp:1849-1868)
+//   k_laplace64, k_limit64, k_explicit64, k_thomas (lt_column_fp64.cu;
+//                   k_tracer64 for the centred and flux schemes), both
+//                   tracers: tspas predictor/limiter, biharmonic
+//                   diffusion, shortwave, explicit and implicit
+//                   vertical diffusion, surface terms, update   (advection_tracer_2/3, tracer_del4_1/2,
 //                                                                tracer_5..9, invtrit)
-//   k_halo_state    ghost fill + fold of the new state          (pop_haloupdate_tracer2, tracer_9 for ghosts)
+//   k_halo_state_parts  ghost fill + fold of the new state and
+//                   of net                                      (pop_haloupdate_tracer1/2, tracer_9 for ghosts)
+// A step whose forcing is still being copied in starts with k_ssh and the
+// continuity, then k_surface_fluxes, the two halves of k_surface.  With
+// diagnostics net's ghost cells are a launch before the columns (k_halo_r8) and
+// each tracer's state halo one after them (k_halo_state).
 #include <cstdio>
 #include "lt_common.cuh"
 #include "lt_halo.cuh"
@@ -528,7 +532,7 @@ __global__ void __launch_bounds__(32 * BY) k_cont_march64(const __grid_constant_
 // (k_cont_levels64: face transports, scaled velocities, divergence; the
 // neighbours' velocities come through L1), then the two sums of each column
 // (k_cont_columns64).  Same expressions in the same order.
-// 36 x 40 x 55: 9 + 17 us against the march's 54.
+// 36 x 40 x 55: 21 us of a step, with the march (and the SSH mean's launch) 59.
 constexpr int kContChunk = 4;   // levels per thread of k_cont_levels64
 __global__ void __launch_bounds__(256) k_cont_levels64(const __grid_constant__ Arena a) {
   chain_grid();

@@ -13,8 +13,8 @@
 // per-thread asynchronous copies where the row pitch does not allow boxes.
 // Every wait is bounded.
 //
-// Bound by the chain of divisions per level and by L2: 377 us at 720 x 460 x 55
-// on the global area-depth curve, 1.44 GB of DRAM traffic (3.8 TB/s).  Two
+// Bound by the chain of divisions per level and by L2: 374 us at 720 x 460 x 55
+// on the global area-depth curve, 1.43 GB of DRAM traffic (3.8 TB/s).  Two
 // stages and five blocks per SM: more blocks (six: 1.73 ms at 1440 x 920 x 55)
 // or more stages (three: 1.54 ms) push the coefficients out of L2 or leave
 // fewer blocks, against 1.34 ms.
@@ -251,10 +251,10 @@ __device__ __forceinline__ void copy_dry(const Arena& a, int x0, int y0, int n) 
 // levels of both tracers, whose transports it reads once, and nothing is written
 // twice.  With such levels in all three passes instead (each read them, the last
 // one wrote the explicit pass's value again) a step with diagnostics took 45.1 ms
-// at 3600 x 2302 x 55 on the linear depth map and 54.1 on the global area-depth
-// curve, with these blocks 33.2 and 50.8; 360 x 218 x 30: 496 and 550 us, 411 and
-// 551.  As a launch of its own (six blocks per SM): 32.6 and 51.1 ms, but 428 and
-// 581 us; chunks of eight levels: 33.6 and 51.1 ms, 414 and 553 us.
+// at 3600 x 2302 x 55 on the linear depth map and 53.6 on the global area-depth
+// curve, with these blocks 33.0 and 49.7; 360 x 218 x 30: 495 and 549 us, now 405
+// and 542.  As a launch of its own 31.4 and 49.9 ms, but 419 and 567 us; in the
+// explicit pass's launch 40.1 and 51.9 ms.
 constexpr int kDryLevels = 16;
 __device__ __forceinline__ void dry_levels(const Arena& a, int x0, int y0, int chunk, int* wmax) {
   const int i = x0 + threadIdx.x % kThX, j = y0 + threadIdx.x / kThX;

@@ -21,7 +21,7 @@
 //
 // Bound by latency: a long chain per level (square roots, atan, acosh,
 // quotients, table gathers) at 20 warps per SM, instruction fetch across its
-// branches, and idle lanes where neighbours differ in stability.  4.00 -> 2.22
+// branches, and idle lanes where neighbours differ in stability.  4.00 -> 2.21
 // ms at 720 x 460 x 55 on the global area-depth curve with interleaved tables,
 // brackets found without logarithms and the angle's cosine and sine taken from
 // its components, which are nearer the exact ones than those of the rounded
