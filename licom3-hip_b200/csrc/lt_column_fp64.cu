@@ -365,10 +365,10 @@ __device__ __forceinline__ void laplace_column(const Arena& a, int i, int j, int
 }
 
 constexpr int kLaplaceLevels = 8;
-__global__ void __launch_bounds__(128) k_laplace64(const __grid_constant__ Arena a) {
+__global__ void __launch_bounds__(128) k_laplace64(const __grid_constant__ Arena a, int row0) {
   chain_grid();
   const int k0 = blockIdx.z * kLaplaceLevels;
-  laplace_column(a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, k0, k0 + kLaplaceLevels);
+  laplace_column(a, blockIdx.x * CX + threadIdx.x, (row0 + blockIdx.y) * CY + threadIdx.y, k0, k0 + kLaplaceLevels);
 }
 
 // The thread's column in the block: warp w is the patch (w % (CX/PX), w / (CX/PX)).
@@ -382,7 +382,7 @@ struct Column {
 };
 // Flag words [tracer][level][patch row][patch column], bit l: the patch's lane l.
 __device__ __forceinline__ int patches_x() { return gridDim.x * (CX / PX); }
-__device__ __forceinline__ int patches_y() { return gridDim.y * (CY / PY); }
+__device__ __forceinline__ int patches_y(const Arena& a) { return (a.jmt + CY - 1) / CY * (CY / PY); }
 
 // Bound by issue and FP64 latency at 16 warps per SM.  Both tracers in one
 // thread: transports, masks, metric terms and the level's bookkeeping are 60 %
@@ -390,13 +390,13 @@ __device__ __forceinline__ int patches_y() { return gridDim.y * (CY / PY); }
 // took 557 us instead of 432, 720 x 460 x 55 deep).
 template <bool DIAG>
 __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant__ Arena a, const __grid_constant__ ColumnMaps maps,
-                                                          int kc, int nch, int tma) {
+                                                          int kc, int nch, int tma, int row0) {
   chain_grid();
   extern __shared__ __align__(128) unsigned char smem_col[];
   LimitSmem& S = *reinterpret_cast<LimitSmem*>(smem_col);
   const Column col;
   const int tx = col.tx, ty = col.ty;
-  const int x0 = blockIdx.x * CX, y0 = blockIdx.y * CY, i = x0 + tx, j = y0 + ty;
+  const int x0 = blockIdx.x * CX, y0 = (row0 + blockIdx.y) * CY, i = x0 + tx, j = y0 + ty;
   const int km = a.km;
   if ((int)blockIdx.z >= nch) {   // the Laplacian's blocks
     const int k = ((int)blockIdx.z - nch) * kc;
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
   if (k0 < k1 && k0 > 0)
     for (int n = 0; n < 2; ++n) up[n] = a.at[a.cur][n * a.F + (long)(k0 - 1) * a.A + q];
   const int r = (ty + 1) * HW + tx + 2, ru = ty * HW + tx, rv = ty * CX + tx;
-  const long level = (long)patches_x() * patches_y();
+  const long level = (long)patches_x() * patches_y(a);
   unsigned* words = a.flags + k0 * level + (long)(j / PY) * patches_x() + i / PX;
   march<false, kLimitDepth>(S, a, maps, tma != 0, x0, y0, k0, kend, [&](int k, const LimitSlot& L, const LimitSlot& D) {
     bool flag[2] = {false, false};
@@ -528,15 +528,17 @@ __global__ void __launch_bounds__(CT, kColCtas) k_limit64(const __grid_constant_
 // dry_from.  Bound as
 // k_limit64: 605 us at 720 x 460 x 55 deep (1216 with neighbours loaded through
 // L1 instead of level slots).
-template <bool DIAG>
+// ROW0: a launch over part of the rows (the offset costs this kernel, at its limit
+// of registers, 1 %).
+template <bool DIAG, bool ROW0>
 __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_constant__ Arena a,
-                                                      const __grid_constant__ ColumnMaps maps, int kc, int tma) {
+                                                      const __grid_constant__ ColumnMaps maps, int kc, int tma, int row0) {
   chain_grid();
   extern __shared__ __align__(128) unsigned char smem_col[];
   ExplicitSmem& S = *reinterpret_cast<ExplicitSmem*>(smem_col);
   const Column col;
   const int tx = col.tx, ty = col.ty, lane = threadIdx.x % 32;
-  const int x0 = blockIdx.x * CX, y0 = blockIdx.y * CY, i = x0 + tx, j = y0 + ty;
+  const int x0 = blockIdx.x * CX, y0 = (ROW0 ? row0 + blockIdx.y : blockIdx.y) * CY, i = x0 + tx, j = y0 + ty;
   const int imt = a.imt, jmt = a.jmt, km = a.km;
   const long A = a.A, F = a.F;
   const bool inner = i >= 2 && i < imt - 2 && j >= 2 && j < jmt - 2;
@@ -575,7 +577,7 @@ __global__ void __launch_bounds__(CT, kColCtas) k_explicit64(const __grid_consta
   // Flag words of the warp's patch at levels k-1, k, k+1; those of level k+1's
   // neighbour patches (west, east, north, south) and of level k+2 are loaded a
   // level ahead, one per lane: lanes 0-4 tracer 0's, lanes 8-12 tracer 1's.
-  const int npx = patches_x(), npy = patches_y(), px = i / PX, py = j / PY, what = lane % 8;
+  const int npx = patches_x(), npy = ROW0 ? patches_y(a) : gridDim.y * (CY / PY), px = i / PX, py = j / PY, what = lane % 8;
   const long level = (long)npx * npy;
   const unsigned* words = a.flags + (lane < 8 ? 0L : km * level) + k0 * level + (long)py * npx + px;
   const bool word_in = lane < 16 && (what == 0 || (what == 1 && px > 0) || (what == 2 && px + 1 < npx) ||
@@ -781,7 +783,8 @@ static int chunk_levels(long column_blocks, int km) {
 int prepare_column_fp64() {
   if (int rc = prepare_thomas()) return rc;
   const void* lim[] = {(const void*)k_limit64<false>, (const void*)k_limit64<true>};
-  const void* ex[] = {(const void*)k_explicit64<false>, (const void*)k_explicit64<true>};
+  const void* ex[] = {(const void*)k_explicit64<false, false>, (const void*)k_explicit64<true, false>,
+                      (const void*)k_explicit64<false, true>, (const void*)k_explicit64<true, true>};
   for (const void* k : lim)
     LT_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LimitSmem)));
   for (const void* k : ex)
@@ -794,22 +797,29 @@ int launch_column_fp64(const Arena& a, const ColumnMaps& maps, bool tma, cudaStr
   const unsigned gx = (a.imt + CX - 1) / CX, gy = (a.jmt + CY - 1) / CY;
   const int kc = chunk_levels((long)gx * gy, a.km);
   const int nch = (a.km + kc - 1) / kc;
-  const dim3 grid(gx, gy, nch);
   const int t = tma ? 1 : 0;
   // The first Laplacian: on a small grid in the limiter's launch, whose blocks
   // leave the GPU partly idle (36 x 40 x 55: a launch of 14 us less per step);
   // on a large one in a kernel of its own, at three times the occupancy.
   const bool together = (long)gx * gy * nch < 148L * kColCtas * 4;
   if (!together) {
-    if (int rc = launch_chained(k_laplace64, dim3(gx, (a.jmt + 3) / 4, (a.km + kLaplaceLevels - 1) / kLaplaceLevels),
-                                dim3(CX, 4), 0, s, a))
+    if (int rc = for_column_rows(a, [&](int r, int rows) {
+          return launch_chained(k_laplace64, dim3(gx, rows, (a.km + kLaplaceLevels - 1) / kLaplaceLevels), dim3(CX, CY), 0, s,
+                                a, r);
+        }))
       return rc;
   }
-  if (int rc = launch_chained(a.diagnostics ? k_limit64<true> : k_limit64<false>,
-                              dim3(gx, gy, together ? 2 * nch : nch), dim3(CT), sizeof(LimitSmem), s, a, maps, kc, nch, t))
+  if (int rc = for_column_rows(a, [&](int r, int rows) {
+        return launch_chained(a.diagnostics ? k_limit64<true> : k_limit64<false>,
+                              dim3(gx, rows, together ? 2 * nch : nch), dim3(CT), sizeof(LimitSmem), s, a, maps, kc, nch, t, r);
+      }))
     return rc;
-  if (int rc = launch_chained(a.diagnostics ? k_explicit64<true> : k_explicit64<false>, grid, dim3(CT),
-                              sizeof(ExplicitSmem), s, a, maps, kc, t))
+  if (int rc = for_column_rows(a, [&](int r, int rows) {
+        const bool part = rows < (int)gy;
+        return launch_chained(a.diagnostics ? (part ? k_explicit64<true, true> : k_explicit64<true, false>)
+                                            : (part ? k_explicit64<false, true> : k_explicit64<false, false>),
+                              dim3(gx, rows, nch), dim3(CT), sizeof(ExplicitSmem), s, a, maps, kc, t, r);
+      }))
     return rc;
   return a.diagnostics ? launch_thomas<true>(a, maps, tma, s) : launch_thomas<false>(a, maps, tma, s);
 }

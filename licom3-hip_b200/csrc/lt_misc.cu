@@ -5,6 +5,7 @@
 #include <vector>
 #include "lt_common.cuh"
 #include "lt_halo.cuh"
+#include "lt_tracer_tma.cuh"
 #include "lt_synth.h"
 #include "../../include/licom_synth.h"
 
@@ -43,15 +44,15 @@ struct ConvTab {
 // 256 us (6.9 TB/s) against 904 us as one kernel with the arrays.
 constexpr int kConvAhead = 4;
 constexpr int kConvLevels = 128;   // most levels taken
-__global__ void __launch_bounds__(128) k_convadj(const __grid_constant__ Arena a) {
+__global__ void __launch_bounds__(kColX * kColY) k_convadj(const __grid_constant__ Arena a, int row0) {
   extern __shared__ double s_conv[];
   const int km = a.km;
-  for (int m = threadIdx.y * blockDim.x + threadIdx.x; m < 12 * km; m += blockDim.x * blockDim.y)
+  for (int m = threadIdx.x; m < 12 * km; m += kColX * kColY)
     s_conv[m] = m < 9 * km ? a.cc[m] : m < 10 * km ? a.to[m - 9 * km] : m < 11 * km ? a.so[m - 10 * km] : a.dzp[m - 11 * km];
   __syncthreads();
   const ConvTab C{s_conv, s_conv + 9 * km, s_conv + 10 * km, s_conv + 11 * km, km};
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int i = blockIdx.x * kColX + threadIdx.x % kColX;
+  const int j = (row0 + blockIdx.y) * kColY + threadIdx.x / kColX;
   if (i >= a.imt || j >= a.jmt) return;
   const long A = a.A, F = a.F;
   const long q = (long)j * a.imt + i;
@@ -342,9 +343,12 @@ __global__ void k_synth_vel(CellTables t, double ncc1, double* utf, double* vtf,
 
 int launch_convadj(const Arena& a, cudaStream_t s) {
   if (a.km > kConvLevels) { set_error("convadj: km > %d", kConvLevels); return LT_E_INVALID; }
-  dim3 b(32, 4), g((a.imt + 31) / 32, (a.jmt + 3) / 4);
-  k_convadj<<<g, b, 12 * a.km * sizeof(double), s>>>(a);
-  LT_LAUNCHED();
+  if (int rc = for_column_rows(a, [&](int r, int rows) {
+        k_convadj<<<dim3((a.imt + kColX - 1) / kColX, rows), kColX * kColY, 12 * a.km * sizeof(double), s>>>(a, r);
+        LT_LAUNCHED();
+        return (int)LT_OK;
+      }))
+    return rc;
   k_convadj_tend<<<dim3((unsigned)((a.A + 1023) / 1024), a.km, 2), 256, 0, s>>>(a, a.p.dts, quotient_reciprocal(a.p.dts));
   LT_LAUNCHED();
   return LT_OK;

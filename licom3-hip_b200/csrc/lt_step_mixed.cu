@@ -1446,6 +1446,7 @@ int launch_tracer_mixed_batch(const MemberDesc* mem, int nmem, long total, doubl
 int launch_continuity_mixed_batch(const MemberDesc* mem, int nmem, int max_imt, int max_jmt, int km_max, int cby,
                                   cudaStream_t s) {
   const unsigned gx = (max_imt + CBX - 1) / CBX;
+  if (cby == kContTileY && (max_jmt + kContTileY - 1) / kContTileY > 65535) cby = 8;   // beyond a grid's y dimension
   switch (cby) {
     case kContTileY:
       k_cont_batch_tma<<<dim3(gx, (max_jmt + kContTileY - 1) / kContTileY, nmem), dim3(CBX, kContTileY), cont_smem(km_max), s>>>(mem);

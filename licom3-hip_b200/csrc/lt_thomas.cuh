@@ -26,6 +26,7 @@ namespace lt {
 
 constexpr int kThX = kThomasX, kThY = kThomasY, kThT = kThX * kThY;
 constexpr int kThLevels = kThomasLevels;
+static_assert(kThX == kColX && kThY == kColY, "the passes share their blocks");
 constexpr int kThStages = 2;
 
 struct ThomasSmem {
@@ -87,7 +88,6 @@ __device__ __forceinline__ void thomas_block(const Arena& a, const ColumnMaps& m
 
   int kout = kz;   // levels of this column the pass writes
   if (DIAG) {
-    static_assert(kThX == kColX && kThY == kColY, "the passes' blocks");
     const bool ring = i >= 1 && i < imt - 1 && j >= 1 && j < jmt - 1;
     kout = dry_from(a, ring, (long)j * imt + i, S.wmax);
   }
@@ -360,14 +360,14 @@ __device__ __forceinline__ void dry_levels(const Arena& a, int x0, int y0, int c
 
 template <bool DIAG>
 __global__ void __launch_bounds__(kThT) k_thomas(const __grid_constant__ Arena a, const __grid_constant__ ColumnMaps maps,
-                                                 int tma, int parts) {
+                                                 int tma, int parts, int row0) {
   chain_grid();
   // blockIdx.x: the column of tiles and the block's part (the sweep of either
   // tracer, then the dry levels: of either tracer, with diagnostics a chunk of
   // levels of both): the copying blocks only move memory, the sweeping ones
   // mostly wait for their chains of divisions, so the two kinds run side by side
   if (!DIAG) parts = 4;
-  const int part = blockIdx.x % parts, x0 = blockIdx.x / parts * kThX, y0 = blockIdx.y * kThY;
+  const int part = blockIdx.x % parts, x0 = blockIdx.x / parts * kThX, y0 = (row0 + blockIdx.y) * kThY;
   if (part < 2) {
     thomas_block<DIAG>(a, maps, tma != 0, x0, y0, part);
   } else if (DIAG) {
@@ -390,8 +390,10 @@ template <bool DIAG>
 int launch_thomas(const Arena& a, const ColumnMaps& maps, bool tma, cudaStream_t s) {
   const size_t sm = sizeof(ThomasSmem);
   const int parts = !DIAG ? 4 : a.kflow ? 2 + (a.km + kDryLevels - 1) / kDryLevels : 2;
-  return launch_chained(k_thomas<DIAG>, dim3((a.imt + kThX - 1) / kThX * parts, (a.jmt + kThY - 1) / kThY), dim3(kThT),
-                        sm, s, a, maps, tma ? 1 : 0, parts);
+  return for_column_rows(a, [&](int r, int rows) {
+    return launch_chained(k_thomas<DIAG>, dim3((a.imt + kThX - 1) / kThX * parts, rows), dim3(kThT), sm, s, a, maps,
+                          tma ? 1 : 0, parts, r);
+  });
 }
 
 }  // namespace lt

@@ -49,6 +49,17 @@ struct alignas(64) MemberDesc {
   int tma;       // 1: level boxes by TMA; 0: by per-thread copies (row pitch TMA cannot take)
 };
 
+// Launches over blocks of 32 x 4 columns: launch(first block row, block rows),
+// again where the rows are more than a grid's y dimension takes (262140 rows).
+template <class Launch>
+int for_column_rows(const Arena& a, Launch launch) {
+  constexpr int most = 65535;
+  const int rows = (a.jmt + kColY - 1) / kColY;
+  for (int r = 0; r < rows; r += most)
+    if (int rc = launch(r, rows - r < most ? rows - r : most)) return rc;
+  return LT_OK;
+}
+
 // The FP64 tspas passes over the columns (lt_column_fp64.cu); tma: their level
 // data by TMA boxes (else per-thread copies)
 int launch_column_fp64(const Arena& a, const ColumnMaps& maps, bool tma, cudaStream_t s);

@@ -89,3 +89,20 @@ def test_batch_continuity_aligned_and_not(lt, tile_y):
         x.sync()
         for n in ("WS", "AT", "UTF_OUT"):
             assert x.get(n).tobytes() == y.get(n).tobytes(), n
+
+
+def test_batch_of_more_rows_than_a_grid_dimension(lt):
+    """262204 rows are more blocks of four than a launch's y dimension takes:
+    the batch's continuity takes taller tiles there, with the same results."""
+    kw = dict(tripole=0, ew_cyclic=0, cap_north=2, cap_south=2, forced=1, hypsometry=1)
+    got = []
+    for tile_y in (4, 16):
+        dom = lt.Synth(8, 262200, 3, seed=4, **kw).domain(precision=lt.PREC_MIXED)
+        b = lt.Batch([dom])
+        b.set_config(continuity_tile_y=tile_y)
+        b.step(1)
+        b.sync()
+        got.append([dom.get(n).tobytes() for n in ("WS", "AT")])
+        b.close()
+        dom.close()
+    assert got[0] == got[1]

@@ -74,6 +74,29 @@ def test_large_grids_bitexact(lt, nx, ny, km, cyclic, tripole, hyp, diagnostics)
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("diagnostics", [False, True])
+def test_more_rows_than_a_grid_dimension_of_blocks(lt, diagnostics):
+    """262204 rows are 65551 blocks of four: more than a launch's y dimension
+    takes.  The step and the convective adjustment after it."""
+    syn = large(lt, 8, 262200, 3, 0, 0, 1)
+    f = syn.all_fields()
+    compare(lt, syn, f, 1, diagnostics)
+    if diagnostics:
+        dom = lt.TracerDomain(syn.nx, syn.ny, syn.km, syn.params, ew_cyclic=False, tripole=False)
+        o = pyoracle.Oracle(syn.nx, syn.ny, syn.km, syn.params, ew_cyclic=0, tripole=0)
+        f["AT"] = f["AT"] + np.random.default_rng(1).normal(0.0, 2.0, size=f["AT"].shape) * np.array([1.0, 1e-4])[:, None, None, None]
+        o.load(f)
+        for n in lt.INPUT_FIELDS:
+            dom.set(n, f[n])
+        dom.convadj()
+        o.convadj()
+        dom.sync()
+        assert (dom.get("AT") != f["AT"]).any()
+        for n in ("AT", "ATB", "DT_CONV"):
+            assert dom.get(n).tobytes() == o.get(n).tobytes(), n
+
+
+@pytest.mark.gpu
 def test_longest_chunk_bitexact(lt):
     syn = large(lt, 1180, 508, 56, 1, 1, 1)
     compare(lt, syn, syn.all_fields(), 1, False)
