@@ -110,6 +110,7 @@ struct alignas(16) Arena {   // copied into shared memory as 16-byte words
 struct TurbTabDev {
   const double* quad;   // [N1][N1][4]: slq2b, smb, shb, ssb of one entry together
   const double *rib, *rilim, *and2on2a1, *amtaun2a1, *sma1, *sha1, *ssa1;   // rilim: rib at irimax
+  const double* rstep;   // 1 / (rib[m + 1] - rib[m])
   const double2* angle;   // [5][LT_TURB_NB]: back_ra_r, sm_r1, sh_r1, ss_r1, slq2_r1, each with its slope to the next
   double rri, rnd2on2, dri, deltheta_r, b1, theta_rcrp, theta_rcrn, dand2on2;
   double rib0, gmax, gm, gm1;   // the first and last Ri; where the two grids turn geometric

@@ -21,7 +21,7 @@
 //
 // Bound by latency: a long chain per level (square roots, atan, acosh,
 // quotients, table gathers) at 20 warps per SM, instruction fetch across its
-// branches, and idle lanes where neighbours differ in stability.  4.00 -> 2.21
+// branches, and idle lanes where neighbours differ in stability.  4.00 -> 2.18
 // ms at 720 x 460 x 55 on the global area-depth curve with interleaved tables,
 // brackets found without logarithms and the angle's cosine and sine taken from
 // its components, which are nearer the exact ones than those of the rounded
@@ -150,6 +150,12 @@ __device__ __noinline__ bool interp1d(double x, const TurbTabDev& T, const TurbC
 struct Stab {
   double slq2, sm, sh, ss;
 };
+// 1 / (rib[b.hi] - rib[b.lo]); infinite at an end, where 0 / 0 is the slope
+__device__ __forceinline__ double step_inverse(const TurbTabDev& T, Bracket b) {
+  if (b.hi == b.lo) return INFINITY;
+  const double y = __ldg(T.rstep + min(b.lo, b.hi));
+  return b.hi > b.lo ? y : -y;
+}
 __device__ __forceinline__ Stab quad_at(const TurbTabDev& T, long c) {
   const double2* p = reinterpret_cast<const double2*>(T.quad) + 2 * c;
   const double2 u = __ldg(p), v = __ldg(p + 1);
@@ -213,9 +219,10 @@ __device__ __forceinline__ bool interp2d(double& ri, double& rid, const TurbTabD
     out = {t00.slq2 + gone + none, t00.sm + gone + none, t00.sh + gone + none, t00.ss + gone + none};
   } else {
     const Stab t10 = quad_at(T, (long)N1 * d.hi + r.lo), t01 = quad_at(T, (long)N1 * d.lo + r.hi);
-    // one reciprocal per direction serves four quotients, rounded as divisions
+    // one reciprocal per direction, laid out with the grid, serves four
+    // quotients, rounded as divisions
     const double dridta = d1 - d0, drita = r1 - r0;
-    const double gd = 1.0 / dridta, gr = 1.0 / drita;
+    const double gd = step_inverse(T, d), gr = step_inverse(T, r);
     auto plane = [&](double v00, double v10, double v01) {
       return v00 + ratio<PLAIN>(v01 - v00, drita, gr) * dri + ratio<PLAIN>(v10 - v00, dridta, gd) * drid;
     };
@@ -675,6 +682,8 @@ int lt_turb_tables_create(const lt_turb_tables* h, lt_turb_tab** out) {
   const int* odd = nullptr;        // set while the 2-D tables are interleaved
   std::vector<double> rilim(n1);   // the realizable limit of Ri itself
   for (int m = 0; m < N1; ++m) rilim[m] = h->rib[MT + h->irimax[m]];
+  std::vector<double> rstep(n1, 0.0);
+  for (size_t m = 0; m + 1 < n1; ++m) rstep[m] = 1.0 / (h->rib[m + 1] - h->rib[m]);
   std::vector<double2> angle(5 * nb);
   const double* angles[] = {h->back_ra_r, h->sm_r1, h->sh_r1, h->ss_r1, h->slq2_r1};
   for (size_t t = 0; t < 5; ++t)
@@ -682,7 +691,8 @@ int lt_turb_tables_create(const lt_turb_tables* h, lt_turb_tab** out) {
       angle[t * nb + m] = {angles[t][m], m + 1 < nb ? (angles[t][m + 1] - angles[t][m]) / h->deltheta_r : 0.0};
   const Item items[] = {
       {nullptr, 4 * n2 * 8, (const void**)&T.quad}, {nullptr, sizeof(int), (const void**)&odd},
-      {h->rib, n1 * 8, (const void**)&T.rib},         {rilim.data(), n1 * 8, (const void**)&T.rilim},
+      {h->rib, n1 * 8, (const void**)&T.rib},         {rstep.data(), n1 * 8, (const void**)&T.rstep},
+      {rilim.data(), n1 * 8, (const void**)&T.rilim},
       {h->and2on2a1, n1 * 8, (const void**)&T.and2on2a1}, {h->amtaun2a1, n1 * 8, (const void**)&T.amtaun2a1},
       {h->sma1, n1 * 8, (const void**)&T.sma1},       {h->sha1, n1 * 8, (const void**)&T.sha1},
       {h->ssa1, n1 * 8, (const void**)&T.ssa1},       {angle.data(), 5 * nb * 16, (const void**)&T.angle}};
